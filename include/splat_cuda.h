@@ -364,9 +364,8 @@ typedef struct sc_train_config {
   sc_adam_groups adam;         /* per-group learning rates                        */
   uint32_t bwd_mode;           /* sc_bwd_mode                                    */
   uint32_t use_graph;          /* capture the iteration as a CUDA graph          */
-  uint32_t blend_batch;        /* blend batch depth: list positions the blend kernels stage per batch
-                                  (a multiple of 32, capped at the tile's thread count); 0 = one per
-                                  thread (tile pixels / 2 with two pixels per thread) */
+  uint32_t blend_batch;        /* blend batch depth: list positions the blend forward takes per stage (a
+                                  multiple of 32; a quarter of them entries, 8 to 32); 0 = 128 */
   uint32_t sort_mode;          /* 0 = auto (two-level), 1 = depth presort + stable sort of the
                                   (tile, splat) pairs, 2 = depth presort + two-level binning
                                   (super tiles of 4x4 tiles, per-tile lists filled in depth order) */

@@ -11,7 +11,7 @@ Tuned axes:
   * tile shape: 16x16, 8x8, 32x8;
   * binning path: two-level super-tile item lists, or the stable sort of the
     (tile, splat) pairs (TrainConfig.sort_mode);
-  * blend batch depth: list positions the blend kernels stage per batch
+  * blend batch depth: list positions the blend forward takes per stage
     (TrainConfig.blend_batch: a quarter, half or all of the tile's threads);
   * sort radix width: 8- or 9-bit digits in the binning sort's onesweep
     passes (TrainConfig.sort_digit_bits).

@@ -231,7 +231,7 @@ __device__ __forceinline__ void adam_rows(const DSplats& s, const DMoments& mo, 
                                           const uint32_t* __restrict__ skip) {
   const uint32_t j0 = (blockIdx.x * blockDim.x + threadIdx.x) * ADAM_SPT;
   if (j0 >= count) return;
-  if (skip && (*skip & SC_DEVERR_CAPACITY)) return;  // a capacity overflow earlier in the step: leave parameters untouched
+  if (skip && (*skip & SC_DEVERR_SKIP)) return;  // a capacity overflow earlier in the step: leave parameters untouched
   if (d_bc) { ap.bc1 = d_bc[0]; ap.bc2 = d_bc[1]; ap.seed = __float_as_uint(d_bc[2]); }  // [2]: the step's bits
   const AdamFast af = adam_fast(ap);
   const int nv = (int)min((uint32_t)ADAM_SPT, count - j0);

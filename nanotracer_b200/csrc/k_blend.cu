@@ -1,38 +1,41 @@
 // k_blend.cu — per-tile alpha blending (forward + adjoint), MSE, tonemap.
 //
-// Forward (rasterize.wgsl:48-118): one CTA per (view, tile); each thread owns
-// PPT vertically adjacent pixels (a warp covers an 8 x 4 PPT block of the
-// tile), two of them in packed f32x2 arithmetic.  The tile's depth-ordered
-// list — its own pair list, or its super tile's item list filtered by the
-// member masks — is staged into shared memory in batches of B list positions
-// (the blend batch depth: one per thread by default, fewer when configured)
-// with cp.async (3 x 16 B per record), double buffered so the gather
-// of batch b+1 overlaps the blending of batch b, and the CTA leaves as soon as
-// every pixel is saturated (T < 1e-4).  The MSE of loss.rs:163-179 — dL/dC =
-// scale * 2 (C - target) / (3 W H) per pixel, squared errors reduced per CTA
-// in FP64 — runs in the forward's epilogue or in the backward's prologue.
+// Forward (rasterize.wgsl:48-118): one CTA per (view, tile), each warp on its
+// own: a thread owns PPT vertically adjacent pixels (a warp an 8 x 4 PPT block
+// of the tile), two of them in packed f32x2 arithmetic.  A warp walks the tile's
+// depth-ordered list — its own pair list, or its super tile's item list filtered
+// by the member masks — through a feed that stages 32 records (3 x 16 B each)
+// ahead with cp.async, and leaves as soon as its pixels are saturated (T <
+// 1e-4).  For an exact backward it writes down the entries that one of its pixels
+// took.  The MSE of loss.rs:163-179 — dL/dC = scale * 2 (C - target) / (3 W H) per pixel, squared
+// errors reduced per CTA in FP64 — runs in the forward's epilogue or in the
+// backward's prologue.
 //
-// Backward (rasterize_backward.wgsl:73-210): same grid, reverse walk from each
-// pixel's last contributor (exact mode) or from the list's end (the
-// reference's mode).  Per (pixel, splat) a thread forms the raw sums of the
-// opacity gradient h and its moments (h, h dx, h dy, h dx^2, h dx dy, h dy^2)
-// and the colour gradient over its pixels; two entries' 18 sums are reduced
-// over the warp together by a recursive-halving reduce-scatter (20 shuffles)
-// that leaves each total on one lane, which adds it to the entry's
-// shared-memory slot; after each batch the slots become the splats' gradients
-// (dmean.xy, dopacity, dconic.abc, dcolor.rgb, with the conic and opacity
-// applied once per entry) and go to global memory with three float4 vector
-// atomics per (tile, splat) — the reference issues nine CAS loops per (pixel,
-// splat).  The transmittance reconstruction T_i = T_{i+1} / (1 - alpha_i) uses
-// one approximate reciprocal per (pixel, splat).
+// Backward (rasterize_backward.wgsl:73-210): same grid, each warp walking back
+// over the entries that its pixels took (or, in the reference's mode and the
+// stage calls, over the list from its last contributor or end).  Per (pixel,
+// splat) a thread forms the opacity gradient h and T alpha; every 8 entries the
+// warp turns its shared-memory rows round and sums h's moments (h, h dx, h dy,
+// h dx^2, h dx dy, h dy^2) and the colour gradient over its 64 pixels, turns the
+// sums into the splats' gradients (dmean.xy, dopacity, dconic.abc, dcolor.rgb)
+// and sends them to global memory with one float4 vector atomic per lane, three
+// per (warp, splat) — the reference issues nine CAS loops per (pixel, splat).
+// The transmittance reconstruction T_i = T_{i+1} / (1 - alpha_i) uses one
+// approximate reciprocal per (pixel, splat).
+// Measured on the 1M-splat, 8-view 1080p step (BF16 storage): backward 2.86 -> 1.40 ms, and on
+// one view of it 0.76 -> 0.27 ms, against a CTA walking the list together with a
+// reduce-scatter over all lanes for every two entries and shared-memory sums.
 #include "sc_internal.cuh"
+
+#include <algorithm>
+#include <type_traits>
 
 namespace sck {
 
 struct BlendArgs {
   uint32_t width, height, tw, th, tiles_x, tiles_y, num_tiles, stride;
   uint64_t pixels;  // per view
-  uint32_t batch;   // list positions staged per batch, at most the block's threads
+  uint32_t stage;   // entries the forward stages at a time, at most STAGE
   const SceneDev* scenes;  // per-view image sizes and MSE scales (many-scene steps), or null
   bool count_pairs;        // with work counters: also count contributing (pixel, entry) pairs
 };
@@ -45,7 +48,7 @@ static BlendArgs blend_args(const sc_tiling* tl, uint32_t stride) {
   a.num_tiles = a.tiles_x * a.tiles_y;
   a.stride = stride;
   a.pixels = (uint64_t)tl->width * tl->height;
-  a.batch = 0;
+  a.stage = 32;
   a.scenes = nullptr;
   a.count_pairs = false;
   return a;
@@ -79,20 +82,11 @@ __device__ __forceinline__ void tile_pixel(const BlendArgs& a, uint32_t tx, uint
   py0 = ty * a.th + PPT * lr;
 }
 
-// the batch depth for a launch of `threads` threads: `batch` rounded down to
-// whole warps and capped at the threads (each stages one position), 0 = threads
-static uint32_t batch_depth(uint32_t batch, uint32_t threads) {
-  batch &= ~31u;
-  return (batch == 0 || batch > threads) ? threads : batch;
-}
-
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   const unsigned s = (unsigned)__cvta_generic_to_shared(smem);
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"(s), "l"(gmem) : "memory");
 }
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
-__device__ __forceinline__ void cp_async_wait_one() { asm volatile("cp.async.wait_group 1;" ::: "memory"); }
 
 #define ALPHA_MIN (1.0f / 255.0f)
 #define ALPHA_MAX 0.99f
@@ -208,7 +202,8 @@ __device__ __forceinline__ void add_pixel_pairs(unsigned long long* work, uint32
 // keeps the items whose member mask (bits 16..31 of keys; bit (ty % 4) * 4 +
 // tx % 4 is tile (tx, ty)) holds its tile.  Both lists are in depth order, so
 // a tile blends the same splats in the same order either way.
-enum { LIST_PAIRS = 0, LIST_ITEMS = 1 };
+// LIST_TAKERS (backward): the entries that the forward wrote down per warp.
+enum { LIST_PAIRS = 0, LIST_ITEMS = 1, LIST_TAKERS = 2 };
 struct ListArgs {
   const uint32_t* ids;
   const uint2* ranges;
@@ -227,84 +222,311 @@ __device__ __forceinline__ uint2 list_range(const ListArgs& l, const BlendArgs& 
   return l.ranges[(size_t)v * l.super_per_view + (ty / SC_SUPER) * l.super_x + tx / SC_SUPER];
 }
 
-// Staging a batch of list positions [p0, p1) (at most B <= blockDim of them) as
-// entries takes two calls, so that a batch's list words are loaded one batch
-// ahead of their use: fetch_list loads this thread's position (the id and, for
-// item lists, the key); place_list then stages the entries — each one's record
-// (3 float4) into rbuf by cp.async, its id into ids_out (when given) and, for
-// item lists, its position relative to `base` into pos.  Pair lists stage
-// every position (entry k = position p0 + k); item lists keep the items of the
-// CTA's tile in list order (a ballot per warp, then a prefix over the warps'
-// counts in wcnt).  place_list returns the entry count; every thread of the
-// CTA calls it.
-struct ListWord {
-  uint32_t key, id, j;
-  bool valid;
+// How a warp gets its entries, in stages of up to 32: gather() starts the copies
+// of the next stage's records (3 float4 each, cp.async) and returns its size, 0
+// at the end; ready() waits for them and returns how many of them are left to
+// blend — the list feed drops those whose alpha stays below 1/255 over the
+// warp's pixels.  The next gather() then runs beside the pixel loop.  Nothing is
+// shared with another warp, so the warps of a CTA never wait for one another:
+// with staging shared by the CTA and a barrier per batch, a tile's warps waited
+// for the slowest of them, for the list words and for the gathers at every
+// batch, about 500 cycles per kept entry in the backward and 200 in the forward (an
+// item list keeps one position in about 5).
+// (Records laid out anew with every operand of the packed arithmetic stored as a
+// pair, 64 B an entry, were slower: backward 1.58 against 1.40 ms.)
+constexpr uint32_t STAGE = 32;
+struct StageSmem {
+  float4 rec[2 * STAGE * 3];
+  uint32_t id[2 * STAGE], pos[2 * STAGE];  // pos: the list feed's
 };
 
-template <int LIST>
-__device__ __forceinline__ ListWord fetch_list(const ListArgs& l, uint32_t p0, uint32_t p1) {
-  ListWord f;
-  f.j = p0 + threadIdx.x;
-  f.valid = f.j < p1;
-  f.key = 0;
-  f.id = 0;
-  if (f.valid) {
-    if (LIST == LIST_ITEMS) f.key = l.keys[f.j];
-    f.id = l.ids[f.j];
-  }
-  return f;
+// The pixel centres of a warp, as a rectangle.
+struct WarpRect {
+  float x0, x1, y0, y1;
+};
+__device__ __forceinline__ WarpRect warp_rect(uint32_t px, uint32_t py0, uint32_t rows) {
+  WarpRect w;
+  w.x0 = (float)__reduce_min_sync(FULL_MASK, px) + 0.5f;
+  w.x1 = (float)__reduce_max_sync(FULL_MASK, px) + 0.5f;
+  w.y0 = (float)__reduce_min_sync(FULL_MASK, py0) + 0.5f;
+  w.y1 = (float)(__reduce_max_sync(FULL_MASK, py0) + rows) - 0.5f;
+  return w;
+}
+// Whether the ellipse alpha >= 1/255 of a record may hold a pixel of the
+// rectangle: its extent in x over the rectangle's band of rows (two square
+// roots, as super_row_hull) against the rectangle's columns, with the binning
+// test's margins, which cover the rounding here and in the blend.  A NaN
+// anywhere keeps the entry.
+__device__ __forceinline__ bool reaches(const float4 ra, const float4 rb, float op, const WarpRect& w) {
+  const CullShape s = cull_shape(ra.x, ra.y, rb.x, rb.y, rb.z, op);
+  const float w0 = w.y0 - s.my, w1 = w.y1 - s.my;
+  const float a0 = fmaxf(w0, -s.yh), a1 = fminf(w1, s.yh);
+  const float wr = fminf(fmaxf(-s.kx, a0), a1), wl = fminf(fmaxf(s.kx, a0), a1);
+  const float ur = (-s.b * wr + cull_sqrt(fmaxf(s.L * s.a - wr * wr * s.det, 0.0f))) * s.inv_a;
+  const float ul = (-s.b * wl - cull_sqrt(fmaxf(s.L * s.a - wl * wl * s.det, 0.0f))) * s.inv_a;
+  const bool out = op * 255.0f <= 1.0f ||
+                   (!s.keep && op == op &&
+                    (w1 < -s.yh || w0 > s.yh || s.mx + ur + 1e-2f < w.x0 || s.mx + ul - 1e-2f > w.x1));
+  return !out;
 }
 
-template <int LIST>
-__device__ __forceinline__ uint32_t place_list(const ListWord& f, uint32_t count, const float4* vrec, uint32_t bit,
-                                               uint32_t base, float4* rbuf, uint32_t* pos, uint32_t* ids_out,
-                                               uint32_t* wcnt) {
-  const uint32_t t = threadIdx.x;
-  bool keep = f.valid;
-  uint32_t slot = t, total = count;
-  if (LIST == LIST_ITEMS) {
-    keep = keep && ((f.key >> (16u + bit)) & 1u);
-    const uint32_t bal = __ballot_sync(FULL_MASK, keep);
-    const uint32_t lane = t & 31u, warp = t >> 5;
-    if (lane == 0) wcnt[warp] = __popc(bal);
-    __syncthreads();
-    uint32_t before = 0;
-    total = 0;
-    for (uint32_t w = 0; w < (blockDim.x >> 5); ++w) {
-      const uint32_t c = wcnt[w];
-      before += w < warp ? c : 0u;
-      total += c;
+__device__ __forceinline__ void copy_record(StageSmem& st, uint32_t slot, const float4* vrec, uint32_t id) {
+  const float4* src = vrec + (size_t)3 * id;
+  float4* dst = st.rec + 3 * slot;
+  cp_async16(dst, src);
+  cp_async16(dst + 1, src + 1);
+  cp_async16(dst + 2, src + 2);
+  st.id[slot] = id;
+}
+
+// List feed: the warp's list, front to back or (REV) back to front.  fill()
+// takes 128 list positions (one 16-byte load of keys and of ids per lane,
+// issued one chunk ahead) and appends the kept ones — the items of the warp's
+// tile (LIST_ITEMS), or all of a pair list — to a queue that gather() takes
+// the stages from.
+constexpr uint32_t QCAP = 256;  // under one stage pending and a chunk, rounded up to a power of two
+struct ListSmem {
+  StageSmem st;
+  uint2 q[QCAP];  // (id, list position)
+};
+
+template <int LIST, bool REV>
+struct ListFeed {
+  using Smem = ListSmem;
+  ListSmem& sm;
+  const uint32_t* ids;
+  const uint32_t* keys;
+  const float4* vrec;
+  uint32_t mask;          // LIST_ITEMS: the tile's member bit
+  uint32_t begin, end;    // the walked positions, as indices into ids
+  uint32_t most;          // entries per stage
+  uint32_t at;            // next chunk: [at, at + 128), REV: [at - 128, at); a multiple of 4
+  uint32_t qtail, qhead;  // entries queued and gathered
+  uint4 key, wid;         // this lane's four words of the next chunk
+
+  __device__ __forceinline__ ListFeed(ListSmem& smem, const ListArgs& l, const float4* rec, uint32_t b, uint32_t n,
+                                      uint32_t bit, uint32_t stage)
+      : sm(smem), ids(l.ids), keys(l.keys), vrec(rec), mask(0x10000u << bit), begin(b), end(b + n), most(stage),
+        at(REV ? (b + n + 3u) & ~3u : b & ~3u), qtail(0), qhead(0), key(make_uint4(0, 0, 0, 0)), wid(key) {
+    load();
+  }
+  __device__ __forceinline__ bool more() const { return REV ? at > begin : at < end; }
+  // first index of this lane's four, and whether they hold a walked position
+  __device__ __forceinline__ uint32_t first() const {
+    const uint32_t lane = threadIdx.x & 31;
+    return REV ? at - 4 - 4 * lane : at + 4 * lane;
+  }
+  __device__ __forceinline__ bool mine() const {
+    return REV ? at > begin + 4 * (threadIdx.x & 31) : first() < end;
+  }
+  // the lists' arrays are 16-byte aligned and go on past their last entry, so a
+  // group of four holding a walked position is readable whole
+  __device__ __forceinline__ void load() {
+    if (mine()) {
+      if (LIST == LIST_ITEMS) key = __ldg(reinterpret_cast<const uint4*>(keys + first()));
+      wid = __ldg(reinterpret_cast<const uint4*>(ids + first()));
     }
-    slot = before + __popc(bal & ((1u << lane) - 1u));
   }
-  if (keep) {
-    const float4* src = vrec + (size_t)3 * f.id;
-    float4* dst = rbuf + 3 * slot;
-    cp_async16(dst, src);
-    cp_async16(dst + 1, src + 1);
-    cp_async16(dst + 2, src + 2);
-    if (LIST == LIST_ITEMS) pos[slot] = f.j - base;
-    if (ids_out) ids_out[slot] = f.id;
+  __device__ __forceinline__ void fill() {
+    const uint32_t lt = (1u << (threadIdx.x & 31)) - 1u, i = first();
+    const bool any = mine();
+    const uint32_t k4[4] = {key.x, key.y, key.z, key.w}, w4[4] = {wid.x, wid.y, wid.z, wid.w};
+    bool keep[4];
+    uint32_t slot = qtail;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      keep[e] = any && i + e >= begin && i + e < end && (LIST == LIST_PAIRS || (k4[e] & mask));
+      const uint32_t bal = __ballot_sync(FULL_MASK, keep[e]);
+      slot += __popc(bal & lt);
+      qtail += __popc(bal);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {  // in walking order
+      const int c = REV ? 3 - e : e;
+      if (keep[c]) sm.q[slot++ % QCAP] = make_uint2(w4[c], i + c - begin);
+    }
+    at = REV ? at - min(at, 128u) : at + 128;
+    if (more()) load();
+    __syncwarp();
   }
-  cp_async_commit();
-  return total;
+  __device__ __forceinline__ uint32_t gather() {
+    while (qtail - qhead < most && more()) fill();
+    const uint32_t n = min(most, qtail - qhead), lane = threadIdx.x & 31;
+    if (lane < n) {
+      const uint2 w = sm.q[(qhead + lane) % QCAP];
+      copy_record(sm.st, lane, vrec, w.x);
+      sm.st.pos[lane] = w.y;
+    }
+    qhead += n;
+    return n;
+  }
+  // the landed stage, culled, moves from the buffer's first half to its second
+  __device__ __forceinline__ uint32_t ready(uint32_t n, const WarpRect& w) {
+    cp_async_wait_all();
+    __syncwarp();
+    const uint32_t lane = threadIdx.x & 31;
+    const float4* r = sm.st.rec + 3 * lane;
+    const float4 ra = r[0], rb = r[1], rc = r[2];
+    const uint32_t id = sm.st.id[lane], pos = sm.st.pos[lane];
+    const bool keep = lane < n && reaches(ra, rb, rc.w, w);
+    const uint32_t bal = __ballot_sync(FULL_MASK, keep);
+    if (keep) {
+      const uint32_t slot = STAGE + __popc(bal & ((1u << lane) - 1u));
+      float4* d = sm.st.rec + 3 * slot;
+      d[0] = ra; d[1] = rb; d[2] = rc;
+      sm.st.id[slot] = id;
+      sm.st.pos[slot] = pos;
+    }
+    __syncwarp();
+    return __popc(bal);
+  }
+  // records, ids and list positions of the entries to blend
+  __device__ __forceinline__ const float4* rec() const { return sm.st.rec + 3 * STAGE; }
+  __device__ __forceinline__ const uint32_t* id() const { return sm.st.id + STAGE; }
+  __device__ __forceinline__ uint32_t pos(uint32_t i) const { return sm.st.pos[STAGE + i]; }
+};
+
+// Taker feed: the entries that some pixel of the warp took in the forward, which
+// wrote them down (TakerOut) in chunks of 32 ids, each chunk naming the one
+// before it; walked back to front.  pos is the entry's index among them.  An
+// exact backward fed so evaluates no entry in vain (30 % of the kept entries of the
+// 1M-splat, 8-view workload have no taker in a warp of 8 x 8 pixels) and scans no list.
+struct TakerFeed {
+  using Smem = StageSmem;
+  StageSmem& sm;
+  const TakerChunks& ch;
+  const float4* vrec;
+  uint32_t left;    // entries not gathered
+  uint32_t n_next;  // size of the next stage (its ids are in wid), and the chunk before it
+  uint32_t wid, prev;
+  uint32_t base, base_next;  // pos of the first entry of the landed stage, and of the one gathered
+  uint32_t par;              // buffer half the next gather fills: 0 or STAGE
+
+  __device__ __forceinline__ TakerFeed(StageSmem& smem, const TakerChunks& c, const float4* rec, uint2 head)
+      : sm(smem), ch(c), vrec(rec), left(head.y), n_next(0), wid(0), prev(head.x), base(0), base_next(0), par(0) {
+    load();
+  }
+  __device__ __forceinline__ void load() {
+    n_next = left ? ((left - 1) & (STAGE - 1)) + 1 : 0;
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t c = prev;
+    if (lane < n_next) wid = __ldg(ch.ids + (size_t)c * STAGE + (n_next - 1 - lane));
+    if (left > STAGE) prev = __ldg(ch.prev + c);
+  }
+  __device__ __forceinline__ uint32_t gather() {
+    const uint32_t n = n_next, lane = threadIdx.x & 31;
+    if (lane < n) copy_record(sm, par + lane, vrec, wid);
+    base_next = left - 1;
+    left -= n;
+    if (n) load();
+    return n;
+  }
+  __device__ __forceinline__ uint32_t ready(uint32_t n, const WarpRect&) {
+    base = base_next;
+    par ^= STAGE;
+    cp_async_wait_all();
+    __syncwarp();
+    return n;
+  }
+  __device__ __forceinline__ const float4* rec() const { return sm.rec + 3 * (par ^ STAGE); }
+  __device__ __forceinline__ const uint32_t* id() const { return sm.id + (par ^ STAGE); }
+  __device__ __forceinline__ uint32_t pos(uint32_t i) const { return base - i; }
+};
+
+// The forward's side: a warp appends its takers' ids to a small ring and writes
+// every 32 of them to a chunk of its own.  A chunk number is drawn when the one
+// before it is written, so that its latency is hidden; the draws go to
+// TAKER_POOLS counters, each with its share of the chunks.  A pool that runs out
+// raises an error: the step's later kernels then do nothing, and the caller runs
+// it again with the chunks it needs.
+struct TakerOut {
+  const TakerChunks& ch;
+  uint32_t* ring;        // 64 ids
+  uint32_t count;        // takers so far
+  uint32_t chunk, last;  // chunk being filled, and the one before it
+  bool ok;
+
+  __device__ __forceinline__ uint32_t draw() {
+    uint32_t c = 0;
+    if ((threadIdx.x & 31) == 0) c = atomicAdd(ch.drawn + blockIdx.x % TAKER_POOLS, 1u);
+    return c;
+  }
+  __device__ __forceinline__ TakerOut(const TakerChunks& c, uint32_t* r)
+      : ch(c), ring(r), count(0), chunk(0), last(0), ok(true) {
+    chunk = draw();
+  }
+  // the chunk drawn, as every lane's number
+  __device__ __forceinline__ uint32_t number() {
+    const uint32_t c = __shfl_sync(FULL_MASK, chunk, 0);
+    ok = ok && c < ch.pool_cap;
+    return (blockIdx.x % TAKER_POOLS) * ch.pool_cap + min(c, ch.pool_cap - 1);
+  }
+  // append the entries of a stage whose bit in m is set (this lane's entry has id)
+  __device__ __forceinline__ void append(uint32_t m, uint32_t id) {
+    const uint32_t lane = threadIdx.x & 31, n = __popc(m), at = count % STAGE;
+    if (m >> lane & 1u) ring[(count + __popc(m & ((1u << lane) - 1u))) % (2 * STAGE)] = id;
+    __syncwarp();
+    if (at + n >= STAGE) {
+      const uint32_t c = number();
+      ch.ids[(size_t)c * STAGE + lane] = ring[(count - at + lane) % (2 * STAGE)];
+      if (lane == 0) ch.prev[c] = last;
+      last = c;
+      chunk = draw();
+      __syncwarp();
+    }
+    count += n;
+  }
+  // the last chunk, and where the walk back starts: (chunk, takers)
+  __device__ __forceinline__ uint2 finish(uint32_t* err) {
+    const uint32_t lane = threadIdx.x & 31, at = count % STAGE;
+    uint32_t head = last;
+    if (at) {
+      const uint32_t c = number();
+      if (lane < at) ch.ids[(size_t)c * STAGE + lane] = ring[(count - at + lane) % (2 * STAGE)];
+      if (lane == 0) ch.prev[c] = last;
+      head = c;
+    }
+    if (!ok && lane == 0) atomicOr(err, SC_DEVERR_TAKERS);
+    return make_uint2(head, ok ? count : 0u);
+  }
+};
+
+struct NoTakers {
+  __device__ __forceinline__ NoTakers(const TakerChunks&, uint32_t*) {}
+};
+
+// The CTA's warps meet only for the work counters: the list positions the
+// furthest warp covered and the entries it kept.
+__device__ __forceinline__ void add_tile_work(unsigned long long* work, uint32_t scanned, uint32_t staged,
+                                              uint32_t* s_work) {
+  if (!work) return;
+  if (threadIdx.x < 2) s_work[threadIdx.x] = 0;
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) {
+    atomicMax(&s_work[0], scanned);
+    atomicMax(&s_work[1], staged);
+  }
+  __syncthreads();
+  add_work(work, s_work[0], s_work[1]);
 }
 
 // ---------------------------------------------------------------- forward
-template <int PPT, int LIST, bool COUNT>
+// TAKERS: write down each warp's takers (TakerOut); aux then holds a pixel's last
+// contributor as its index among them plus one, else as its list position plus one.
+struct TakerRing { uint32_t id[2 * STAGE]; };
+template <int PPT, int LIST, bool COUNT, bool TAKERS>
 __global__ void __launch_bounds__(256) k_composite(const float4* __restrict__ rec, ListArgs l, BlendArgs a,
                                                    float4* __restrict__ image, uint2* __restrict__ aux,
                                                    const float* __restrict__ target, float gscale,
                                                    float4* __restrict__ dl_dc, double* __restrict__ loss,
-                                                   const uint32_t* __restrict__ skip,
-                                                   unsigned long long* __restrict__ work) {
-  extern __shared__ float4 sbuf[];  // records [2][B][3], item positions [2][B] (u32)
+                                                   uint32_t* __restrict__ skip, unsigned long long* __restrict__ work,
+                                                   TakerChunks takers) {
+  extern __shared__ float4 sbuf[];  // one ListSmem per warp, then one TakerRing per warp
   __shared__ double sred[8];
-  __shared__ uint32_t s_wcnt[2][8];
+  __shared__ uint32_t s_work[2];
   if (skip && (*skip & SC_DEVERR_CAPACITY)) return;  // the lists of this step are incomplete
-  const uint32_t B = a.batch;
-  uint32_t* spos = reinterpret_cast<uint32_t*>(sbuf + (size_t)6 * B);
+  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_warps = blockDim.x >> 5;
+  ListSmem& sm = reinterpret_cast<ListSmem*>(sbuf)[warp];
   const uint32_t vt = blockIdx.x;
   const uint32_t v = vt / a.num_tiles, tile = vt - v * a.num_tiles;
   const uint32_t ty = tile / a.tiles_x, tx = tile - ty * a.tiles_x;
@@ -316,139 +538,123 @@ __global__ void __launch_bounds__(256) k_composite(const float4* __restrict__ re
   view_dims(a, v, gscale, W, H, gs);
   uint32_t bit;
   const uint2 r = list_range<LIST>(l, a, v, tx, ty, tile, bit);
-  const uint32_t begin = r.x, end = r.y > r.x ? r.y : r.x;
-  const uint32_t nb = (end - begin + B - 1) / B;
+  const uint32_t begin = r.x, len = r.y > r.x ? r.y - r.x : 0u;
   const float4* vrec = rec + (size_t)3 * v * a.stride;
-
-  auto fetch = [&](uint32_t b) -> ListWord {
-    const uint32_t p0 = begin + b * B;
-    return fetch_list<LIST>(l, p0, min(end, p0 + B));
-  };
-  auto place = [&](uint32_t b, const ListWord& f) -> uint32_t {
-    return place_list<LIST>(f, min(B, end - (begin + b * B)), vrec, bit, begin, sbuf + (size_t)(b & 1) * 3 * B,
-                            spos + (b & 1) * B, nullptr, s_wcnt[b & 1]);
-  };
-  // list position (relative to begin) of entry k of batch b
-  auto position = [&](uint32_t b, uint32_t k) -> uint32_t {
-    return LIST == LIST_PAIRS ? b * B + k : spos[(b & 1) * B + k];
-  };
 
   float T[PPT], cr[PPT], cg[PPT], cb[PPT], fy[PPT];
   uint32_t last[PPT];
-  bool done[PPT];
+  bool in[PPT];
   bool all_done = true;
 #pragma unroll
   for (int k = 0; k < PPT; ++k) {
-    T[k] = 1.0f; cr[k] = cg[k] = cb[k] = 0.f; last[k] = 0;
+    cr[k] = cg[k] = cb[k] = 0.f; last[k] = 0;
     fy[k] = (float)(py0 + k) + 0.5f;
-    done[k] = !(px < W && py0 + k < H);
-    all_done &= done[k];
+    in[k] = px < W && py0 + k < H;
+    // a pixel is done exactly when its T < 1e-4: one outside the image, never
+    // written, runs with T = 0
+    T[k] = in[k] ? 1.0f : 0.0f;
+    all_done &= !in[k];
   }
-  ListWord f = fetch(0);
-  uint32_t cnt_next = nb > 0 ? place(0, f) : 0u;
-  if (nb > 1) f = fetch(1);
-  uint32_t w_scan = 0, w_staged = 0, w_pix = 0;
-  for (uint32_t b = 0; b < nb; ++b) {
-    const uint32_t cnt = cnt_next;
-    w_scan += min(B, end - (begin + b * B));
-    w_staged += cnt;
-    if (b + 1 < nb) {
-      cnt_next = place(b + 1, f);
-      if (b + 2 < nb) f = fetch(b + 2);
-      cp_async_wait_one();
-    } else {
-      cp_async_wait_all();
-    }
-    __syncthreads();
-    if (!all_done) {
-      const float4* sb = sbuf + (size_t)(b & 1) * 3 * B;
-      if constexpr (PPT == 2) {
-        // both pixels in packed arithmetic; a pixel that skips the splat gets
-        // alpha 0, which leaves its colour and T bit for bit unchanged.  A
-        // pixel is done exactly when its T < 1e-4 (a pixel outside the image,
-        // never written, runs with T = 0).
-        const bool in0 = px < W && py0 < H, in1 = px < W && py0 + 1 < H;
-        float2 T2 = make_float2(in0 ? T[0] : 0.0f, in1 ? T[1] : 0.0f);
-        float2 R2 = make_float2(cr[0], cr[1]), G2 = make_float2(cg[0], cg[1]), B2 = make_float2(cb[0], cb[1]);
-        const float2 fy2 = make_float2(fy[0], fy[1]);
-        int lk0 = -1, lk1 = -1;  // this batch's last contributing entries, as list positions below
-        auto blend1 = [&](uint32_t k) {
-          const float4 ra = sb[3 * k], rb = sb[3 * k + 1], rc = sb[3 * k + 2];
-          const EntryGeom e = entry_geom(fx, ra, rb);
+  uint32_t w_pix = 0, scanned = 0, staged = 0;
+  uint2 taken = make_uint2(0u, 0u);
+  if (len > 0 && !__all_sync(FULL_MASK, all_done)) {
+    ListFeed<LIST, false> feed(sm, l, vrec, begin, len, bit, a.stage);
+    TakerRing* rings = reinterpret_cast<TakerRing*>(reinterpret_cast<ListSmem*>(sbuf) + n_warps);
+    typename std::conditional<TAKERS, TakerOut, NoTakers>::type out(takers, rings[warp].id);
+    float2 T2 = make_float2(T[0], T[PPT - 1]);
+    float2 R2 = f2(0.f), G2 = R2, B2 = R2;
+    const float2 fy2 = make_float2(fy[0], fy[PPT - 1]);
+    bool sat = false;
+    const WarpRect rect = warp_rect(px, py0, PPT);
+    for (uint32_t n_raw = feed.gather(); n_raw > 0 && !sat;) {
+      const uint32_t n = feed.ready(n_raw, rect);
+      n_raw = feed.gather();
+      const float4* sr = feed.rec();
+      uint32_t took[PPT];  // this stage's entries that the pixels took
+#pragma unroll
+      for (int q = 0; q < PPT; ++q) took[q] = 0;
+      auto blend = [&](const float4* r, uint32_t b) {
+        const float4 ra = r[0], rb = r[1], rc = r[2];
+        const EntryGeom e = entry_geom(fx, ra, rb);
+        if constexpr (PPT == 2) {
+          // both pixels, without a branch: a pixel that skips the splat gets
+          // alpha 0, which leaves its colour and T bit for bit unchanged
           float2 dy, g, araw, al;
           bool v0, v1;
           eval_alpha2(e, rb.z, fy2, ra.y, rc.w, dy, g, araw, al, v0, v1);
           v0 &= T2.x >= 1e-4f;
           v1 &= T2.y >= 1e-4f;
-          // without a branch: a pixel that skips gets alpha 0, which changes no bit
           const float2 am = make_float2(v0 ? al.x : 0.0f, v1 ? al.y : 0.0f);
           const float2 ta = __fmul2_rn(T2, am);
           R2 = __ffma2_rn(ta, f2(rc.x), R2);
           G2 = __ffma2_rn(ta, f2(rc.y), G2);
           B2 = __ffma2_rn(ta, f2(rc.z), B2);
-          T2 = __fmul2_rn(T2, __fadd2_rn(f2(1.0f), make_float2(-am.x, -am.y)));
+          T2 = __fmul2_rn(T2, __ffma2_rn(am, f2(-1.0f), f2(1.0f)));
           if constexpr (COUNT) w_pix += (uint32_t)v0 + (uint32_t)v1;
-          lk0 = v0 ? (int)k : lk0;
-          lk1 = v1 ? (int)k : lk1;
-        };
-        // one saturation test per four entries (1M splats, 8 views of 1920x1080:
-        // 0.986 ms with a test per entry, 0.928 per two, 0.893 per four, no
-        // gain per eight at 69 registers): an entry past a pixel's saturation
-        // gives it alpha 0 and changes nothing
-        uint32_t k = 0;
-        bool sat = false;
-        for (; k + 3 < cnt; k += 4) {
-          blend1(k);
-          blend1(k + 1);
-          blend1(k + 2);
-          blend1(k + 3);
-          if (T2.x < 1e-4f && T2.y < 1e-4f) { sat = true; break; }
-        }
-        if (!sat)
-          for (; k < cnt; ++k) blend1(k);
-        if (lk0 >= 0) last[0] = position(b, (uint32_t)lk0) + 1;
-        if (lk1 >= 0) last[1] = position(b, (uint32_t)lk1) + 1;
-        done[0] = T2.x < 1e-4f;
-        done[1] = T2.y < 1e-4f;
-        T[0] = T2.x; T[1] = T2.y; cr[0] = R2.x; cr[1] = R2.y;
-        cg[0] = G2.x; cg[1] = G2.y; cb[0] = B2.x; cb[1] = B2.y;
-        all_done = done[0] && done[1];
-      } else {
-        for (uint32_t k = 0; k < cnt; ++k) {
-          const float4 ra = sb[3 * k], rb = sb[3 * k + 1], rc = sb[3 * k + 2];
-          const EntryGeom e = entry_geom(fx, ra, rb);
-          all_done = true;
-#pragma unroll
-          for (int q = 0; q < PPT; ++q) {
-            if (!done[q]) {
-              float g, araw, alpha;
-              if (eval_alpha(e, rb.z, __fadd_rn(fy[q], -ra.y), rc.w, g, araw, alpha)) {
-                const float ta = __fmul_rn(T[q], alpha);
-                cr[q] = __fmaf_rn(ta, rc.x, cr[q]);
-                cg[q] = __fmaf_rn(ta, rc.y, cg[q]);
-                cb[q] = __fmaf_rn(ta, rc.z, cb[q]);
-                T[q] = __fmul_rn(T[q], __fadd_rn(1.0f, -alpha));
-                if constexpr (COUNT) ++w_pix;
-                last[q] = position(b, k) + 1;
-                if (T[q] < 1e-4f) done[q] = true;
-              }
-            }
-            all_done &= done[q];
+          if (v0) took[0] |= b;
+          if (v1) took[PPT - 1] |= b;
+        } else {
+          float g, araw, alpha;
+          if (eval_alpha(e, rb.z, __fadd_rn(fy2.x, -ra.y), rc.w, g, araw, alpha) && T2.x >= 1e-4f) {
+            const float ta = __fmul_rn(T2.x, alpha);
+            R2.x = __fmaf_rn(ta, rc.x, R2.x);
+            G2.x = __fmaf_rn(ta, rc.y, G2.x);
+            B2.x = __fmaf_rn(ta, rc.z, B2.x);
+            T2.x = __fmul_rn(T2.x, __fadd_rn(1.0f, -alpha));
+            if constexpr (COUNT) ++w_pix;
+            took[0] |= b;
           }
-          if (all_done) break;
         }
+      };
+      // one saturation test per four entries: an entry past a pixel's
+      // saturation gives it alpha 0 and changes nothing
+      auto saturated = [&]() {
+        return __all_sync(FULL_MASK, T2.x < 1e-4f && (PPT == 1 || T2.y < 1e-4f));
+      };
+      uint32_t i = 0;
+      for (; i + 3 < n; i += 4, sr += 12) {
+        blend(sr, 1u << i);
+        blend(sr + 3, 2u << i);
+        blend(sr + 6, 4u << i);
+        blend(sr + 9, 8u << i);
+        if ((sat = saturated())) break;
       }
+      if (!sat && i < n) {
+        for (; i < n; ++i, sr += 3) blend(sr, 1u << i);
+        sat = saturated();
+      }
+      if constexpr (TAKERS) {
+        uint32_t mine = took[0];
+        if constexpr (PPT == 2) mine |= took[1];
+        const uint32_t m = __reduce_or_sync(FULL_MASK, mine);
+#pragma unroll
+        for (int q = 0; q < PPT; ++q)
+          if (took[q]) last[q] = out.count + __popc(m & (0xFFFFFFFFu >> __clz(took[q])));
+        out.append(m, feed.id()[lane]);
+      } else {
+#pragma unroll
+        for (int q = 0; q < PPT; ++q)
+          if (took[q]) last[q] = feed.pos(31 - __clz(took[q])) + 1;
+      }
+      __syncwarp();  // the stage may be written again
     }
-    if (__syncthreads_count(all_done) == (int)blockDim.x) break;
+    cp_async_wait_all();
+    if constexpr (TAKERS) taken = out.finish(skip);
+    scanned = min(feed.at, begin + len) - begin;
+    staged = feed.qtail;
+    T[0] = T2.x; cr[0] = R2.x; cg[0] = G2.x; cb[0] = B2.x;
+    if constexpr (PPT == 2) { T[1] = T2.y; cr[1] = R2.y; cg[1] = G2.y; cb[1] = B2.y; }
   }
-  cp_async_wait_all();
-  add_work(work, w_scan, w_staged);
+  if constexpr (TAKERS) {
+    if (lane == 0) takers.head[(size_t)vt * n_warps + warp] = taken;
+  }
+  add_tile_work(work, scanned, staged, s_work);
   if constexpr (COUNT) add_pixel_pairs(work, w_pix, sred);
   double sq = 0.0;
 #pragma unroll
   for (int q = 0; q < PPT; ++q) {
     const uint32_t py = py0 + q;
-    if (px < W && py < H) {
+    if (in[q]) {
       const size_t pix = (size_t)v * a.pixels + (size_t)py * a.width + px;
       image[pix] = make_float4(cr[q], cg[q], cb[q], 1.0f - T[q]);
       if (aux) aux[pix] = make_uint2(__float_as_uint(T[q]), last[q]);
@@ -467,17 +673,16 @@ __global__ void __launch_bounds__(256) k_composite(const float4* __restrict__ re
 template <int PPT, int LIST>
 static sc_status composite_ppt(sc_ctx* ctx, const BlendArgs& a, uint32_t grid, uint32_t threads, const float4* rec,
                                const ListArgs& l, float4* image, uint2* aux, const float* target, float gscale,
-                               float4* dl_dc, double* loss, const uint32_t* d_skip, uint64_t* work) {
-  const size_t smem = (size_t)2 * 3 * threads * sizeof(float4) + (size_t)2 * threads * sizeof(uint32_t);
-  BlendArgs ab = a;
-  ab.batch = batch_depth(a.batch, threads);
-  unsigned long long* w = reinterpret_cast<unsigned long long*>(work);
-  if (work && a.count_pairs)
-    k_composite<PPT, LIST, true><<<grid, threads, smem, ctx->stream>>>(rec, l, ab, image, aux, target, gscale, dl_dc,
-                                                                       loss, d_skip, w);
-  else
-    k_composite<PPT, LIST, false><<<grid, threads, smem, ctx->stream>>>(rec, l, ab, image, aux, target, gscale, dl_dc,
-                                                                        loss, d_skip, w);
+                               float4* dl_dc, double* loss, uint32_t* d_skip, uint64_t* work,
+                               const TakerChunks& takers) {
+  const bool count = work && a.count_pairs;
+  auto kern = takers.head ? (count ? k_composite<PPT, LIST, true, true> : k_composite<PPT, LIST, false, true>)
+                          : (count ? k_composite<PPT, LIST, true, false> : k_composite<PPT, LIST, false, false>);
+  const size_t smem = threads / 32 * (sizeof(ListSmem) + (takers.head ? sizeof(TakerRing) : 0));
+  if (smem > 48 * 1024)
+    SC_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
+  kern<<<grid, threads, smem, ctx->stream>>>(rec, l, a, image, aux, target, gscale, dl_dc, loss, d_skip,
+                                             reinterpret_cast<unsigned long long*>(work), takers);
   return sc_check_launch(ctx, "k_composite");
 }
 
@@ -492,10 +697,12 @@ static int pick_ppt(const sc_tiling* tl) {
 template <int LIST>
 static sc_status composite_list(sc_ctx* ctx, const float4* rec, uint32_t stride, uint32_t n_views, const ListArgs& l,
                                 const sc_tiling* tl, float4* image, uint2* aux, const float* target, float mse_scale,
-                                float4* dl_dc, double* loss, const uint32_t* d_skip, uint64_t* work,
-                                uint32_t batch, const SceneDev* scenes, bool count_pairs) {
+                                float4* dl_dc, double* loss, uint32_t* d_skip, uint64_t* work,
+                                uint32_t batch, const SceneDev* scenes, bool count_pairs,
+                                const TakerChunks* takers) {
   BlendArgs a = blend_args(tl, stride);
-  a.batch = batch;
+  // an item list keeps about a quarter of its positions
+  if (batch) a.stage = std::min(std::max(batch / 4, 8u), STAGE) & ~3u;
   a.scenes = scenes;
   a.count_pairs = count_pairs;
   const uint32_t pixels = tl->tile_w * tl->tile_h;
@@ -506,32 +713,35 @@ static sc_status composite_list(sc_ctx* ctx, const float4* rec, uint32_t stride,
   const float gscale = (2.0f / n_scalars) * mse_scale;
   const int ppt = pick_ppt(tl);
   if (ppt == 1 && pixels > 256) return sc_fail(ctx, SC_ERR_INVALID_ARG, "tile too large for one pixel per thread");
-  if (ppt == 2)
-    return composite_ppt<2, LIST>(ctx, a, (uint32_t)grid, pixels / 2, rec, l, image, aux, target, gscale, dl_dc, loss,
-                                  d_skip, work);
-  return composite_ppt<1, LIST>(ctx, a, (uint32_t)grid, pixels, rec, l, image, aux, target, gscale, dl_dc, loss,
-                                d_skip, work);
+  const TakerChunks tk = takers ? *takers : TakerChunks{};
+  return (ppt == 2 ? composite_ppt<2, LIST> : composite_ppt<1, LIST>)(
+      ctx, a, (uint32_t)grid, pixels / ppt, rec, l, image, aux, target, gscale, dl_dc, loss, d_skip, work, tk);
 }
 
 sc_status launch_composite(sc_ctx* ctx, const float4* rec, uint32_t stride, uint32_t n_views, const uint32_t* payloads,
                            const uint32_t* ranges, const sc_tiling* tl, float4* image, uint2* aux, const float* target,
-                           float mse_scale, float4* dl_dc, double* loss, const uint32_t* d_skip) {
+                           float mse_scale, float4* dl_dc, double* loss, uint32_t* d_skip,
+                           const TakerChunks* takers) {
   ListArgs l{payloads, reinterpret_cast<const uint2*>(ranges), nullptr, 0, 0};
   return composite_list<LIST_PAIRS>(ctx, rec, stride, n_views, l, tl, image, aux, target, mse_scale, dl_dc, loss,
-                                    d_skip, nullptr, 0, nullptr, false);
+                                    d_skip, nullptr, 0, nullptr, false, takers);
 }
 
 sc_status launch_composite_items(sc_ctx* ctx, const float4* rec, uint32_t stride, uint32_t n_views,
                                  const uint32_t* item_keys, const uint32_t* item_ids, const uint32_t* item_ranges,
                                  const sc_tiling* tl, float4* image, uint2* aux, const float* target, float mse_scale,
-                                 float4* dl_dc, double* loss, const uint32_t* d_skip, uint64_t* work,
-                                 uint32_t batch, const SceneDev* scenes, bool count_pairs) {
+                                 float4* dl_dc, double* loss, uint32_t* d_skip, uint64_t* work,
+                                 uint32_t batch, const SceneDev* scenes, bool count_pairs,
+                                 const TakerChunks* takers) {
   const BlendArgs a = blend_args(tl, stride);
   ListArgs l{item_ids, reinterpret_cast<const uint2*>(item_ranges), item_keys, (a.tiles_x + SC_SUPER - 1) / SC_SUPER,
              super_tiles_per_view(tl)};
   return composite_list<LIST_ITEMS>(ctx, rec, stride, n_views, l, tl, image, aux, target, mse_scale, dl_dc, loss,
-                                    d_skip, work, batch, scenes, count_pairs);
+                                    d_skip, work, batch, scenes, count_pairs, takers);
 }
+
+// warps per (view, tile) of a blend launch: one takers' head each
+uint32_t blend_warps_per_tile(const sc_tiling* tl) { return tl->tile_w * tl->tile_h / pick_ppt(tl) / 32; }
 
 // ---------------------------------------------------------------- MSE (standalone)
 __global__ void k_mse_views(const float4* __restrict__ pred, const float* __restrict__ target, uint64_t P,
@@ -572,9 +782,9 @@ sc_status launch_mse(sc_ctx* ctx, const float4* pred, const float* target, uint6
 // rs_owner<N>(lane) is the value index that slot totals (-1: a padding
 // slot).  N = 9: 12 shuffles; N = 18: 20.
 template <int N, int O>
-__device__ __forceinline__ float rs_level(const float* x, int lane) {
+__device__ __forceinline__ void rs_half(const float* x, float* y, int lane) {
   constexpr int M = (N + 1) / 2;
-  float y[M], kp[M], rv[M];
+  float kp[M], rv[M];
   const bool bit = lane & O;
 #pragma unroll
   for (int i = 0; i < M; ++i) {
@@ -590,6 +800,12 @@ __device__ __forceinline__ float rs_level(const float* x, int lane) {
     y[i] = t.x; y[i + 1] = t.y;
   }
   if constexpr (M & 1) y[M - 1] = kp[M - 1] + rv[M - 1];
+}
+template <int N, int O>
+__device__ __forceinline__ float rs_level(const float* x, int lane) {
+  constexpr int M = (N + 1) / 2;
+  float y[M];
+  rs_half<N, O>(x, y, lane);
   if constexpr (O == 1) {
     static_assert(M == 1, "at most 32 values");
     return y[0];
@@ -612,10 +828,41 @@ __device__ __forceinline__ int rs_owner(int lane) {
   return len >= 1 ? lo : -1;
 }
 
-// Entries per warp reduction: 2 (an 18-value reduce-scatter, 20 shuffles for
-// two entries).  3 entries (27 values, 28 shuffles) measured slower at 80
-// registers; more than 3 do not fit the 32 lanes.
+// Entries per warp reduction of the general path: 2 (an 18-value
+// reduce-scatter, 20 shuffles for two entries).  3 entries (27 values, 28
+// shuffles) measured slower at 80 registers; more than 3 do not fit the 32
+// lanes.
 constexpr int RS_E = 2;
+
+// Octet reduction (two pixels per thread, tile width a multiple of 8: the 8
+// lanes of an octet own 8 consecutive columns of one row pair).  While a warp
+// walks its entries, each lane writes its two pixels' h and T alpha of an entry
+// that some pixel of the warp takes into one row of a warp-private shared
+// buffer; every OCT_E rows the warp turns round: lane (q, e) sums entry e over
+// the 8 columns and 2 rows of octet q, in packed f32x2 over the two rows, so
+// the 64-pixel sums of 9 quantities cost 8 row loads and 7 packed operations a
+// column for 8 entries at once, and the four octets' partial sums meet in a
+// two-level reduce-scatter (8 shuffles for 8 entries).  Per entry and warp that
+// is about 17 instructions instead of the about 50 of the reduce-scatter over
+// all 32 lanes.  A row is padded by one float4, so both the rows' stores and
+// the turned loads (8 lanes, 8 rows, one column) touch all banks once.
+constexpr int OCT_E = 8;
+constexpr int OCT_ROW = 33;  // float4 per row: 32 lanes and the pad
+
+// shared memory of one backward warp
+struct OctSmem {
+  float4 row[OCT_E * OCT_ROW];
+  float4 rg[36];  // dL/dC red and green of a lane's two pixels; octet q at 9 q
+  float2 b[36];   // blue
+};
+struct SumSmem {
+  float sum[20];  // a reduce-scatter's 18 totals
+};
+template <typename FEED, bool OCT>
+struct BwdSmem {
+  typename FEED::Smem feed;
+  typename std::conditional<OCT, OctSmem, SumSmem>::type red;
+};
 
 // Compensated accumulation of x into the sum *s, the rounding error of the
 // addition going to *c: the atomic returns the old sum, the device forms the
@@ -647,7 +894,11 @@ __device__ __forceinline__ void twosum_atomic_add4(float4* s, float4* c, float4 
 // here from the forward image instead of being read from dl_dc.
 // COMP: the per-(view, splat) totals across tiles are accumulated with
 // twosum_atomic_add into proj_grad and the compensation records proj_comp.
-template <int PPT, int MODE, int LIST, bool COMP, bool COUNT>
+// OCT: the octet reduction (PPT 2 and a tile width that is a multiple of 8).
+// LIST_TAKERS: exact mode over the entries that the forward wrote down per warp.
+// A warp sends its sums of an entry to global memory itself, one float4 atomic
+// per part of the entry's record.
+template <int PPT, int MODE, int LIST, bool COMP, bool COUNT, bool OCT>
 __global__ void __launch_bounds__(256) k_composite_backward(const float4* __restrict__ rec, ListArgs l, BlendArgs a,
                                                             const float4* __restrict__ fwd,
                                                             const float4* __restrict__ dl_dc,
@@ -657,17 +908,16 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
                                                             float4* __restrict__ proj_grad,
                                                             const uint32_t* __restrict__ skip,
                                                             unsigned long long* __restrict__ work,
-                                                            float4* __restrict__ proj_comp) {
-  // records [2][B][3], acc [B][3] (float4), ids [2][B], item positions [2][B] (u32)
-  extern __shared__ float4 sbuf[];
-  __shared__ uint32_t s_max;
+                                                            float4* __restrict__ proj_comp, TakerChunks takers) {
+  static_assert(!OCT || PPT == 2, "the octet reduction takes two pixels per thread");
+  static_assert(LIST != LIST_TAKERS || MODE == SC_BWD_EXACT, "the takers are the exact mode's entries");
+  using FEED = typename std::conditional<LIST == LIST_TAKERS, TakerFeed, ListFeed<LIST, true>>::type;
+  extern __shared__ float4 sbuf[];  // one BwdSmem per warp
   __shared__ double s_red[8];
-  __shared__ uint32_t s_wcnt[2][8];
-  if (skip && (*skip & SC_DEVERR_CAPACITY)) return;
-  const uint32_t B = a.batch;
-  float4* sacc = sbuf + (size_t)6 * B;
-  uint32_t* sids = reinterpret_cast<uint32_t*>(sbuf + (size_t)9 * B);
-  uint32_t* spos = sids + 2 * B;
+  __shared__ uint32_t s_work[2];
+  if (skip && (*skip & SC_DEVERR_SKIP)) return;
+  const uint32_t warp = threadIdx.x >> 5;
+  BwdSmem<FEED, OCT>& sm = reinterpret_cast<BwdSmem<FEED, OCT>*>(sbuf)[warp];
   const uint32_t vt = blockIdx.x;
   const uint32_t v = vt / a.num_tiles, tile = vt - v * a.num_tiles;
   const uint32_t ty = tile / a.tiles_x, tx = tile - ty * a.tiles_x;
@@ -677,9 +927,16 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
   uint32_t W, H;
   float gs;
   view_dims(a, v, gscale, W, H, gs);
-  uint32_t bit;
-  const uint2 r = list_range<LIST>(l, a, v, tx, ty, tile, bit);
-  const uint32_t begin = r.x, end = r.y > r.x ? r.y : r.x;
+  uint32_t begin = 0, len = 0, bit = 0;
+  uint2 head = make_uint2(0u, 0u);
+  if constexpr (LIST == LIST_TAKERS) {
+    head = takers.head[(size_t)vt * (blockDim.x >> 5) + warp];
+    len = head.y;
+  } else {
+    const uint2 r = list_range<LIST>(l, a, v, tx, ty, tile, bit);
+    begin = r.x;
+    len = r.y > r.x ? r.y - r.x : 0u;
+  }
   const float4* vrec = rec + (size_t)3 * v * a.stride;
   float4* vgrad = proj_grad + (size_t)3 * v * a.stride;
 
@@ -688,7 +945,7 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
   float T[PPT], gr[PPT], gg[PPT], gb[PPT], GS[PPT], fy[PPT];
   uint32_t stop[PPT];
   bool done[PPT];
-  uint32_t tstop = begin;
+  uint32_t tstop = 0;
   bool all_done = true;
   double sq = 0.0;
 #pragma unroll
@@ -696,7 +953,7 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
     const uint32_t py = py0 + q;
     fy[q] = (float)py + 0.5f;
     T[q] = 1.0f; gr[q] = gg[q] = gb[q] = 0.f; GS[q] = 0.f;
-    stop[q] = begin;
+    stop[q] = 0;
     done[q] = !(px < W && py < H);
     if (!done[q]) {
       const size_t pix = (size_t)v * a.pixels + (size_t)py * a.width + px;
@@ -711,11 +968,11 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
       }
       if (MODE == SC_BWD_REF) {
         T[q] = 1.0f - c.w;
-        stop[q] = end;
+        stop[q] = len;
       } else {
         const uint2 x = aux[pix];
         T[q] = __uint_as_float(x.x);
-        stop[q] = begin + min(x.y, end - begin);
+        stop[q] = min(x.y, len);
       }
       tstop = max(tstop, stop[q]);
     }
@@ -725,255 +982,230 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
     const double sum = block_sum(sq, s_red);
     if (threadIdx.x == 0 && sum != 0.0) atomicAdd(&loss[v], sum);
   }
-  if (end <= begin) return;
-  if (threadIdx.x == 0) s_max = begin;
-  if (threadIdx.x < B) {
-    sacc[3 * threadIdx.x] = make_float4(0, 0, 0, 0);
-    sacc[3 * threadIdx.x + 1] = make_float4(0, 0, 0, 0);
-    sacc[3 * threadIdx.x + 2] = make_float4(0, 0, 0, 0);
-  }
-  __syncthreads();
-  if (tstop > begin) atomicMax(&s_max, tstop);
-  __syncthreads();
-  const uint32_t hi0 = s_max;
-  if (hi0 <= begin) return;
-  const uint32_t nb = (hi0 - begin + B - 1) / B;
-  // batch b: list positions [hi - min(B, hi - begin), hi), hi = hi0 - b B
-  auto fetch = [&](uint32_t b) -> ListWord {
-    const uint32_t hi = hi0 - b * B, lo = hi - min(B, hi - begin);
-    return fetch_list<LIST>(l, lo, hi);
-  };
-  auto place = [&](uint32_t b, const ListWord& f) -> uint32_t {
-    const uint32_t hi = hi0 - b * B, lo = hi - min(B, hi - begin);
-    return place_list<LIST>(f, hi - lo, vrec, bit, begin, sbuf + (size_t)(b & 1) * 3 * B, spos + (b & 1) * B,
-                            sids + (b & 1) * B, s_wcnt[b & 1]);
-  };
-
-  const int lane = threadIdx.x & 31;
-  // after the 18-value reduce-scatter of entries (k, k - 1) this lane adds one
-  // value: of entry k - rs_ent, at float rs_off of its 3 float4 slot (w unused)
-  const int rs_idx = rs_owner<9 * RS_E>(lane);
-  const int rs_ent = rs_idx / 9;
-  const int rs_off = rs_idx >= 0 ? rs_idx % 9 + (rs_idx % 9) / 3 : -1;
-  ListWord f = fetch(0);
-  uint32_t cnt_next = place(0, f);
-  if (nb > 1) f = fetch(1);
-  uint32_t w_staged = 0, w_pix = 0;
-  for (uint32_t b = 0; b < nb; ++b) {
-    const uint32_t cnt = cnt_next;
-    w_staged += cnt;
-    if (b + 1 < nb) {
-      cnt_next = place(b + 1, f);
-      if (b + 2 < nb) f = fetch(b + 2);
-      cp_async_wait_one();
-    } else {
-      cp_async_wait_all();
+  // the walk starts at the warp's last contributor
+  const uint32_t hi0 = __reduce_max_sync(FULL_MASK, tstop);
+  uint32_t staged = 0, w_pix = 0;
+  if (hi0 > 0) {
+    const int lane = threadIdx.x & 31;
+    // general path: after the 18-value reduce-scatter of two entries this lane
+    // holds one value: value rs_idx % 9 of entry rs_idx / 9
+    const int rs_idx = rs_owner<9 * RS_E>(lane);
+    // octet reduction: this lane turns to entry row oe of octet oq, and holds
+    // after the two levels the three sums of part oq of that entry's gradient
+    const int oe = lane & 7, oq = lane >> 3;
+    const float fx_oct = fx - (float)oe;  // the octet's first column (the lane's own octet is oq)
+    if constexpr (OCT) {  // warp-private: read after the __syncwarp of the first turn
+      sm.red.rg[oq * 9 + oe] = make_float4(gr[0], gr[PPT - 1], gg[0], gg[PPT - 1]);
+      sm.red.b[oq * 9 + oe] = make_float2(gb[0], gb[PPT - 1]);
     }
-    __syncthreads();
-    const uint32_t hi = hi0 - b * B;
-    const uint32_t lo = hi - min(B, hi - begin);
-    const uint32_t* bpos = spos + (b & 1) * B;
-    const float4* sb = sbuf + (size_t)(b & 1) * 3 * B;
-    if (!__all_sync(FULL_MASK, all_done)) {
-      float2 T2 = make_float2(T[0], T[PPT - 1]), GS2 = make_float2(GS[0], GS[PPT - 1]);
-      const float2 gr2 = make_float2(gr[0], gr[PPT - 1]), gg2 = make_float2(gg[0], gg[PPT - 1]);
-      const float2 gb2 = make_float2(gb[0], gb[PPT - 1]), fy2 = make_float2(fy[0], fy[PPT - 1]);
-      // one entry: this thread's raw sums of it into c[0..8] (zeros when none of
-      // its pixels takes part); returns whether one does
-      auto entry = [&](int k, float* c) -> bool {
-          const uint32_t j = LIST == LIST_PAIRS ? lo + (uint32_t)k : begin + bpos[k];
-          // this thread's sums over its pixels: h = dL/dalpha * gauss (the opacity
-          // gradient), its first and second moments in (dx, dy), and the colour
-          // gradient; the per-splat terms are formed from them once per entry
-          float sh = 0.f, shx = 0.f, shy = 0.f, shxx = 0.f, shxy = 0.f, shyy = 0.f;
-          float scr = 0.f, scg = 0.f, scb = 0.f;
-          bool contrib = false;
-          const float4 ra = sb[3 * k], rb = sb[3 * k + 1], rc = sb[3 * k + 2];
-          const EntryGeom e = entry_geom(fx, ra, rb);
-          if constexpr (PPT == 2) {
-            // both pixels in packed arithmetic; a pixel that skips the splat gets
-            // zero alpha and weight, so it adds nothing and keeps its T
-            float2 dy, g, araw, al;
-            bool v0, v1;
-            eval_alpha2(e, rb.z, fy2, ra.y, rc.w, dy, g, araw, al, v0, v1);
-            v0 &= (MODE == SC_BWD_EXACT || !done[0]) && j < stop[0];
-            v1 &= (MODE == SC_BWD_EXACT || !done[1]) && j < stop[1];
-            // the exact mode takes no branch here: with both pixels skipping, every
-            // sum below is zero and T and GS keep their values
-            if (MODE == SC_BWD_REF ? (v0 || v1) : true) {
-              const float2 oma = __fadd2_rn(f2(1.0f), make_float2(-al.x, -al.y));
-              const float2 inv = make_float2(rcp_approx(oma.x), rcp_approx(oma.y));
-              const float2 Tn = __fmul2_rn(T2, inv);  // T_i = T_{i+1} / (1 - alpha_i)
-              if (MODE == SC_BWD_REF) {
-                if (v0 && Tn.x > 1.0001f) { done[0] = true; v0 = false; }
-                if (v1 && Tn.y > 1.0001f) { done[1] = true; v1 = false; }
-              }
-              if (MODE == SC_BWD_REF ? (v0 || v1) : true) {
-                const float2 am = make_float2(v0 ? al.x : 0.0f, v1 ? al.y : 0.0f);
-                const float2 gm = make_float2(v0 && araw.x < ALPHA_MAX ? g.x : 0.0f,
-                                              v1 && araw.y < ALPHA_MAX ? g.y : 0.0f);
-                const float2 ta = __fmul2_rn(Tn, am);
-                const float2 p = __fmul2_rn(ta, gr2), q = __fmul2_rn(ta, gg2), w = __fmul2_rn(ta, gb2);
-                scr = p.x + p.y; scg = q.x + q.y; scb = w.x + w.y;
-                // dC/dalpha = T_i c - S / (1 - alpha) = (T_{i+1} c - S) / (1 - alpha)
-                const float2 dc = __ffma2_rn(gb2, f2(rc.z), __ffma2_rn(gg2, f2(rc.y), __fmul2_rn(gr2, f2(rc.x))));
-                const float2 galpha = __fmul2_rn(inv, __ffma2_rn(T2, dc, make_float2(-GS2.x, -GS2.y)));
-                const float2 h = __fmul2_rn(galpha, gm);
-                const float2 hy = __fmul2_rn(h, dy);
-                sh = h.x + h.y;
-                shy = hy.x + hy.y;
-                shyy = fmaf(hy.x, dy.x, hy.y * dy.y);
-                shx = sh * e.dx;  // both pixels share dx
-                shxx = shx * e.dx;
-                shxy = shy * e.dx;
-                GS2 = __ffma2_rn(ta, dc, GS2);
-                T2 = make_float2(v0 ? Tn.x : T2.x, v1 ? Tn.y : T2.y);
-                if constexpr (COUNT) w_pix += (uint32_t)v0 + (uint32_t)v1;
-                contrib = v0 || v1;
-              }
-            }
-            if (MODE == SC_BWD_REF) all_done = (done[0] || j <= begin) && (done[1] || j <= begin);
-          } else {
-            all_done = true;
-  #pragma unroll
-            for (int q = 0; q < PPT; ++q) {
-              if ((MODE == SC_BWD_EXACT || !done[q]) && j < stop[q]) {
-                const float dy = __fadd_rn(fy[q], -ra.y);
-                float g, araw, alpha;
-                if (eval_alpha(e, rb.z, dy, rc.w, g, araw, alpha)) {
-                  const float inv = rcp_approx(__fadd_rn(1.0f, -alpha));
-                  const float Tn = __fmul_rn(T[q], inv);  // T_i = T_{i+1} / (1 - alpha_i)
-                  if (MODE == SC_BWD_REF && Tn > 1.0001f) {
-                    done[q] = true;
-                  } else {
-                    const float ta = __fmul_rn(Tn, alpha);
-                    scr += gr[q] * ta; scg += gg[q] * ta; scb += gb[q] * ta;
-                    const float dc = gr[q] * rc.x + gg[q] * rc.y + gb[q] * rc.z;
-                    const float galpha = inv * (T[q] * dc - GS[q]);
-                    const float h = araw < ALPHA_MAX ? galpha * g : 0.0f;
-                    const float hx = h * e.dx, hy = h * dy;
-                    sh += h;
-                    shx += hx; shy += hy;
-                    shxx += hx * e.dx; shxy += hx * dy; shyy += hy * dy;
-                    GS[q] += ta * dc;
-                    T[q] = Tn;
-                    if constexpr (COUNT) ++w_pix;
-                    contrib = true;
-                  }
-                }
-              }
-              if (MODE == SC_BWD_REF) all_done &= done[q] || j <= begin;
+    FEED feed = [&]() {
+      if constexpr (LIST == LIST_TAKERS) return TakerFeed(sm.feed, takers, vrec, head);
+      else return ListFeed<LIST, true>(sm.feed, l, vrec, begin, hi0, bit, STAGE);
+    }();
+    // part `part` of the gradient record of the stage's entry i, from its sums m
+    // over the warp's pixels of h = dL/dalpha * gauss and its moments in (dx,
+    // dy): with the splat's opacity and conic (a, b, c)
+    // (rasterize_backward.wgsl:174-185) dpower = op h, dmean = dpower (a dx +
+    // b dy, b dx + c dy), dconic = dpower (-1/2)(dx^2, 2 dx dy, dy^2); the
+    // opacity and colour gradients are the sums themselves
+    auto send = [&](uint32_t i, int part, float3 m) {
+      float4 g = make_float4(m.x, m.y, m.z, 0.0f);
+      if (part < 2) {
+        const float4 cb = feed.rec()[3 * i + 1];
+        const float op = feed.rec()[3 * i + 2].w;
+        if (part == 0) {
+          g.x = op * (cb.x * m.x + cb.y * m.y);
+          g.y = op * (cb.y * m.x + cb.z * m.y);
+        } else {
+          g.x = -0.5f * op * m.x; g.y = -op * m.y; g.z = -0.5f * op * m.z;
+        }
+      }
+      const size_t o = (size_t)3 * feed.id()[i] + part;
+      if constexpr (COMP)
+        twosum_atomic_add4(vgrad + o, proj_comp + (size_t)3 * v * a.stride + o, g);
+      else if (g.x != 0.f || g.y != 0.f || g.z != 0.f)
+        atomicAdd(vgrad + o, g);
+    };
+    float2 T2 = make_float2(T[0], T[PPT - 1]), NG2 = f2(0.f);  // NG = -GS
+    const float2 gr2 = make_float2(gr[0], gr[PPT - 1]), gg2 = make_float2(gg[0], gg[PPT - 1]);
+    const float2 gb2 = make_float2(gb[0], gb[PPT - 1]), fy2 = make_float2(fy[0], fy[PPT - 1]);
+    bool stopped = false;
+    // octet path: a thread's two pixels' (h, -T alpha) of entry i (zeros where a
+    // pixel skips it).  Alpha is carried negated, which needs no negations in
+    // the packed operations; a skipping pixel gets alpha 0, so it keeps its T
+    // (1 / 1 is exact) and its sums.
+    auto entry2 = [&](uint32_t i, const float4* r) -> float4 {
+      const uint32_t j = feed.pos(i);
+      const float4 ra = r[0], rb = r[1], rc = r[2];
+      const EntryGeom e = entry_geom(fx, ra, rb);
+      float2 dy, g, araw, al;
+      bool v0, v1;
+      eval_alpha2(e, rb.z, fy2, ra.y, rc.w, dy, g, araw, al, v0, v1);
+      v0 &= (MODE == SC_BWD_EXACT || !done[0]) && j < stop[0];
+      v1 &= (MODE == SC_BWD_EXACT || !done[PPT - 1]) && j < stop[PPT - 1];
+      float2 am = make_float2(v0 ? -al.x : 0.0f, v1 ? -al.y : 0.0f);
+      const float2 oma = __fadd2_rn(f2(1.0f), am);
+      const float2 inv = make_float2(rcp_approx(oma.x), rcp_approx(oma.y));
+      float2 Tn = __fmul2_rn(T2, inv);  // T_i = T_{i+1} / (1 - alpha_i)
+      if (MODE == SC_BWD_REF) {
+        if (v0 && Tn.x > 1.0001f) { done[0] = true; v0 = false; am.x = 0.0f; Tn.x = T2.x; }
+        if (v1 && Tn.y > 1.0001f) { done[PPT - 1] = true; v1 = false; am.y = 0.0f; Tn.y = T2.y; }
+      }
+      const float2 gm = make_float2(v0 && araw.x < ALPHA_MAX ? g.x : 0.0f, v1 && araw.y < ALPHA_MAX ? g.y : 0.0f);
+      const float2 ta = __fmul2_rn(Tn, am);
+      // dC/dalpha = T_i c - S / (1 - alpha) = (T_{i+1} c - S) / (1 - alpha)
+      const float2 dc = make_float2(fmaf(gb2.x, rc.z, fmaf(gg2.x, rc.y, gr2.x * rc.x)),
+                                    fmaf(gb2.y, rc.z, fmaf(gg2.y, rc.y, gr2.y * rc.x)));
+      const float2 h = __fmul2_rn(__fmul2_rn(inv, __ffma2_rn(T2, dc, NG2)), gm);
+      NG2 = __ffma2_rn(ta, dc, NG2);
+      T2 = Tn;
+      if constexpr (COUNT) w_pix += (uint32_t)v0 + (uint32_t)v1;
+      if (MODE == SC_BWD_REF) all_done = (done[0] || j == 0) && (done[PPT - 1] || j == 0);
+      return make_float4(h.x, h.y, ta.x, ta.y);
+    };
+    // turn round: the sums of entries i0 .. i0 + rows - 1 over the warp's pixels, and out
+    auto turn = [&](uint32_t i0, uint32_t rows) {
+      if constexpr (OCT) {
+        __syncwarp();
+        const float4* w = sm.red.row + oe * OCT_ROW + oq * 8;
+        const float4 m = feed.rec()[3 * (i0 + oe)];
+        float2 sh = f2(0.f), shx = sh, shxx = sh, cr = sh, cg = sh, cb = sh;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) {
+          const float4 x = w[j], rg = sm.red.rg[oq * 9 + j];
+          const float2 b = sm.red.b[oq * 9 + j], h = make_float2(x.x, x.y), ta = make_float2(x.z, x.w);
+          const float2 dx = f2(__fadd_rn(fx_oct + (float)j, -m.x));
+          const float2 hx = __fmul2_rn(h, dx);
+          sh = __fadd2_rn(sh, h);
+          shx = __fadd2_rn(shx, hx);
+          shxx = __ffma2_rn(hx, dx, shxx);
+          cr = __ffma2_rn(ta, make_float2(rg.x, rg.y), cr);
+          cg = __ffma2_rn(ta, make_float2(rg.z, rg.w), cg);
+          cb = __ffma2_rn(ta, b, cb);
+        }
+        const float2 dy = __fadd2_rn(fy2, f2(-m.y));
+        const float2 hy = __fmul2_rn(sh, dy), hxy = __fmul2_rn(shx, dy);
+        const float c[12] = {shx.x + shx.y,   hy.x + hy.y,   sh.x + sh.y,
+                             shxx.x + shxx.y, hxy.x + hxy.y, fmaf(hy.x, dy.x, hy.y * dy.y),
+                             -(cr.x + cr.y),  -(cg.x + cg.y), -(cb.x + cb.y), 0.f, 0.f, 0.f};
+        float c6[6], c3[3];
+        rs_half<12, 16>(c, c6, lane);
+        rs_half<6, 8>(c6, c3, lane);
+        if (oe < rows && oq < 3) send(i0 + oe, oq, make_float3(c3[0], c3[1], c3[2]));
+        __syncwarp();  // the rows may be written again
+      }
+    };
+    // general path: this thread's raw sums of entry i over its pixels into
+    // c[0..8]: h = dL/dalpha * gauss (the opacity gradient), its first and second
+    // moments in (dx, dy), and the colour gradient
+    auto entry = [&](uint32_t i, const float4* r, float* c) {
+      const uint32_t j = feed.pos(i);
+      const float4 ra = r[0], rb = r[1], rc = r[2];
+      const EntryGeom e = entry_geom(fx, ra, rb);
+      all_done = true;
+#pragma unroll
+      for (int q = 0; q < PPT; ++q) {
+        float& Tq = q ? T2.y : T2.x;
+        float& ng = q ? NG2.y : NG2.x;
+        if ((MODE == SC_BWD_EXACT || !done[q]) && j < stop[q]) {
+          const float dy = __fadd_rn(fy[q], -ra.y);
+          float g, araw, alpha;
+          if (eval_alpha(e, rb.z, dy, rc.w, g, araw, alpha)) {
+            const float inv = rcp_approx(__fadd_rn(1.0f, -alpha));
+            const float Tn = __fmul_rn(Tq, inv);  // T_i = T_{i+1} / (1 - alpha_i)
+            if (MODE == SC_BWD_REF && Tn > 1.0001f) {
+              done[q] = true;
+            } else {
+              const float ta = __fmul_rn(Tn, alpha);
+              c[6] += gr[q] * ta; c[7] += gg[q] * ta; c[8] += gb[q] * ta;
+              const float dc = gr[q] * rc.x + gg[q] * rc.y + gb[q] * rc.z;
+              const float galpha = inv * (Tq * dc + ng);
+              const float h = araw < ALPHA_MAX ? galpha * g : 0.0f;
+              const float hx = h * e.dx, hy = h * dy;
+              c[0] += hx; c[1] += hy; c[2] += h;
+              c[3] += hx * e.dx; c[4] += hx * dy; c[5] += hy * dy;
+              ng -= ta * dc;
+              Tq = Tn;
+              if constexpr (COUNT) ++w_pix;
             }
           }
-        c[0] = shx; c[1] = shy; c[2] = sh; c[3] = shxx; c[4] = shxy; c[5] = shyy;
-        c[6] = scr; c[7] = scg; c[8] = scb;
-        return contrib;
-      };
-      // entries k .. k - RS_E + 1 together: one 9 RS_E-value reduce-scatter
-      for (int k = (int)cnt - 1; k >= 0; k -= RS_E) {
-        float c[9 * RS_E];
-        bool any = false;
-#pragma unroll
-        for (int q = 0; q < RS_E; ++q) {
-          if (k - q >= 0) {
-            any |= entry(k - q, c + 9 * q);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 9; ++i) c[9 * q + i] = 0.0f;
-          }
         }
-        if (MODE == SC_BWD_EXACT) all_done = false;
-        if (__any_sync(FULL_MASK, any)) {
-          // the splats' raw sums; the flush turns them into their gradients
-          const float w = warp_reduce_scatter<9 * RS_E>(c, lane);
-          if (rs_off >= 0 && k >= rs_ent) atomicAdd(reinterpret_cast<float*>(sacc + 3 * (k - rs_ent)) + rs_off, w);
+        if (MODE == SC_BWD_REF) all_done &= done[q] || j == 0;
+      }
+    };
+    const WarpRect rect = LIST == LIST_TAKERS ? WarpRect{} : warp_rect(px, py0, PPT);
+    for (uint32_t n_raw = feed.gather(); n_raw > 0 && !stopped;) {
+      const uint32_t n = feed.ready(n_raw, rect);
+      n_raw = feed.gather();
+      const float4* sr = feed.rec();
+      staged += n;
+      uint32_t i = 0;
+      if constexpr (OCT) {
+        float4* row = sm.red.row + lane;
+        for (; i + OCT_E <= n && !stopped; i += OCT_E) {
+#pragma unroll 4
+          for (int e = 0; e < OCT_E; ++e) row[e * OCT_ROW] = entry2(i + e, sr + 3 * (i + e));
+          turn(i, OCT_E);
+          if (MODE == SC_BWD_REF) stopped = __all_sync(FULL_MASK, all_done);
         }
-        if (MODE == SC_BWD_REF && __all_sync(FULL_MASK, all_done)) break;
-      }
-      if constexpr (PPT == 2) {
-        T[0] = T2.x; T[1] = T2.y; GS[0] = GS2.x; GS[1] = GS2.y;
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x < cnt) {
-      // the entry's sums over the CTA's pixels of h = dL/dalpha * gauss and its
-      // moments in (dx, dy) become, with the splat's opacity and conic (a, b, c)
-      // (rasterize_backward.wgsl:174-185): dpower = op h, dmean = dpower (a dx +
-      // b dy, b dx + c dy), dconic = dpower (-1/2)(dx^2, 2 dx dy, dy^2); the
-      // opacity and colour gradients are the sums themselves
-      float4* acc = sacc + 3 * threadIdx.x;
-      const float4 m0 = acc[0], m1 = acc[1], a2 = acc[2];  // (SHX, SHY, SH), (SHXX, SHXY, SHYY), colour
-      const float4 cb = sb[3 * threadIdx.x + 1];
-      const float op = sb[3 * threadIdx.x + 2].w;
-      const float4 a0 = make_float4(op * (cb.x * m0.x + cb.y * m0.y), op * (cb.y * m0.x + cb.z * m0.y), m0.z, 0.0f);
-      const float4 a1 = make_float4(-0.5f * op * m1.x, -op * m1.y, -0.5f * op * m1.z, 0.0f);
-      const uint32_t id = sids[(b & 1) * B + threadIdx.x];
-      float4* dst = vgrad + (size_t)3 * id;
-      if constexpr (COMP) {
-        float4* cdst = proj_comp + (size_t)3 * v * a.stride + (size_t)3 * id;
-        twosum_atomic_add4(dst, cdst, a0);
-        twosum_atomic_add4(dst + 1, cdst + 1, a1);
-        twosum_atomic_add4(dst + 2, cdst + 2, a2);
+        if (i < n && !stopped) {
+          for (uint32_t e = 0; i + e < n; ++e) row[e * OCT_ROW] = entry2(i + e, sr + 3 * (i + e));
+          turn(i, n - i);
+          if (MODE == SC_BWD_REF) stopped = __all_sync(FULL_MASK, all_done);
+        }
       } else {
-        if (a0.x != 0.f || a0.y != 0.f || a0.z != 0.f) atomicAdd(dst, a0);
-        if (a1.x != 0.f || a1.y != 0.f || a1.z != 0.f) atomicAdd(dst + 1, a1);
-        if (a2.x != 0.f || a2.y != 0.f || a2.z != 0.f) atomicAdd(dst + 2, a2);
+        // two entries together: one 18-value reduce-scatter
+        for (; i < n && !stopped; i += 2) {
+          const bool two = i + 1 < n;
+          float c[9 * RS_E];
+#pragma unroll
+          for (int q = 0; q < 9 * RS_E; ++q) c[q] = 0.0f;
+          entry(i, sr + 3 * i, c);
+          if (two) entry(i + 1, sr + 3 * i + 3, c + 9);
+          const float w = warp_reduce_scatter<9 * RS_E>(c, lane);
+          if (rs_idx >= 0) sm.red.sum[rs_idx] = w;
+          __syncwarp();
+          if (lane < (two ? 6 : 3)) {
+            const float* m = sm.red.sum + 3 * lane;
+            send(i + lane / 3, lane % 3, make_float3(m[0], m[1], m[2]));
+          }
+          __syncwarp();
+          if (MODE == SC_BWD_REF) stopped = __all_sync(FULL_MASK, all_done);
+        }
       }
-      acc[0] = make_float4(0, 0, 0, 0); acc[1] = acc[0]; acc[2] = acc[0];
+      __syncwarp();  // the stage may be written again
     }
-    if (__syncthreads_count(all_done) == (int)blockDim.x) break;
+    cp_async_wait_all();
   }
-  cp_async_wait_all();
-  add_work(work, hi0 - begin, w_staged);
+  add_tile_work(work, hi0, staged, s_work);
   if constexpr (COUNT) add_pixel_pairs(work, w_pix, s_red);
 }
 
-template <int PPT, int LIST, int MODE>
-static void backward_launch(const BlendArgs& a, uint32_t grid, uint32_t threads, size_t smem, cudaStream_t st,
-                            const float4* rec, const ListArgs& l, const float4* fwd, const float4* dl_dc,
-                            const float* target, float gscale, double* loss, const uint2* aux, float4* proj_grad,
-                            const uint32_t* d_skip, unsigned long long* w, float4* proj_comp) {
-  const bool count = w && a.count_pairs;
-  if (proj_comp && count)
-    k_composite_backward<PPT, MODE, LIST, true, true><<<grid, threads, smem, st>>>(
-        rec, l, a, fwd, dl_dc, target, gscale, loss, aux, proj_grad, d_skip, w, proj_comp);
-  else if (proj_comp)
-    k_composite_backward<PPT, MODE, LIST, true, false><<<grid, threads, smem, st>>>(
-        rec, l, a, fwd, dl_dc, target, gscale, loss, aux, proj_grad, d_skip, w, proj_comp);
-  else if (count)
-    k_composite_backward<PPT, MODE, LIST, false, true><<<grid, threads, smem, st>>>(
-        rec, l, a, fwd, dl_dc, target, gscale, loss, aux, proj_grad, d_skip, w, nullptr);
-  else
-    k_composite_backward<PPT, MODE, LIST, false, false><<<grid, threads, smem, st>>>(
-        rec, l, a, fwd, dl_dc, target, gscale, loss, aux, proj_grad, d_skip, w, nullptr);
-}
-
-template <int PPT, int LIST>
+template <int PPT, int LIST, int MODE, bool OCT>
 static sc_status backward_ppt(sc_ctx* ctx, const BlendArgs& a, uint32_t grid, uint32_t threads, const float4* rec,
                               const ListArgs& l, const float4* fwd, const float4* dl_dc, const float* target,
-                              float gscale, double* loss, int mode, const uint2* aux, float4* proj_grad,
-                              const uint32_t* d_skip, uint64_t* work, float4* proj_comp) {
-  const size_t smem = (size_t)9 * threads * sizeof(float4) + (size_t)4 * threads * sizeof(uint32_t);
-  unsigned long long* w = reinterpret_cast<unsigned long long*>(work);
-  BlendArgs ab = a;
-  ab.batch = batch_depth(a.batch, threads);
-  if (mode == SC_BWD_EXACT)
-    backward_launch<PPT, LIST, SC_BWD_EXACT>(ab, grid, threads, smem, ctx->stream, rec, l, fwd, dl_dc, target, gscale,
-                                             loss, aux, proj_grad, d_skip, w, proj_comp);
-  else
-    backward_launch<PPT, LIST, SC_BWD_REF>(ab, grid, threads, smem, ctx->stream, rec, l, fwd, dl_dc, target, gscale,
-                                           loss, aux, proj_grad, d_skip, w, proj_comp);
+                              float gscale, double* loss, const uint2* aux, float4* proj_grad,
+                              const uint32_t* d_skip, uint64_t* work, float4* proj_comp, const TakerChunks& takers) {
+  using FEED = typename std::conditional<LIST == LIST_TAKERS, TakerFeed, ListFeed<LIST, true>>::type;
+  const bool count = work && a.count_pairs;
+  auto kern = proj_comp ? (count ? k_composite_backward<PPT, MODE, LIST, true, true, OCT>
+                                 : k_composite_backward<PPT, MODE, LIST, true, false, OCT>)
+                        : (count ? k_composite_backward<PPT, MODE, LIST, false, true, OCT>
+                                 : k_composite_backward<PPT, MODE, LIST, false, false, OCT>);
+  const size_t smem = threads / 32 * sizeof(BwdSmem<FEED, OCT>);
+  if (smem > 48 * 1024)
+    SC_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
+  kern<<<grid, threads, smem, ctx->stream>>>(rec, l, a, fwd, dl_dc, target, gscale, loss, aux, proj_grad, d_skip,
+                                             reinterpret_cast<unsigned long long*>(work), proj_comp, takers);
   return sc_check_launch(ctx, "k_composite_backward");
 }
 
-template <int LIST>
-static sc_status backward_list(sc_ctx* ctx, const float4* rec, uint32_t stride, uint32_t n_views, const ListArgs& l,
-                               const sc_tiling* tl, const float4* fwd, const float4* dl_dc, const float* target,
-                               float mse_scale, double* loss, int mode, const uint2* aux, float4* proj_grad,
-                               const uint32_t* d_skip, uint64_t* work, float4* proj_comp, uint32_t batch,
-                               const SceneDev* scenes, bool count_pairs) {
+static sc_status backward_list(sc_ctx* ctx, const float4* rec, uint32_t stride, uint32_t n_views, int list,
+                               const ListArgs& l, const sc_tiling* tl, const float4* fwd, const float4* dl_dc,
+                               const float* target, float mse_scale, double* loss, int mode, const uint2* aux,
+                               float4* proj_grad, const uint32_t* d_skip, uint64_t* work, float4* proj_comp,
+                               const SceneDev* scenes, bool count_pairs, const TakerChunks* takers) {
   BlendArgs a = blend_args(tl, stride);
-  a.batch = batch;
   a.scenes = scenes;
   a.count_pairs = count_pairs;
   const float gscale = (2.0f / ((float)tl->width * (float)tl->height * 3.0f)) * mse_scale;
@@ -984,21 +1216,30 @@ static sc_status backward_list(sc_ctx* ctx, const float4* rec, uint32_t stride, 
   if (grid == 0) return SC_OK;
   const int ppt = pick_ppt(tl);
   if (ppt == 1 && pixels > 256) return sc_fail(ctx, SC_ERR_INVALID_ARG, "tile too large for one pixel per thread");
-  if (ppt == 2)
-    return backward_ppt<2, LIST>(ctx, a, (uint32_t)grid, pixels / 2, rec, l, fwd, dl_dc, target, gscale, loss, mode,
-                                 aux, proj_grad, d_skip, work, proj_comp);
-  return backward_ppt<1, LIST>(ctx, a, (uint32_t)grid, pixels, rec, l, fwd, dl_dc, target, gscale, loss, mode, aux,
-                               proj_grad, d_skip, work, proj_comp);
+  // the octet reduction needs an octet's lanes in one row pair of the tile
+  const bool oct = ppt == 2 && tl->tile_w % 8 == 0;
+  const TakerChunks tk = takers ? *takers : TakerChunks{};
+#define SC_BWD_SHAPES(LIST, MODE) \
+  (oct ? backward_ppt<2, LIST, MODE, true> : ppt == 2 ? backward_ppt<2, LIST, MODE, false> \
+                                                      : backward_ppt<1, LIST, MODE, false>)
+  auto launch = takers && mode == SC_BWD_EXACT ? SC_BWD_SHAPES(LIST_TAKERS, SC_BWD_EXACT)
+                : list == LIST_ITEMS ? (mode == SC_BWD_EXACT ? SC_BWD_SHAPES(LIST_ITEMS, SC_BWD_EXACT)
+                                                             : SC_BWD_SHAPES(LIST_ITEMS, SC_BWD_REF))
+                                     : (mode == SC_BWD_EXACT ? SC_BWD_SHAPES(LIST_PAIRS, SC_BWD_EXACT)
+                                                             : SC_BWD_SHAPES(LIST_PAIRS, SC_BWD_REF));
+#undef SC_BWD_SHAPES
+  return launch(ctx, a, (uint32_t)grid, pixels / ppt, rec, l, fwd, dl_dc, target, gscale, loss, aux, proj_grad, d_skip,
+                work, proj_comp, tk);
 }
 
 sc_status launch_composite_backward(sc_ctx* ctx, const float4* rec, uint32_t stride, uint32_t n_views,
                                     const uint32_t* payloads, const uint32_t* ranges, const sc_tiling* tl,
                                     const float4* fwd, const float4* dl_dc, int mode, const uint2* aux,
                                     float4* proj_grad, const uint32_t* d_skip, const float* target,
-                                    float mse_scale, double* loss, float4* proj_comp) {
+                                    float mse_scale, double* loss, float4* proj_comp, const TakerChunks* takers) {
   ListArgs l{payloads, reinterpret_cast<const uint2*>(ranges), nullptr, 0, 0};
-  return backward_list<LIST_PAIRS>(ctx, rec, stride, n_views, l, tl, fwd, dl_dc, target, mse_scale, loss, mode, aux,
-                                   proj_grad, d_skip, nullptr, proj_comp, 0, nullptr, false);
+  return backward_list(ctx, rec, stride, n_views, LIST_PAIRS, l, tl, fwd, dl_dc, target, mse_scale, loss, mode, aux,
+                       proj_grad, d_skip, nullptr, proj_comp, nullptr, false, takers);
 }
 
 sc_status launch_composite_backward_items(sc_ctx* ctx, const float4* rec, uint32_t stride, uint32_t n_views,
@@ -1006,13 +1247,13 @@ sc_status launch_composite_backward_items(sc_ctx* ctx, const float4* rec, uint32
                                           const uint32_t* item_ranges, const sc_tiling* tl, const float4* fwd,
                                           const float4* dl_dc, int mode, const uint2* aux, float4* proj_grad,
                                           const uint32_t* d_skip, const float* target, float mse_scale,
-                                          double* loss, uint64_t* work, float4* proj_comp, uint32_t batch,
-                                          const SceneDev* scenes, bool count_pairs) {
+                                          double* loss, uint64_t* work, float4* proj_comp, const SceneDev* scenes,
+                                          bool count_pairs, const TakerChunks* takers) {
   const BlendArgs a = blend_args(tl, stride);
   ListArgs l{item_ids, reinterpret_cast<const uint2*>(item_ranges), item_keys, (a.tiles_x + SC_SUPER - 1) / SC_SUPER,
              super_tiles_per_view(tl)};
-  return backward_list<LIST_ITEMS>(ctx, rec, stride, n_views, l, tl, fwd, dl_dc, target, mse_scale, loss, mode, aux,
-                                   proj_grad, d_skip, work, proj_comp, batch, scenes, count_pairs);
+  return backward_list(ctx, rec, stride, n_views, LIST_ITEMS, l, tl, fwd, dl_dc, target, mse_scale, loss, mode, aux,
+                       proj_grad, d_skip, work, proj_comp, scenes, count_pairs, takers);
 }
 
 // proj_grad += proj_comp over n float4 (the compensated totals rounded once)

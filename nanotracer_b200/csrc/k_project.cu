@@ -535,7 +535,7 @@ __device__ __forceinline__ void project_backward_rows(const DSplats& s, const fl
   float gpos[3] = {0.f, 0.f, 0.f}, grot[4] = {0.f, 0.f, 0.f, 0.f}, gsc[3] = {0.f, 0.f, 0.f}, gop = 0.f;
   float gdc[3] = {0.f, 0.f, 0.f};
   // padding splats, or a step whose emission overflowed, contribute nothing
-  if (i < s.n && !(skip && (*skip & SC_DEVERR_CAPACITY))) {
+  if (i < s.n && !(skip && (*skip & SC_DEVERR_SKIP))) {
     const uint32_t si = (uint32_t)i;
     const float px = sp_row(s, 0, si), py = sp_row(s, 1, si), pz = sp_row(s, 2, si);
     const float qw = sp_row(s, 3, si), qx = sp_row(s, 4, si), qy = sp_row(s, 5, si), qz = sp_row(s, 6, si);

@@ -30,6 +30,9 @@
 // device error word bits
 #define SC_DEVERR_TIMEOUT 1u
 #define SC_DEVERR_CAPACITY 2u
+#define SC_DEVERR_TAKERS 4u  // a blend forward ran out of taker chunks (the trainer grows them)
+// a step whose lists are incomplete: its gradients are not formed and its parameters stay
+#define SC_DEVERR_SKIP (SC_DEVERR_CAPACITY | SC_DEVERR_TAKERS)
 
 // bounded spin limit for decoupled look-back waits (iterations of a poll loop
 // with a nanosleep back-off; ~1 s worst case before giving up)
@@ -496,10 +499,25 @@ sc_status launch_super_emit(sc_ctx* ctx, const float4* rec, uint32_t stride, uin
 uint32_t super_tiles_per_view(const sc_tiling* tl);
 
 // blending
+// The entries ("takers") that some pixel of a blend warp took in a forward, per
+// warp in blend order, in chunks of 32 ids: head[(view, tile) * warps + warp] =
+// (last chunk, takers), prev[chunk] the chunk before it.  Chunk numbers are
+// drawn from TAKER_POOLS counters (zeroed by the caller before the forward), pool p
+// holding chunks [p pool_cap, (p + 1) pool_cap); a pool that runs out raises
+// SC_DEVERR_TAKERS and goes on counting.
+constexpr uint32_t TAKER_POOLS = 64;
+struct TakerChunks {
+  uint32_t* ids;    // TAKER_POOLS x pool_cap x 32
+  uint32_t* prev;   // TAKER_POOLS x pool_cap
+  uint2* head;
+  uint32_t* drawn;  // TAKER_POOLS
+  uint32_t pool_cap;
+};
+uint32_t blend_warps_per_tile(const sc_tiling* tl);
 sc_status launch_composite(sc_ctx* ctx, const float4* rec, uint32_t stride, uint32_t n_views,
                            const uint32_t* payloads, const uint32_t* ranges, const sc_tiling* tl, float4* image,
                            uint2* aux, const float* target, float mse_scale, float4* dl_dc, double* loss,
-                           const uint32_t* d_skip);
+                           uint32_t* d_skip, const TakerChunks* takers = nullptr);
 sc_status launch_mse(sc_ctx* ctx, const float4* pred, const float* target, uint64_t pixels_per_view,
                      uint32_t n_views, float scale, float4* dl_dc, double* loss);
 // with a target, dL/dC of the MSE (mse_scale as in launch_composite) and its
@@ -508,7 +526,8 @@ sc_status launch_composite_backward(sc_ctx* ctx, const float4* rec, uint32_t str
                                     const uint32_t* payloads, const uint32_t* ranges, const sc_tiling* tl,
                                     const float4* fwd, const float4* dl_dc, int mode, const uint2* aux,
                                     float4* proj_grad, const uint32_t* d_skip, const float* target = nullptr,
-                                    float mse_scale = 0.0f, double* loss = nullptr, float4* proj_comp = nullptr);
+                                    float mse_scale = 0.0f, double* loss = nullptr, float4* proj_comp = nullptr,
+                                    const TakerChunks* takers = nullptr);
 // proj_comp (nullable, same layout as proj_grad, zeroed by the caller): the
 // per-(view, splat) totals across tiles are then TwoSum-compensated atomic sums,
 // their rounding errors accumulated in proj_comp (the total is grad + comp)
@@ -516,8 +535,10 @@ sc_status launch_fold_comp(sc_ctx* ctx, float4* proj_grad, const float4* proj_co
 // the same two passes over super-tile item lists (launch_super_emit's items
 // sorted by super tile, item_ranges per (view, super tile)): each tile blends
 // the items whose member mask holds it, in list order; aux then holds
-// positions within the super tile's list.  batch: list positions staged per
-// batch (0 = one per thread).  scenes (nullable): view v's pixels are those
+// positions within the super tile's list.  batch: list positions the forward
+// takes per stage, a quarter of them entries (at most 32, 0 = 32).  takers (nullable): the forward
+// writes the warps' takers down, and aux holds indices among them; the exact
+// backward walks them instead of the lists.  scenes (nullable): view v's pixels are those
 // inside scene v's width x height (the images keep the tiling's row pitch) and
 // its MSE scale is the scene's.  work (nullable, 3 BLEND_WORK_SLOTS u64,
 // accumulated): BLEND_WORK_SLOTS (scanned, staged) pairs — the list positions
@@ -527,16 +548,17 @@ constexpr uint32_t BLEND_WORK_SLOTS = 64;
 sc_status launch_composite_items(sc_ctx* ctx, const float4* rec, uint32_t stride, uint32_t n_views,
                                  const uint32_t* item_keys, const uint32_t* item_ids, const uint32_t* item_ranges,
                                  const sc_tiling* tl, float4* image, uint2* aux, const float* target, float mse_scale,
-                                 float4* dl_dc, double* loss, const uint32_t* d_skip, uint64_t* work = nullptr,
-                                 uint32_t batch = 0, const SceneDev* scenes = nullptr, bool count_pairs = false);
+                                 float4* dl_dc, double* loss, uint32_t* d_skip, uint64_t* work = nullptr,
+                                 uint32_t batch = 0, const SceneDev* scenes = nullptr, bool count_pairs = false,
+                                 const TakerChunks* takers = nullptr);
 sc_status launch_composite_backward_items(sc_ctx* ctx, const float4* rec, uint32_t stride, uint32_t n_views,
                                           const uint32_t* item_keys, const uint32_t* item_ids,
                                           const uint32_t* item_ranges, const sc_tiling* tl, const float4* fwd,
                                           const float4* dl_dc, int mode, const uint2* aux, float4* proj_grad,
                                           const uint32_t* d_skip, const float* target = nullptr,
                                           float mse_scale = 0.0f, double* loss = nullptr, uint64_t* work = nullptr,
-                                          float4* proj_comp = nullptr, uint32_t batch = 0,
-                                          const SceneDev* scenes = nullptr, bool count_pairs = false);
+                                          float4* proj_comp = nullptr, const SceneDev* scenes = nullptr,
+                                          bool count_pairs = false, const TakerChunks* takers = nullptr);
 sc_status launch_tonemap(sc_ctx* ctx, const float4* img, uint32_t w, uint32_t h, uint8_t* out);
 
 // SSIM (loss.rs:22-375): scale * dL_ssim/dC added into dl_dc, per-view sum of

@@ -43,14 +43,15 @@ struct StepOut {
   unsigned long long pairs;
   unsigned long long items;  // two-level binning items
   uint32_t err;
-  uint32_t pad;
+  uint32_t chunks;  // taker chunks drawn from the fullest pool
 };
 
 // loss = mean over the views, or (weight > 0) weight * sum over the views, of
 // (1 - lambda) MSE + lambda (1 - SSIM) (loss.rs:383-410; MSE alone without SSIM sums)
 __global__ void k_finalize(const double* __restrict__ loss_sums, const double* __restrict__ ssim_sums, float lambda,
                            uint32_t n_views, double inv_count, double weight, const uint64_t* __restrict__ d_total,
-                           const uint32_t* __restrict__ err, StepOut* __restrict__ out) {
+                           const uint32_t* __restrict__ err, const uint32_t* __restrict__ drawn,
+                           StepOut* __restrict__ out) {
   double acc = 0.0;
   for (uint32_t v = 0; v < n_views; ++v) {
     const double m = loss_sums[v] * inv_count;
@@ -62,6 +63,9 @@ __global__ void k_finalize(const double* __restrict__ loss_sums, const double* _
   out->pairs = d_total[0];
   out->items = d_total[1];
   out->err = *err;
+  uint32_t most = 0;
+  for (uint32_t p = 0; p < sck::TAKER_POOLS; ++p) most = max(most, drawn[p]);
+  out->chunks = most;
 }
 
 // stage names of the two-level binning step (the pair-sort step uses kStageNames)
@@ -121,6 +125,8 @@ struct sc_trainer {
   cudaEvent_t ev_view[SC_MAX_VIEWS] = {};  // view v's targets copied
   cudaStream_t bwd_stream[SC_MAX_VIEWS] = {};  // view v's blend backward (host targets)
   cudaEvent_t ev_bwd[SC_MAX_VIEWS] = {};
+  // exact backward: the forward's takers (ids, prev, head, drawn)
+  sck::TakerChunks takers{};
   double* d_loss = nullptr;
   uint64_t* d_total = nullptr;
   void* scratch = nullptr; size_t scratch_bytes = 0;
@@ -278,6 +284,24 @@ static sc_status ensure_pairs(sc_trainer* tr, uint64_t K) {
   return ensure_scratch(tr);
 }
 
+// taker chunks per pool
+static sc_status ensure_takers(sc_trainer* tr, uint64_t chunks) {
+  if (tr->cfg.bwd_mode != SC_BWD_EXACT || chunks <= tr->takers.pool_cap) return SC_OK;
+  sc_ctx* ctx = tr->ctx;
+  const uint64_t cap = chunks + chunks / 4 + 64;
+  if (cap * sck::TAKER_POOLS > 0xFFFFFFFFull) return sc_fail(ctx, SC_ERR_CAPACITY, "too many blended entries in one step");
+  SC_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "sync");
+  cudaFree(tr->takers.ids);
+  cudaFree(tr->takers.prev);
+  tr->takers.ids = tr->takers.prev = nullptr;
+  tr->takers.pool_cap = 0;
+  SC_CUDA_TRY(ctx, cudaMalloc(&tr->takers.ids, cap * sck::TAKER_POOLS * 32 * 4), "takers");
+  SC_CUDA_TRY(ctx, cudaMalloc(&tr->takers.prev, cap * sck::TAKER_POOLS * 4), "takers");
+  tr->takers.pool_cap = (uint32_t)cap;
+  trainer_drop_graph(tr);
+  return SC_OK;
+}
+
 static void mark(sc_trainer* tr, int i, bool capturing) {
   if (!tr->profiling) return;
   if (capturing)
@@ -314,7 +338,8 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
       SC_CUDA_TRY(ctx, cudaEventRecord(tr->ev_view[v], tr->copy_stream), "copied");
     }
   }
-  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->d_loss, 0, 8 * (size_t)V, ctx->stream), "zero loss");
+  // the loss sums and, behind them, the taker pools' counters
+  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->d_loss, 0, 8 * (size_t)V + sck::TAKER_POOLS * 4, ctx->stream), "zero loss");
   uint64_t* work_fwd = tr->profiling ? tr->d_work : nullptr;
   uint64_t* work_bwd = tr->profiling ? tr->d_work + 3 * sck::BLEND_WORK_SLOTS : nullptr;
   if (tr->profiling)
@@ -395,15 +420,16 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
   // are needed only from the backward on (a host upload overlaps the forward)
   const bool mse_in_bwd = lam == 0.0f;
   const float* fwd_target = mse_in_bwd ? nullptr : tr->targets;
+  const sck::TakerChunks* takers = tr->cfg.bwd_mode == SC_BWD_EXACT ? &tr->takers : nullptr;
   if (tr->h_targets && !mse_in_bwd)  // the copies run in order: the last view's event covers all
     SC_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->stream, tr->ev_view[V - 1], 0), "join");
   if (tr->two_level)
     SC_TRY(sck::launch_composite_items(ctx, tr->rec, tr->stride, V, item_keys, item_ids, tr->iranges, &tr->cfg.tiling,
                                        tr->image, tr->aux, fwd_target, mse_w, tr->dl_dc, tr->d_loss, ctx->d_error,
-                                       work_fwd, tr->cfg.blend_batch, scenes, tr->profiling >= 2));
+                                       work_fwd, tr->cfg.blend_batch, scenes, tr->profiling >= 2, takers));
   else
     SC_TRY(sck::launch_composite(ctx, tr->rec, tr->stride, V, svals, tr->ranges, &tr->cfg.tiling, tr->image, tr->aux,
-                                 fwd_target, mse_w, tr->dl_dc, tr->d_loss, ctx->d_error));
+                                 fwd_target, mse_w, tr->dl_dc, tr->d_loss, ctx->d_error, takers));
   if (lam > 0.0f) {
     SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->d_ssim, 0, 8 * (size_t)V, ctx->stream), "zero ssim");
     SC_TRY(sck::launch_ssim(ctx, tr->image, tr->targets, tr->cfg.tiling.width, tr->cfg.tiling.height, V,
@@ -427,6 +453,8 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
     }
     const size_t so = (size_t)3 * v0 * tr->stride, po = (size_t)v0 * tr->P;
     const float* tg = bwd_target ? bwd_target + 3 * po : nullptr;
+    sck::TakerChunks vt = tr->takers;  // the views' heads
+    if (takers) vt.head += (size_t)v0 * tr->T * sck::blend_warps_per_tile(&tr->cfg.tiling);
     sc_status st;
     if (tr->two_level)
       st = (sck::launch_composite_backward_items(ctx, tr->rec + so, tr->stride, nv, item_keys, item_ids,
@@ -434,14 +462,15 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
                                                   tr->image + po, tr->dl_dc ? tr->dl_dc + po : nullptr,
                                                   (int)tr->cfg.bwd_mode, tr->aux + po,
                                                   tr->pgrad + so, ctx->d_error, tg, mse_w, tr->d_loss + v0, work_bwd,
-                                                  tr->pcomp ? tr->pcomp + so : nullptr, tr->cfg.blend_batch,
-                                                  scenes ? scenes + v0 : nullptr, tr->profiling >= 2));
+                                                  tr->pcomp ? tr->pcomp + so : nullptr,
+                                                  scenes ? scenes + v0 : nullptr, tr->profiling >= 2,
+                                                  takers ? &vt : nullptr));
     else
       st = (sck::launch_composite_backward(ctx, tr->rec + so, tr->stride, nv, svals, tr->ranges + (size_t)2 * v0 * tr->T,
                                             &tr->cfg.tiling, tr->image + po, tr->dl_dc ? tr->dl_dc + po : nullptr,
                                             (int)tr->cfg.bwd_mode,
                                             tr->aux + po, tr->pgrad + so, ctx->d_error, tg, mse_w, tr->d_loss + v0,
-                                            tr->pcomp ? tr->pcomp + so : nullptr));
+                                            tr->pcomp ? tr->pcomp + so : nullptr, takers ? &vt : nullptr));
     ctx->stream = main_stream;
     SC_TRY(st);
     if (per_view) SC_CUDA_TRY(ctx, cudaEventRecord(tr->ev_bwd[v0], tr->bwd_stream[v0]), "view done");
@@ -472,7 +501,7 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
   mark(tr, 9, capturing);
   k_finalize<<<1, 1, 0, ctx->stream>>>(tr->d_loss, lam > 0.0f ? tr->d_ssim : nullptr, lam, V,
                                        1.0 / (3.0 * (double)tr->P), tr->grads_mode ? (double)tr->loss_weight : 0.0,
-                                       tr->d_total, ctx->d_error, tr->d_out);
+                                       tr->d_total, ctx->d_error, tr->takers.drawn, tr->d_out);
   SC_TRY(sc_check_launch(ctx, "k_finalize"));
   SC_CUDA_TRY(ctx, cudaMemcpyAsync(tr->h_out, tr->d_out, sizeof(StepOut), cudaMemcpyDeviceToHost, ctx->stream), "out D2H");
   if (tr->scenes_mode)
@@ -534,7 +563,9 @@ sc_status sc_trainer_create(sc_ctx* ctx, const sc_train_config* cfg, sc_trainer*
   if (e == cudaSuccess) e = cudaMalloc(&tr->image, pix * 16);
   if (e == cudaSuccess) e = cudaMalloc(&tr->aux, pix * 8);
   if (e == cudaSuccess) e = cudaMalloc(&tr->dl_dc, pix * 16);
-  if (e == cudaSuccess) e = cudaMalloc(&tr->d_loss, 8 * (size_t)tr->V);
+  if (e == cudaSuccess) e = cudaMalloc(&tr->d_loss, 8 * (size_t)tr->V + sck::TAKER_POOLS * 4);
+  const size_t heads = (size_t)tr->V * tr->T * sck::blend_warps_per_tile(&t);
+  if (e == cudaSuccess && cfg->bwd_mode == SC_BWD_EXACT) e = cudaMalloc(&tr->takers.head, heads * sizeof(uint2));
   if (e == cudaSuccess) e = cudaMalloc(&tr->d_work, 6 * sck::BLEND_WORK_SLOTS * 8);
   if (e == cudaSuccess) e = cudaMalloc(&tr->d_total, 64);
   if (e == cudaSuccess) e = cudaMemset(tr->d_total, 0, 64);
@@ -547,6 +578,13 @@ sc_status sc_trainer_create(sc_ctx* ctx, const sc_train_config* cfg, sc_trainer*
     return sc_cuda_fail(ctx, e, "trainer alloc");
   }
   std::memset(tr->h_params, 0, sizeof(StepParams));
+  tr->takers.drawn = reinterpret_cast<uint32_t*>(tr->d_loss + tr->V);
+  // a first guess of 4 chunks a warp; a step that draws more runs again with the number it needs
+  const sc_status st = ensure_takers(tr, sc_div_up(4 * heads, sck::TAKER_POOLS) + 1);
+  if (st != SC_OK) {
+    sc_trainer_free(ctx, tr);
+    return st;
+  }
   *out = tr;
   return SC_OK;
 }
@@ -559,6 +597,7 @@ void sc_trainer_free(sc_ctx* ctx, sc_trainer* tr) {
   trainer_free_pairs(tr);
   trainer_free_items(tr);
   cudaFree(tr->iranges);
+  cudaFree(tr->takers.ids); cudaFree(tr->takers.prev); cudaFree(tr->takers.head);
   cudaFree(tr->ranges); cudaFree(tr->image); cudaFree(tr->aux); cudaFree(tr->dl_dc);
   cudaFree(tr->d_loss); cudaFree(tr->d_work); cudaFree(tr->d_total); cudaFree(tr->d_params); cudaFree(tr->d_out);
   cudaFree(tr->ssim_terms); cudaFree(tr->d_ssim);
@@ -680,11 +719,12 @@ static sc_status run_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, float* a
       cudaMemsetAsync(ctx->d_error, 0, 4, ctx->stream);
       return sc_fail(ctx, SC_ERR_TIMEOUT, "a bounded device wait gave up during the step");
     }
-    if (o.err & SC_DEVERR_CAPACITY) {
+    if (o.err & SC_DEVERR_SKIP) {
       // the blend and Adam kernels skipped this step; grow and run it again
       SC_CUDA_TRY(ctx, cudaMemsetAsync(ctx->d_error, 0, 4, ctx->stream), "clear error");
       SC_TRY(ensure_items(tr, o.items));
       SC_TRY(ensure_pairs(tr, o.pairs));
+      SC_TRY(ensure_takers(tr, o.chunks));
       continue;
     }
     if (tr->profiling) {

@@ -52,7 +52,7 @@ class TrainConfig:
     sort_mode: int = 0  # 0 auto (two-level binning), 1 sort of the (tile, splat) pairs, 2 two-level
     fp64_det: bool = False  # FP64 determinant / inverse of near-degenerate splats (projection and adjoint)
     compensated_sums: bool = False  # TwoSum-compensated per-(view, splat) gradient totals across tiles
-    blend_batch: int = 0  # list positions staged per blend batch (multiple of 32); 0 = one per thread
+    blend_batch: int = 0  # list positions the blend forward takes per stage (multiple of 32); 0 = 128
     sort_digit_bits: int = 0  # radix digit width of the binning sort: 8, 9, or 0 = fewer passes wins
 
     def struct(self) -> sc_train_config:

@@ -1,0 +1,111 @@
+"""The blends at the sizes where a warp's own walk can go wrong: tile shapes
+that split into 8 x 8 blocks, whole rows or single pixels per thread, images
+that cut tiles, lists shorter than a stage, of a whole number of stages and
+much longer, and warps that take more entries than the trainer first has room
+for.
+
+The trainer's backward walks the entries that its forward wrote down, the
+stage calls' backward walks the lists; both form the same terms (the same
+instructions) and add them in float in another order, so their projected
+gradients agree to float rounding: a sum of m terms differs by at most
+m 2^-24 of the terms' magnitudes, and sqrt(m) of that in the mean — 1e-5 of the
+norm for the few thousand terms here.  The stage calls themselves are held to
+the oracle as in the other parity tests."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from nanotracer_b200 import CameraUniform, GpuSplatBuffer, GradSplatBuffers, TilingParams
+from nanotracer_b200._lib import SC_BWD_EXACT, SC_BWD_REF, check, lib
+from nanotracer_b200.raster import cameras_array
+from nanotracer_b200.scene import FOV_Y, orbit_pose, random_scene
+from nanotracer_b200.train import TrainConfig, Trainer
+from tests.util import GpuPipe, check_pg_explained, margins
+
+pytestmark = pytest.mark.gpu
+
+# (tile_w, tile_h): 8 x 8 blocks; a warp of whole rows; a tile width that is no
+# multiple of 8; one pixel per thread (odd height)
+TILES = [(16, 16), (8, 8), (32, 8), (32, 2), (4, 16), (32, 3)]
+
+
+def _scene(n, opaque=True):
+    s = random_scene(n, 7 * n + 1)
+    if not opaque:  # wide and faint: every pixel takes nearly every splat
+        s.scales[:] = np.log(0.6)
+        s.opacities[:] = -4.0
+    return s
+
+
+def _targets(W, H):
+    y, x = np.mgrid[0:H, 0:W]
+    return np.stack([0.5 + 0.4 * np.sin(0.1 * x), 0.5 + 0.4 * np.cos(0.07 * y), 0.3 + 0.002 * (x + y) % 0.5],
+                    -1).astype(np.float32)[None]
+
+
+def _stage_grads(ctx, scene, cam, tl, tgt, W, H):
+    """Parameter gradient rows (59, n) and the image through the stage calls (exact mode)."""
+    pipe = GpuPipe(ctx, scene, cam, tl)
+    pipe.project(), pipe.bin()
+    img, _ = pipe.composite()
+    pipe.backward((np.concatenate([img[..., :3] - tgt, np.zeros_like(img[..., :1])], -1) *
+                   np.float32(2.0 / (3.0 * W * H))).astype(np.float32), SC_BWD_EXACT)
+    grads = GradSplatBuffers(ctx, pipe.g.capacity)
+    pipe.r.project_backward(pipe.g, pipe.pg, cam, grads)
+    return grads.readback(len(scene)).flat().T, img[0]
+
+
+def _trainer_grads(ctx, scene, cam, cfg, tgt):
+    n = len(scene)
+    g = GpuSplatBuffer.upload(ctx, scene)
+    tr = Trainer(ctx, cfg)
+    tr.set_targets(ctx.storage_buffer("t", tgt))
+    shard = (n + 63) // 64 * 64
+    out = ctx.storage_buffer_zeroed("grads", 59 * shard * 4)
+    loss = C.c_double()
+    for _ in range(2):  # the sizing step, then the captured one
+        check(lib().sc_trainer_step_grads(tr.handle, g.handle, cameras_array([cam]), 1.0, 1, shard, out.cptr,
+                                          C.byref(loss)), ctx.handle)
+    return out.readback(np.float32, 59 * shard).reshape(59, shard)[:, :n], tr.images()[0]
+
+
+@pytest.mark.parametrize("tile", TILES)
+@pytest.mark.parametrize("n,opaque,size", [(1, True, (33, 17)), (31, False, (40, 24)), (32, False, (40, 24)),
+                                           (33, False, (61, 35)), (700, False, (50, 30)), (4000, True, (203, 117))])
+def test_trainer_backward_over_the_takers_equals_the_list_backward(ctx, tile, n, opaque, size):
+    W, H = size
+    scene = _scene(n, opaque)
+    cam = CameraUniform.from_pose(*orbit_pose(20.0), FOV_Y, W, H, n)
+    tl = TilingParams(W, H, tile[0], 8.0, tile_h_override=tile[1])
+    tgt = _targets(W, H)
+    want, img = _stage_grads(ctx, scene, cam, tl, tgt, W, H)
+    cfg = TrainConfig(n_views=1, width=W, height=H, tile_w=tile[0], tile_h=tile[1], depth_max=8.0, tile_cull=False)
+    got, timg = _trainer_grads(ctx, scene, cam, cfg, tgt)
+    assert np.array_equal(img, timg)
+    for lo, hi in [(0, 3), (3, 7), (7, 10), (10, 11), (11, 14), (14, 59)]:
+        d = np.linalg.norm((got[lo:hi] - want[lo:hi]).astype(np.float64))
+        assert d <= 1e-5 * np.linalg.norm(want[lo:hi].astype(np.float64)) + 1e-30, (lo, d)
+
+
+@pytest.mark.parametrize("mode", [SC_BWD_EXACT, SC_BWD_REF])
+@pytest.mark.parametrize("tile", TILES)
+def test_list_backward_against_the_oracle_for_every_warp_layout(ctx, oracle, tile, mode):
+    n, W, H = 1500, 101, 67
+    cam = CameraUniform.from_pose(*orbit_pose(35.0), FOV_Y, W, H, n)
+    tl = TilingParams(W, H, tile[0], 8.0, tile_h_override=tile[1])
+    pipe = GpuPipe(ctx, _scene(n), cam, tl)
+    rec = pipe.project()[0]
+    _, payloads, ranges = pipe.bin()
+    img, aux = pipe.composite()
+    rng = np.random.default_rng(5)
+    dl = np.zeros((H, W, 4), np.float32)
+    dl[..., :3] = rng.normal(0, 1e-3, (H, W, 3))
+    pg = pipe.backward(dl[None], mode)[0]
+    otl = oracle.tiling(W, H, tile[0], tile[1], 8.0)
+    _, flags, _ = margins(oracle, rec, payloads, ranges, otl, mode)
+    tfin = np.ascontiguousarray(aux[0, ..., 0]).view(np.float32)
+    want, absum = oracle.composite_backward(rec, payloads, ranges.reshape(-1), otl, img[0].reshape(-1, 4),
+                                            dl.reshape(-1, 4), mode, np.ascontiguousarray(aux[0, ..., 1]).reshape(-1),
+                                            tfin.reshape(-1), want_abs=True)
+    check_pg_explained(pg, want, absum, flags, label=f"tile {tile} mode {mode}")
