@@ -110,3 +110,17 @@ def test_trainer_with_ssim_term_matches_oracle_iteration(ctx, oracle):
     assert abs(losses[0] - oloss) <= 1e-5 * oloss
     got, want = g.readback().flat(), os_.flat()
     assert np.mean(np.abs(got - want) <= 1e-6 + 1e-6 * np.abs(want)) > 0.995
+
+
+@pytest.mark.parametrize("w,h,V", [(32, 32, 1), (33, 31, 2), (31, 65, 1), (64, 6, 1), (6, 70, 1), (38, 37, 3)])
+def test_ssim_at_the_edges_of_its_tiles(ctx, oracle, w, h, V):
+    """Image sides of whole 32-pixel tiles, one more and one less, borders whose
+    reflections reach into a neighbouring tile, and the smallest side: the
+    bounds of test_ssim_matches_oracle."""
+    pred4, tgt = _images(w, h, V, seed=3 * w + h)
+    loss, dl = _device_loss(ctx, "sc_ssim_loss_grad", pred4, tgt, C.c_float(0.7))
+    for v in range(V):
+        ol, odl = oracle.ssim(pred4[v], tgt[v], w, h, 0.7)
+        odl = odl.reshape(h, w, 4)
+        assert abs(loss[v, 0] - ol) <= 1e-6 + 1e-5 * abs(ol)
+        assert np.allclose(dl[v], odl, rtol=1e-4, atol=1e-5 * np.abs(odl).max())
