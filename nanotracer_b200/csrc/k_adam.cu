@@ -354,68 +354,101 @@ sc_status launch_adam_shard(sc_ctx* ctx, const DSplats& s, const DMoments& mo, f
   return launch_adam_rows(ctx, s, mo, acc, g, lo, count, shard, ap, nullptr, nullptr);
 }
 
-// grid.y = row
-__global__ void k_pack_params(DSplats s, uint32_t lo, uint32_t count, uint32_t shard, float* __restrict__ out) {
-  const int r = blockIdx.y;
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count; j += gridDim.x * blockDim.x)
-    out[(size_t)r * shard + j] = sp_row(s, r, lo + j);
+// The copies below move one row of PACK_IPT x 256 elements per CTA (grid.y = row),
+// each thread's PACK_IPT loads in flight together: one element at a time left
+// them waiting on memory at half the copy rate (1M
+// splats, parameters of f32: 136 -> 68 us, bf16 SH rest: 130 -> 57 us).
+// Elements stay 256 apart per thread, so any count, offset and pitch is coalesced.
+constexpr uint32_t PACK_IPT = 8;
+template <typename LD, typename ST>
+__device__ __forceinline__ void copy_row(uint32_t n, LD&& ld, ST&& st) {
+  const uint64_t j0 = (uint64_t)blockIdx.x * (256 * PACK_IPT) + threadIdx.x;
+  if (j0 >= n) return;
+  float x[PACK_IPT];
+#pragma unroll
+  for (uint32_t u = 0; u < PACK_IPT; ++u) x[u] = j0 + u * 256 < n ? ld((uint32_t)j0 + u * 256) : 0.0f;
+#pragma unroll
+  for (uint32_t u = 0; u < PACK_IPT; ++u)
+    if (j0 + u * 256 < n) st((uint32_t)j0 + u * 256, x[u]);
 }
+static dim3 copy_grid(uint64_t n, unsigned rows) { return dim3((unsigned)sc_div_up(n, 256 * PACK_IPT), rows); }
 
-// in = n_shards chunks of SC_NROWS rows x shard; splat i = q * shard + j
-__global__ void k_unpack_params(DSplats s, const float* __restrict__ in, uint32_t n_shards, uint32_t shard) {
+__global__ void __launch_bounds__(256) k_pack_params(DSplats s, uint32_t lo, uint32_t count, uint32_t shard,
+                                                     float* __restrict__ out) {
   const int r = blockIdx.y;
-  const uint64_t total = std::min<uint64_t>((uint64_t)n_shards * shard, s.n);
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t q = i / shard, j = i % shard;
-    sp_set(s, r, (uint32_t)i, in[(q * SC_NROWS + r) * shard + j]);
+  float* o = out + (size_t)r * shard;
+  if (r >= SC_ROW_REST && s.bf16) {
+    const __nv_bfloat16* src = s.rest16 + (size_t)(r - SC_ROW_REST) * s.cap + lo;
+    copy_row(count, [&](uint32_t j) { return __bfloat162float(src[j]); }, [&](uint32_t j, float x) { o[j] = x; });
+  } else {
+    const float* src = s.slab + (size_t)r * s.cap + lo;
+    copy_row(count, [&](uint32_t j) { return src[j]; }, [&](uint32_t j, float x) { o[j] = x; });
   }
 }
 
-__global__ void k_pack_moments(DMoments mo, uint32_t lo, uint32_t count, uint32_t shard, float* __restrict__ out) {
-  const int r = blockIdx.y >> 1, which = blockIdx.y & 1;  // m rows then v rows, interleaved by grid.y
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count; j += gridDim.x * blockDim.x) {
-    const size_t k = (size_t)r * mo.cap + lo + j;
-    const float x = which ? mo_ld(mo, mo.v, mo.v16, k) : mo_ld(mo, mo.m, mo.m16, k);
-    out[((size_t)which * SC_NROWS + r) * shard + j] = x;
+// in = n_shards chunks of SC_NROWS rows x shard; splat i = q * shard + j
+__global__ void __launch_bounds__(256) k_unpack_params(DSplats s, const float* __restrict__ in, uint32_t total,
+                                                       uint32_t shard) {
+  const int r = blockIdx.y;
+  copy_row(total,
+           [&](uint32_t i) {
+             const uint32_t q = i / shard;
+             return in[((size_t)q * SC_NROWS + r) * shard + (i - q * shard)];
+           },
+           [&](uint32_t i, float x) { sp_set(s, r, i, x); });
+}
+
+// grid.y = (row, m or v)
+__global__ void __launch_bounds__(256) k_pack_moments(DMoments mo, uint32_t lo, uint32_t count, uint32_t shard,
+                                                      float* __restrict__ out) {
+  const int r = blockIdx.y >> 1, which = blockIdx.y & 1;
+  float* o = out + ((size_t)which * SC_NROWS + r) * shard;
+  const size_t k0 = (size_t)r * mo.cap + lo;
+  if (mo.bf16) {
+    const __nv_bfloat16* src = (which ? mo.v16 : mo.m16) + k0;
+    copy_row(count, [&](uint32_t j) { return __bfloat162float(src[j]); }, [&](uint32_t j, float x) { o[j] = x; });
+  } else {
+    const float* src = (which ? mo.v : mo.m) + k0;
+    copy_row(count, [&](uint32_t j) { return src[j]; }, [&](uint32_t j, float x) { o[j] = x; });
   }
 }
 
 // in = n_shards chunks of 2 * SC_NROWS rows (m then v) x shard
-__global__ void k_unpack_moments(DMoments mo, uint32_t n, const float* __restrict__ in, uint32_t n_shards,
-                                 uint32_t shard) {
+__global__ void __launch_bounds__(256) k_unpack_moments(DMoments mo, uint32_t total, const float* __restrict__ in,
+                                                        uint32_t shard) {
   const int r = blockIdx.y >> 1, which = blockIdx.y & 1;
-  const uint64_t total = std::min<uint64_t>((uint64_t)n_shards * shard, n);
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t q = i / shard, j = i % shard;
-    const float x = in[((q * 2 + which) * SC_NROWS + r) * shard + j];
-    const size_t k = (size_t)r * mo.cap + i;
-    if (which) mo_st(mo, mo.v, mo.v16, k, x); else mo_st(mo, mo.m, mo.m16, k, x);
-  }
-}
-
-static unsigned rows_grid_x(sc_ctx* ctx, uint64_t n) {
-  return (unsigned)std::max<uint64_t>(1, std::min<uint64_t>(sc_div_up(n, 256), (uint64_t)ctx->sm_count * 4));
+  copy_row(total,
+           [&](uint32_t i) {
+             const uint32_t q = i / shard;
+             return in[(((size_t)q * 2 + which) * SC_NROWS + r) * shard + (i - q * shard)];
+           },
+           [&](uint32_t i, float x) {
+             const size_t k = (size_t)r * mo.cap + i;
+             if (which) mo_st(mo, mo.v, mo.v16, k, x); else mo_st(mo, mo.m, mo.m16, k, x);
+           });
 }
 
 sc_status launch_pack_params(sc_ctx* ctx, const DSplats& s, uint32_t lo, uint32_t count, uint32_t shard, float* out) {
   if (count == 0) return SC_OK;
-  k_pack_params<<<dim3(rows_grid_x(ctx, count), SC_NROWS), 256, 0, ctx->stream>>>(s, lo, count, shard, out);
+  k_pack_params<<<copy_grid(count, SC_NROWS), 256, 0, ctx->stream>>>(s, lo, count, shard, out);
   return sc_check_launch(ctx, "k_pack_params");
 }
 sc_status launch_unpack_params(sc_ctx* ctx, const DSplats& s, const float* in, uint32_t n_shards, uint32_t shard) {
-  if (s.n == 0 || n_shards == 0 || shard == 0) return SC_OK;
-  k_unpack_params<<<dim3(rows_grid_x(ctx, s.n), SC_NROWS), 256, 0, ctx->stream>>>(s, in, n_shards, shard);
+  const uint32_t total = (uint32_t)std::min<uint64_t>((uint64_t)n_shards * shard, s.n);
+  if (total == 0) return SC_OK;
+  k_unpack_params<<<copy_grid(total, SC_NROWS), 256, 0, ctx->stream>>>(s, in, total, shard);
   return sc_check_launch(ctx, "k_unpack_params");
 }
 sc_status launch_pack_moments(sc_ctx* ctx, const DMoments& mo, uint32_t lo, uint32_t count, uint32_t shard, float* out) {
   if (count == 0) return SC_OK;
-  k_pack_moments<<<dim3(rows_grid_x(ctx, count), 2 * SC_NROWS), 256, 0, ctx->stream>>>(mo, lo, count, shard, out);
+  k_pack_moments<<<copy_grid(count, 2 * SC_NROWS), 256, 0, ctx->stream>>>(mo, lo, count, shard, out);
   return sc_check_launch(ctx, "k_pack_moments");
 }
 sc_status launch_unpack_moments(sc_ctx* ctx, const DMoments& mo, uint32_t n, const float* in, uint32_t n_shards,
                                 uint32_t shard) {
-  if (n == 0 || n_shards == 0 || shard == 0) return SC_OK;
-  k_unpack_moments<<<dim3(rows_grid_x(ctx, n), 2 * SC_NROWS), 256, 0, ctx->stream>>>(mo, n, in, n_shards, shard);
+  const uint32_t total = (uint32_t)std::min<uint64_t>((uint64_t)n_shards * shard, n);
+  if (total == 0) return SC_OK;
+  k_unpack_moments<<<copy_grid(total, 2 * SC_NROWS), 256, 0, ctx->stream>>>(mo, total, in, shard);
   return sc_check_launch(ctx, "k_unpack_moments");
 }
 
