@@ -244,8 +244,8 @@ __global__ void __launch_bounds__(256) k_tile_ranges_u32x4(const uint32_t* __res
 
 sc_status launch_tile_ranges(sc_ctx* ctx, const void* keys, int key_mode, const uint64_t* d_total, uint64_t cap,
                              uint32_t num_tiles, uint32_t* ranges, uint32_t tiles_per_view, uint32_t tile_bits,
-                             uint32_t key_bits, uint64_t* high_popc) {
-  SC_CUDA_TRY(ctx, cudaMemsetAsync(ranges, 0, (size_t)num_tiles * 8, ctx->stream), "memset ranges");
+                             uint32_t key_bits, uint64_t* high_popc, bool clean) {
+  if (!clean) SC_CUDA_TRY(ctx, cudaMemsetAsync(ranges, 0, (size_t)num_tiles * 8, ctx->stream), "memset ranges");
   if (cap == 0) return SC_OK;
   const unsigned g = (unsigned)std::min<uint64_t>(sc_div_up(cap, 256), (uint64_t)ctx->sm_count * 16);
   if (key_mode == 0)

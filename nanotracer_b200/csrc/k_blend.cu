@@ -446,9 +446,13 @@ struct TakerOut {
   uint32_t chunk, last;  // chunk being filled, and the one before it
   bool ok;
 
+  // neighbouring tiles and the tiles of a column go to different pools
+  static __device__ __forceinline__ uint32_t pool() {
+    return (blockIdx.x * 2654435761u) >> 16 & (TAKER_POOLS - 1);
+  }
   __device__ __forceinline__ uint32_t draw() {
     uint32_t c = 0;
-    if ((threadIdx.x & 31) == 0) c = atomicAdd(ch.drawn + blockIdx.x % TAKER_POOLS, 1u);
+    if ((threadIdx.x & 31) == 0) c = atomicAdd(ch.drawn + pool(), 1u);
     return c;
   }
   __device__ __forceinline__ TakerOut(const TakerChunks& c, uint32_t* r)
@@ -459,7 +463,7 @@ struct TakerOut {
   __device__ __forceinline__ uint32_t number() {
     const uint32_t c = __shfl_sync(FULL_MASK, chunk, 0);
     ok = ok && c < ch.pool_cap;
-    return (blockIdx.x % TAKER_POOLS) * ch.pool_cap + min(c, ch.pool_cap - 1);
+    return pool() * ch.pool_cap + min(c, ch.pool_cap - 1);
   }
   // append the entries of a stage whose bit in m is set (this lane's entry has id)
   __device__ __forceinline__ void append(uint32_t m, uint32_t id) {

@@ -193,7 +193,7 @@ size_t scan_scratch_bytes(uint64_t n) {
 }
 
 static sc_status scan_u32_impl(sc_ctx* ctx, uint32_t* data, uint64_t n, uint64_t* d_total, void* scratch,
-                               size_t bytes, ScanGather gather) {
+                               size_t bytes, ScanGather gather, bool clean) {
   if (n == 0) {
     if (d_total) SC_CUDA_TRY(ctx, cudaMemsetAsync(d_total, 0, 8, ctx->stream), "memset total");
     return SC_OK;
@@ -202,19 +202,20 @@ static sc_status scan_u32_impl(sc_ctx* ctx, uint32_t* data, uint64_t n, uint64_t
   if (bytes < scan_scratch_bytes(n)) return sc_fail(ctx, SC_ERR_INVALID_ARG, "scan scratch too small");
   unsigned* ticket = reinterpret_cast<unsigned*>(scratch);
   unsigned long long* status = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(scratch) + 256);
-  SC_CUDA_TRY(ctx, cudaMemsetAsync(scratch, 0, scan_scratch_bytes(n), ctx->stream), "memset scan status");
+  if (!clean)
+    SC_CUDA_TRY(ctx, cudaMemsetAsync(scratch, 0, scan_scratch_bytes(n), ctx->stream), "memset scan status");
   k_scan<<<(unsigned)tiles, SCAN_THREADS, 0, ctx->stream>>>(data, n, status, ticket, d_total, ctx->d_error, gather);
   return sc_check_launch(ctx, "k_scan");
 }
 
 sc_status scan_u32(sc_ctx* ctx, uint32_t* data, uint64_t n, uint64_t* d_total, void* scratch, size_t bytes) {
-  return scan_u32_impl(ctx, data, n, d_total, scratch, bytes, ScanGather{nullptr, nullptr, 1, 0});
+  return scan_u32_impl(ctx, data, n, d_total, scratch, bytes, ScanGather{nullptr, nullptr, 1, 0}, false);
 }
 
 sc_status scan_u32_gather(sc_ctx* ctx, uint32_t* out, uint64_t n, const uint32_t* src, const uint32_t* idx,
-                          uint32_t seg, uint64_t gn, uint64_t* d_total, void* scratch, size_t bytes) {
+                          uint32_t seg, uint64_t gn, uint64_t* d_total, void* scratch, size_t bytes, bool clean) {
   if (seg == 0 || seg % SCAN_IPT) return sc_fail(ctx, SC_ERR_INVALID_ARG, "gather segment must be a multiple of 16");
-  return scan_u32_impl(ctx, out, n, d_total, scratch, bytes, ScanGather{src, idx, seg, gn});
+  return scan_u32_impl(ctx, out, n, d_total, scratch, bytes, ScanGather{src, idx, seg, gn}, clean);
 }
 
 // ---------------------------------------------------------------- allocation-free scan
@@ -289,6 +290,7 @@ namespace sck {
 #define RS_HIST_UNROLL 8  // keys each histogram thread loads before counting them
 #define RS_MAX_PASSES 8         // 64-bit keys at 8 or 9 bits per pass
 #define RS_HIST_BYTES (RS_MAX_PASSES * 512 * 4)
+#define RS_DONE 15              // of the 16 tickets: histogram blocks finished
 
 template <typename K> struct RsCfg;
 template <> struct RsCfg<uint32_t> { static constexpr int IPT = 16; };
@@ -308,11 +310,45 @@ __host__ __device__ __forceinline__ uint32_t rs_digit_mask(uint32_t key_bits, in
   return rem >= rb ? (1u << rb) - 1u : (rem <= 0 ? 0u : (1u << rem) - 1u);
 }
 
-// Global digit histograms of all passes in one read of the keys.
+// Exclusive scans of `rows` histograms of RADIX bins, each starting at its
+// segment's base, by the block of a histogram launch that finishes last (a
+// launch of its own cost a node of the step's graph): true in that block.
+__device__ __forceinline__ bool rs_last_block(unsigned* done) {
+  __shared__ bool s_last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) == gridDim.x * gridDim.y - 1;
+  __syncthreads();
+  if (s_last) __threadfence();
+  return s_last;
+}
+template <int RADIX>
+__device__ __forceinline__ void rs_scan_rows(uint32_t* hist, uint32_t rows, uint32_t n_segs, uint32_t seg_len) {
+  constexpr int PER = RADIX / 32;
+  const int lane = threadIdx.x & 31;
+  for (uint32_t row = threadIdx.x >> 5; row < rows; row += RS_WARPS) {
+    uint32_t* h = hist + (size_t)row * RADIX + lane * PER;
+    uint32_t x[PER], sum = 0;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) { x[k] = __ldcg(h + k); sum += x[k]; }
+    uint32_t incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += y;
+    }
+    uint32_t run = incl - sum + (row % n_segs) * seg_len;
+#pragma unroll
+    for (int k = 0; k < PER; ++k) { h[k] = run; run += x[k]; }
+  }
+}
+
+// Global digit histograms of all passes in one read of the keys, scanned.
 template <typename K, int RB>
 __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const K* __restrict__ keys, uint64_t n_cap,
                                                         const uint64_t* __restrict__ d_n, int passes,
-                                                        uint32_t key_bits, uint32_t* __restrict__ hist /* passes x RADIX */) {
+                                                        uint32_t key_bits, uint32_t* __restrict__ hist /* passes x RADIX */,
+                                                        unsigned* __restrict__ done) {
   constexpr int RADIX = Rdx<RB>::RADIX;
   __shared__ uint32_t sh[RS_MAX_PASSES * RADIX];
   for (int t = threadIdx.x; t < passes * RADIX; t += RS_THREADS) sh[t] = 0;
@@ -342,24 +378,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const K* __restrict__ ke
     const uint32_t c = sh[t];
     if (c) atomicAdd(&hist[t], c);
   }
-}
-
-// exclusive scan of each pass's RADIX bins (one block of RADIX threads per pass)
-template <int RB>
-__global__ void __launch_bounds__(1 << RB) k_rs_hist_scan(uint32_t* __restrict__ hist) {
-  constexpr int RADIX = Rdx<RB>::RADIX;
-  __shared__ uint32_t s[RADIX];
-  uint32_t* h = hist + blockIdx.x * RADIX;
-  const uint32_t v = h[threadIdx.x];
-  s[threadIdx.x] = v;
-  __syncthreads();
-  for (int o = 1; o < RADIX; o <<= 1) {
-    uint32_t y = threadIdx.x >= (unsigned)o ? s[threadIdx.x - o] : 0u;
-    __syncthreads();
-    s[threadIdx.x] += y;
-    __syncthreads();
-  }
-  h[threadIdx.x] = s[threadIdx.x] - v;
+  if (rs_last_block(done)) rs_scan_rows<RADIX>(hist, (uint32_t)passes, 1u, 0u);
 }
 
 template <typename K, int RB>
@@ -637,10 +656,9 @@ static sc_status radix_passes(sc_ctx* ctx, K* keys, uint32_t* vals, K* keys_tmp,
   SC_CUDA_TRY(ctx, cudaMemsetAsync(scratch, 0, need, ctx->stream), "memset radix scratch");
   const unsigned hist_blocks = (unsigned)std::min<uint64_t>(sc_div_up(n_cap, RS_THREADS),
                                                             (uint64_t)ctx->sm_count * RS_HIST_BLOCKS_PER_SM);
-  k_rs_hist<K, RB><<<hist_blocks, RS_THREADS, 0, ctx->stream>>>(keys, n_cap, d_n, passes, key_bits, hist);
+  k_rs_hist<K, RB><<<hist_blocks, RS_THREADS, 0, ctx->stream>>>(keys, n_cap, d_n, passes, key_bits, hist,
+                                                                tickets + RS_DONE);
   SC_TRY(sc_check_launch(ctx, "k_rs_hist"));
-  k_rs_hist_scan<RB><<<passes, RADIX, 0, ctx->stream>>>(hist);
-  SC_TRY(sc_check_launch(ctx, "k_rs_hist_scan"));
   const size_t smem = sizeof(RsSmem<K, RB>);
   static bool attr_set = false;
   if (!attr_set) {
@@ -707,7 +725,8 @@ sc_status radix_sort(sc_ctx* ctx, K* keys, uint32_t* vals, K* keys_tmp, uint32_t
 template <int RB>
 __global__ void __launch_bounds__(RS_THREADS) k_rs_hist_seg(const uint32_t* __restrict__ keys, uint32_t seg_len,
                                                             uint32_t n_segs, int passes, uint32_t key_bits,
-                                                            uint32_t* __restrict__ hist /* [passes][n_segs][RADIX] */) {
+                                                            uint32_t* __restrict__ hist /* [passes][n_segs][RADIX] */,
+                                                            unsigned* __restrict__ done) {
   constexpr int RADIX = Rdx<RB>::RADIX;
   __shared__ uint32_t sh[4 * RADIX];
   for (int t = threadIdx.x; t < passes * RADIX; t += RS_THREADS) sh[t] = 0;
@@ -735,26 +754,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_hist_seg(const uint32_t* __re
     const uint32_t c = sh[t];
     if (c) atomicAdd(&hist[((size_t)(t / RADIX) * n_segs + g) * RADIX + t % RADIX], c);
   }
-}
-
-// exclusive scan of each (pass, segment) histogram plus the segment's base
-template <int RB>
-__global__ void __launch_bounds__(1 << RB) k_rs_hist_scan_seg(uint32_t* __restrict__ hist, uint32_t n_segs,
-                                                              uint32_t seg_len) {
-  constexpr int RADIX = Rdx<RB>::RADIX;
-  __shared__ uint32_t s[RADIX];
-  uint32_t* h = hist + (size_t)blockIdx.x * RADIX;
-  const uint32_t base = (blockIdx.x % n_segs) * seg_len;
-  const uint32_t v = h[threadIdx.x];
-  s[threadIdx.x] = v;
-  __syncthreads();
-  for (int o = 1; o < RADIX; o <<= 1) {
-    uint32_t y = threadIdx.x >= (unsigned)o ? s[threadIdx.x - o] : 0u;
-    __syncthreads();
-    s[threadIdx.x] += y;
-    __syncthreads();
-  }
-  h[threadIdx.x] = base + s[threadIdx.x] - v;
+  if (rs_last_block(done)) rs_scan_rows<RADIX>(hist, (uint32_t)passes * n_segs, n_segs, seg_len);
 }
 
 template <bool NARROW>
@@ -781,14 +781,14 @@ __global__ void __launch_bounds__(RS_THREADS, 4) k_rs_pass_seg(const uint32_t* _
                                           lookback + (size_t)g * tiles_per_seg * RADIX, err, local, tbase, dbits);
 }
 
-size_t radix_seg_scratch_bytes(uint64_t seg_len, uint32_t n_segs) {
-  const uint64_t tiles = sc_div_up(seg_len, RS_SEG_TILE) * n_segs;
-  return (size_t)4 * n_segs * 256 * 4 + 64 + (size_t)4 * tiles * 256 * 4;
+size_t radix_seg_scratch_bytes(uint64_t seg_len, uint32_t n_segs, uint32_t key_bits) {
+  const uint64_t tiles = sc_div_up(seg_len, RS_SEG_TILE) * n_segs, passes = (key_bits + 7) / 8;
+  return (size_t)passes * n_segs * 256 * 4 + 64 + (size_t)passes * tiles * 256 * 4;
 }
 
 sc_status radix_sort_segments(sc_ctx* ctx, uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint32_t* vals_tmp,
                               uint32_t seg_len, uint32_t n_segs, uint32_t key_bits, void* scratch, size_t bytes,
-                              bool* result_in_tmp) {
+                              bool* result_in_tmp, bool clean) {
   constexpr int RB = 8, RADIX = 256;
   *result_in_tmp = false;
   const uint64_t n = (uint64_t)seg_len * n_segs;
@@ -805,13 +805,12 @@ sc_status radix_sort_segments(sc_ctx* ctx, uint32_t* keys, uint32_t* vals, uint3
   uint32_t* hist = reinterpret_cast<uint32_t*>(scratch);
   unsigned* tickets = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(scratch) + hist_bytes);
   unsigned* lookback = reinterpret_cast<unsigned*>(reinterpret_cast<char*>(scratch) + hist_bytes + 64);
-  SC_CUDA_TRY(ctx, cudaMemsetAsync(scratch, 0, need, ctx->stream), "memset radix scratch");
+  if (!clean) SC_CUDA_TRY(ctx, cudaMemsetAsync(scratch, 0, need, ctx->stream), "memset radix scratch");
   const unsigned bx = (unsigned)std::max<uint64_t>(
       1, std::min<uint64_t>(sc_div_up(seg_len, RS_THREADS), (uint64_t)ctx->sm_count * RS_HIST_BLOCKS_PER_SM / n_segs));
-  k_rs_hist_seg<RB><<<dim3(bx, n_segs), RS_THREADS, 0, ctx->stream>>>(keys, seg_len, n_segs, passes, key_bits, hist);
+  k_rs_hist_seg<RB><<<dim3(bx, n_segs), RS_THREADS, 0, ctx->stream>>>(keys, seg_len, n_segs, passes, key_bits, hist,
+                                                                      tickets + RS_DONE);
   SC_TRY(sc_check_launch(ctx, "k_rs_hist_seg"));
-  k_rs_hist_scan_seg<RB><<<(unsigned)(passes * n_segs), RADIX, 0, ctx->stream>>>(hist, n_segs, seg_len);
-  SC_TRY(sc_check_launch(ctx, "k_rs_hist_scan_seg"));
   const size_t smem = sizeof(RsSmem<uint32_t, RB>);
   static bool attr_set = false;
   if (!attr_set) {

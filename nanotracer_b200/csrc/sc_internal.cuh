@@ -452,9 +452,11 @@ sc_status launch_unpack_moments(sc_ctx* ctx, const DMoments& mo, uint32_t n, con
 // scan / sort
 sc_status scan_u32(sc_ctx* ctx, uint32_t* data, uint64_t n, uint64_t* d_total, void* scratch, size_t scratch_bytes);
 // the same exclusive scan of out[0..n), out[i] = src[(i / seg) seg + idx[i]]
-// for i < gn and 0 beyond (seg a multiple of 16), gathered as it is read
+// for i < gn and 0 beyond (seg a multiple of 16), gathered as it is read.
+// clean (here and below): the caller has zeroed the scratch on the stream.
 sc_status scan_u32_gather(sc_ctx* ctx, uint32_t* out, uint64_t n, const uint32_t* src, const uint32_t* idx,
-                          uint32_t seg, uint64_t gn, uint64_t* d_total, void* scratch, size_t scratch_bytes);
+                          uint32_t seg, uint64_t gn, uint64_t* d_total, void* scratch, size_t scratch_bytes,
+                          bool clean = false);
 size_t scan_scratch_bytes(uint64_t n);
 template <typename K>
 sc_status radix_sort(sc_ctx* ctx, K* keys, uint32_t* vals, K* keys_tmp, uint32_t* vals_tmp, uint64_t n,
@@ -466,8 +468,8 @@ size_t radix_scratch_bytes(uint64_t n, uint32_t key_bytes);
 constexpr uint32_t RADIX_SEG_TILE = 4096;
 sc_status radix_sort_segments(sc_ctx* ctx, uint32_t* keys, uint32_t* vals, uint32_t* keys_tmp, uint32_t* vals_tmp,
                               uint32_t seg_len, uint32_t n_segs, uint32_t key_bits, void* scratch, size_t bytes,
-                              bool* result_in_tmp);
-size_t radix_seg_scratch_bytes(uint64_t seg_len, uint32_t n_segs);
+                              bool* result_in_tmp, bool clean = false);
+size_t radix_seg_scratch_bytes(uint64_t seg_len, uint32_t n_segs, uint32_t key_bits);
 // one look-back pass whose predecessor never publishes (bounded-wait self-test)
 sc_status selftest_lookback_timeout(sc_ctx* ctx);
 
@@ -482,7 +484,8 @@ sc_status launch_tile_emit(sc_ctx* ctx, const float4* rec, uint32_t n, uint32_t 
 // whose set bits are added to *high_popc when it is given)
 sc_status launch_tile_ranges(sc_ctx* ctx, const void* keys, int key_mode, const uint64_t* d_total, uint64_t cap,
                              uint32_t num_tiles, uint32_t* ranges, uint32_t tiles_per_view = 0,
-                             uint32_t tile_bits = 0, uint32_t key_bits = 32, uint64_t* high_popc = nullptr);
+                             uint32_t tile_bits = 0, uint32_t key_bits = 32, uint64_t* high_popc = nullptr,
+                             bool clean = false);
 // depth-presorted emission for the native pipeline
 sc_status launch_presorted_emit(sc_ctx* ctx, const float4* rec, uint32_t stride, uint32_t n_views,
                                 const uint32_t* sorted_ids, const uint32_t* offsets, const uint32_t* counts_by_id,
@@ -505,7 +508,7 @@ uint32_t super_tiles_per_view(const sc_tiling* tl);
 // drawn from TAKER_POOLS counters (zeroed by the caller before the forward), pool p
 // holding chunks [p pool_cap, (p + 1) pool_cap); a pool that runs out raises
 // SC_DEVERR_TAKERS and goes on counting.
-constexpr uint32_t TAKER_POOLS = 64;
+constexpr uint32_t TAKER_POOLS = 64;  // a power of two
 struct TakerChunks {
   uint32_t* ids;    // TAKER_POOLS x pool_cap x 32
   uint32_t* prev;   // TAKER_POOLS x pool_cap

@@ -47,11 +47,19 @@ struct StepOut {
 };
 
 // loss = mean over the views, or (weight > 0) weight * sum over the views, of
-// (1 - lambda) MSE + lambda (1 - SSIM) (loss.rs:383-410; MSE alone without SSIM sums)
+// (1 - lambda) MSE + lambda (1 - SSIM) (loss.rs:383-410; MSE alone without SSIM sums).
+// One warp; out and losses (nullable, the views' sums) are page-locked host
+// memory, which the host reads after the step's synchronize.
 __global__ void k_finalize(const double* __restrict__ loss_sums, const double* __restrict__ ssim_sums, float lambda,
                            uint32_t n_views, double inv_count, double weight, const uint64_t* __restrict__ d_total,
                            const uint32_t* __restrict__ err, const uint32_t* __restrict__ drawn,
-                           StepOut* __restrict__ out) {
+                           StepOut* __restrict__ out, double* __restrict__ losses) {
+  uint32_t most = 0;
+  for (uint32_t p = threadIdx.x; p < sck::TAKER_POOLS; p += 32) most = max(most, drawn[p]);
+  most = __reduce_max_sync(0xffffffffu, most);
+  if (losses)
+    for (uint32_t v = threadIdx.x; v < n_views; v += 32) losses[v] = loss_sums[v];
+  if (threadIdx.x != 0) return;
   double acc = 0.0;
   for (uint32_t v = 0; v < n_views; ++v) {
     const double m = loss_sums[v] * inv_count;
@@ -63,8 +71,6 @@ __global__ void k_finalize(const double* __restrict__ loss_sums, const double* _
   out->pairs = d_total[0];
   out->items = d_total[1];
   out->err = *err;
-  uint32_t most = 0;
-  for (uint32_t p = 0; p < sck::TAKER_POOLS; ++p) most = max(most, drawn[p]);
   out->chunks = most;
 }
 
@@ -91,8 +97,7 @@ struct sc_trainer {
   uint32_t stride = 0;
   StepParams* h_params = nullptr;
   StepParams* d_params = nullptr;
-  StepOut* h_out = nullptr;
-  StepOut* d_out = nullptr;
+  StepOut* h_out = nullptr;  // page-locked, written by the step's last kernel
   // per (view, splat)
   float4* rec = nullptr; float4* pgrad = nullptr;
   float4* pcomp = nullptr;  // compensation records of pgrad (cfg.compensated_sums)
@@ -127,8 +132,14 @@ struct sc_trainer {
   cudaEvent_t ev_bwd[SC_MAX_VIEWS] = {};
   // exact backward: the forward's takers (ids, prev, head, drawn)
   sck::TakerChunks takers{};
+  // one block that every step zeroes first, in one go (a fill per array cost a
+  // node of the graph each): loss sums, totals, the pools' counters, the
+  // super tiles' (or tiles') ranges and the depth sort's and scan's scratch
+  void* zero = nullptr; size_t zero_bytes = 0;
   double* d_loss = nullptr;
   uint64_t* d_total = nullptr;
+  void* seg_scratch = nullptr; size_t seg_bytes = 0;
+  void* scan_scratch = nullptr; size_t scan_bytes = 0;
   void* scratch = nullptr; size_t scratch_bytes = 0;
   // gradient-only steps (data-parallel views): shard-major output
   bool grads_mode = false;
@@ -198,19 +209,45 @@ static void trainer_drop_graph(sc_trainer* tr) {
 
 static sc_status ensure_scratch(sc_trainer* tr) {
   sc_ctx* ctx = tr->ctx;
-  const uint64_t nsp = (uint64_t)tr->V * tr->stride;
-  size_t need = std::max({sck::radix_seg_scratch_bytes(tr->stride, tr->V),
-                          sck::radix_scratch_bytes(std::max<uint64_t>(tr->kcap, 1), 4),
-                          sck::radix_scratch_bytes(std::max<uint64_t>(tr->icap, 1), 4), sck::scan_scratch_bytes(nsp + 1),
-                          sck::scan_scratch_bytes((uint64_t)tr->V * tr->T + 1)});
+  size_t need = std::max(sck::radix_scratch_bytes(std::max<uint64_t>(tr->kcap, 1), 4),
+                         sck::radix_scratch_bytes(std::max<uint64_t>(tr->icap, 1), 4));
   if (need <= tr->scratch_bytes) return SC_OK;
   SC_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "sync");
   cudaFree(tr->scratch);
   tr->scratch = nullptr;
+  tr->scratch_bytes = 0;
   need = need + need / 4;
   SC_CUDA_TRY(ctx, cudaMalloc(&tr->scratch, need), "trainer scratch");
   tr->scratch_bytes = need;
   trainer_drop_graph(tr);
+  return SC_OK;
+}
+
+// the block of a step's zeroed arrays, for the current stride
+static sc_status ensure_zero_block(sc_trainer* tr) {
+  sc_ctx* ctx = tr->ctx;
+  const uint64_t nsp = (uint64_t)tr->V * tr->stride;
+  size_t off = 0;
+  auto take = [&](size_t b) { const size_t o = off; off += (b + 255) & ~(size_t)255; return o; };
+  const size_t o_loss = take(8 * (size_t)tr->V), o_ssim = take(8 * (size_t)tr->V), o_total = take(16),
+               o_drawn = take(sck::TAKER_POOLS * 4),
+               o_ranges = take((size_t)tr->V * (tr->two_level ? tr->ST : tr->T) * 8),
+               o_scan = take(sck::scan_scratch_bytes(nsp + 1)),
+               o_seg = take(sck::radix_seg_scratch_bytes(tr->stride, tr->V, 16));
+  cudaFree(tr->zero);
+  tr->zero = nullptr;
+  SC_CUDA_TRY(ctx, cudaMalloc(&tr->zero, off), "zeroed arrays");
+  tr->zero_bytes = off;
+  char* z = reinterpret_cast<char*>(tr->zero);
+  tr->d_loss = reinterpret_cast<double*>(z + o_loss);
+  tr->d_ssim = reinterpret_cast<double*>(z + o_ssim);
+  tr->d_total = reinterpret_cast<uint64_t*>(z + o_total);
+  tr->takers.drawn = reinterpret_cast<uint32_t*>(z + o_drawn);
+  (tr->two_level ? tr->iranges : tr->ranges) = reinterpret_cast<uint32_t*>(z + o_ranges);
+  tr->scan_scratch = z + o_scan;
+  tr->scan_bytes = o_seg - o_scan;
+  tr->seg_scratch = z + o_seg;
+  tr->seg_bytes = off - o_seg;
   return SC_OK;
 }
 
@@ -237,6 +274,11 @@ static sc_status ensure_splat_arrays(sc_trainer* tr, uint32_t cap) {
   SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->rec, 0, nv * 48, ctx->stream), "zero");
   tr->stride = cap;
   trainer_drop_graph(tr);
+  const sc_status st = ensure_zero_block(tr);
+  if (st != SC_OK) {
+    tr->stride = 0;  // the next step allocates again
+    return st;
+  }
   return ensure_scratch(tr);
 }
 
@@ -338,13 +380,11 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
       SC_CUDA_TRY(ctx, cudaEventRecord(tr->ev_view[v], tr->copy_stream), "copied");
     }
   }
-  // the loss sums and, behind them, the taker pools' counters
-  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->d_loss, 0, 8 * (size_t)V + sck::TAKER_POOLS * 4, ctx->stream), "zero loss");
+  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->zero, 0, tr->zero_bytes, ctx->stream), "zero");
   uint64_t* work_fwd = tr->profiling ? tr->d_work : nullptr;
   uint64_t* work_bwd = tr->profiling ? tr->d_work + 3 * sck::BLEND_WORK_SLOTS : nullptr;
   if (tr->profiling)
     SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->d_work, 0, 6 * sck::BLEND_WORK_SLOTS * 8, ctx->stream), "zero work");
-  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->counts + nsp, 0, 4, ctx->stream), "zero count tail");
   mark(tr, 0, capturing);
   SC_TRY(sck::launch_project(ctx, ds, d_cams, V, tr->stride, tr->rec, &tr->cfg.tiling, tr->dkeys, tr->ids,
                              tr->counts_by_id, tr->cfg.fp64_det ? 1 : 0,
@@ -352,8 +392,8 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
                              tr->scenes_mode ? tr->d_scenes : nullptr));
   mark(tr, 1, capturing);
   bool in_tmp = false;
-  SC_TRY(sck::radix_sort_segments(ctx, tr->dkeys, tr->ids, tr->dkeys_tmp, tr->ids_tmp, tr->stride, V, 16, tr->scratch,
-                                  tr->scratch_bytes, &in_tmp));
+  SC_TRY(sck::radix_sort_segments(ctx, tr->dkeys, tr->ids, tr->dkeys_tmp, tr->ids_tmp, tr->stride, V, 16,
+                                  tr->seg_scratch, tr->seg_bytes, &in_tmp, true));
   const uint32_t* sorted_ids = in_tmp ? tr->ids_tmp : tr->ids;
   mark(tr, 2, capturing);
   const uint32_t all_tiles = V * tr->T;
@@ -368,7 +408,7 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
     uint64_t* d_items = tr->d_total + 1;
     // item counts in depth order (gathered through the sorted ids) -> offsets
     SC_TRY(sck::scan_u32_gather(ctx, tr->counts, nsp + 1, tr->counts_by_id, sorted_ids, tr->stride, nsp, d_items,
-                                tr->scratch, tr->scratch_bytes));
+                                tr->scan_scratch, tr->scan_bytes, true));
     if (sizing) {
       uint64_t I = 0;
       SC_CUDA_TRY(ctx, cudaMemcpyAsync(&I, d_items, 8, cudaMemcpyDeviceToHost, ctx->stream), "items");
@@ -385,12 +425,11 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
     item_ids = in_tmp ? tr->ivals_tmp : tr->ivals;
     mark(tr, 5, capturing);
     // the super tiles' ranges; the member bits of the masks add up to the pair count
-    SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->d_total, 0, 8, ctx->stream), "zero pairs");
     SC_TRY(sck::launch_tile_ranges(ctx, item_keys, 2, d_items, tr->icap, V * tr->ST, tr->iranges, tr->ST,
-                                   tr->super_bits, tr->super_bits + bits_for(V - 1), tr->d_total));
+                                   tr->super_bits, tr->super_bits + bits_for(V - 1), tr->d_total, true));
   } else {
   SC_TRY(sck::scan_u32_gather(ctx, tr->counts, nsp + 1, tr->counts_by_id, sorted_ids, tr->stride, nsp, tr->d_total,
-                              tr->scratch, tr->scratch_bytes));
+                              tr->scan_scratch, tr->scan_bytes, true));
   if (sizing) {
     uint64_t K = 0;
     SC_CUDA_TRY(ctx, cudaMemcpyAsync(&K, tr->d_total, 8, cudaMemcpyDeviceToHost, ctx->stream), "K");
@@ -410,7 +449,8 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
   const uint32_t* skeys = in_tmp ? tr->keys_tmp : tr->keys;
   svals = in_tmp ? tr->vals_tmp : tr->vals;
   mark(tr, 5, capturing);
-  SC_TRY(sck::launch_tile_ranges(ctx, skeys, 2, tr->d_total, tr->kcap, all_tiles, tr->ranges, tr->T, tile_bits));
+  SC_TRY(sck::launch_tile_ranges(ctx, skeys, 2, tr->d_total, tr->kcap, all_tiles, tr->ranges, tr->T, tile_bits,
+                                 32, nullptr, true));
   }
   mark(tr, 6, capturing);
   const float weight = tr->grads_mode ? tr->loss_weight : 1.0f / (float)V;
@@ -431,7 +471,6 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
     SC_TRY(sck::launch_composite(ctx, tr->rec, tr->stride, V, svals, tr->ranges, &tr->cfg.tiling, tr->image, tr->aux,
                                  fwd_target, mse_w, tr->dl_dc, tr->d_loss, ctx->d_error, takers));
   if (lam > 0.0f) {
-    SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->d_ssim, 0, 8 * (size_t)V, ctx->stream), "zero ssim");
     SC_TRY(sck::launch_ssim(ctx, tr->image, tr->targets, tr->cfg.tiling.width, tr->cfg.tiling.height, V,
                             weight * lam, tr->dl_dc, tr->d_ssim, tr->ssim_terms));
   }
@@ -499,14 +538,11 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
     SC_TRY(sck::launch_adam_rows(ctx, ds, dm, acc, tr->grads, 0, ds.n, tr->grad_stride, ap, d_bc, ctx->d_error));
   }
   mark(tr, 9, capturing);
-  k_finalize<<<1, 1, 0, ctx->stream>>>(tr->d_loss, lam > 0.0f ? tr->d_ssim : nullptr, lam, V,
-                                       1.0 / (3.0 * (double)tr->P), tr->grads_mode ? (double)tr->loss_weight : 0.0,
-                                       tr->d_total, ctx->d_error, tr->takers.drawn, tr->d_out);
+  k_finalize<<<1, 32, 0, ctx->stream>>>(tr->d_loss, lam > 0.0f ? tr->d_ssim : nullptr, lam, V,
+                                        1.0 / (3.0 * (double)tr->P), tr->grads_mode ? (double)tr->loss_weight : 0.0,
+                                        tr->d_total, ctx->d_error, tr->takers.drawn, tr->h_out,
+                                        tr->scenes_mode ? tr->h_losses : nullptr);
   SC_TRY(sc_check_launch(ctx, "k_finalize"));
-  SC_CUDA_TRY(ctx, cudaMemcpyAsync(tr->h_out, tr->d_out, sizeof(StepOut), cudaMemcpyDeviceToHost, ctx->stream), "out D2H");
-  if (tr->scenes_mode)
-    SC_CUDA_TRY(ctx, cudaMemcpyAsync(tr->h_losses, tr->d_loss, 8 * (size_t)V, cudaMemcpyDeviceToHost, ctx->stream),
-                "losses D2H");
   tr->kernels_per_step = (uint32_t)(ctx->launches - launches0);
   return SC_OK;
 }
@@ -558,29 +594,22 @@ sc_status sc_trainer_create(sc_ctx* ctx, const sc_train_config* cfg, sc_trainer*
   cudaError_t e = cudaMallocHost(&tr->h_params, sizeof(StepParams));
   if (e == cudaSuccess) e = cudaMallocHost(&tr->h_out, sizeof(StepOut));
   if (e == cudaSuccess) e = cudaMalloc(&tr->d_params, sizeof(StepParams));
-  if (e == cudaSuccess) e = cudaMalloc(&tr->d_out, sizeof(StepOut));
-  if (e == cudaSuccess) e = cudaMalloc(&tr->ranges, (size_t)tr->V * tr->T * 8);
   if (e == cudaSuccess) e = cudaMalloc(&tr->image, pix * 16);
   if (e == cudaSuccess) e = cudaMalloc(&tr->aux, pix * 8);
   if (e == cudaSuccess) e = cudaMalloc(&tr->dl_dc, pix * 16);
-  if (e == cudaSuccess) e = cudaMalloc(&tr->d_loss, 8 * (size_t)tr->V + sck::TAKER_POOLS * 4);
   const size_t heads = (size_t)tr->V * tr->T * sck::blend_warps_per_tile(&t);
   if (e == cudaSuccess && cfg->bwd_mode == SC_BWD_EXACT) e = cudaMalloc(&tr->takers.head, heads * sizeof(uint2));
   if (e == cudaSuccess) e = cudaMalloc(&tr->d_work, 6 * sck::BLEND_WORK_SLOTS * 8);
-  if (e == cudaSuccess) e = cudaMalloc(&tr->d_total, 64);
-  if (e == cudaSuccess) e = cudaMemset(tr->d_total, 0, 64);
-  if (e == cudaSuccess && tr->two_level) e = cudaMalloc(&tr->iranges, (size_t)tr->V * tr->ST * 8);
   if (e == cudaSuccess && cfg->ssim_lambda > 0.0f) e = cudaMalloc(&tr->ssim_terms, sck::ssim_terms_bytes(tr->P, tr->V));
-  if (e == cudaSuccess && cfg->ssim_lambda > 0.0f) e = cudaMalloc(&tr->d_ssim, 8 * (size_t)tr->V);
   for (int i = 0; i <= kStages && e == cudaSuccess; ++i) e = cudaEventCreate(&tr->ev[i]);
   if (e != cudaSuccess) {
     sc_trainer_free(ctx, tr);
     return sc_cuda_fail(ctx, e, "trainer alloc");
   }
   std::memset(tr->h_params, 0, sizeof(StepParams));
-  tr->takers.drawn = reinterpret_cast<uint32_t*>(tr->d_loss + tr->V);
-  // a first guess of 4 chunks a warp; a step that draws more runs again with the number it needs
-  const sc_status st = ensure_takers(tr, sc_div_up(4 * heads, sck::TAKER_POOLS) + 1);
+  // a first guess of 5 chunks a warp and a quarter more; a step that draws more
+  // runs again with the number it needs
+  const sc_status st = ensure_takers(tr, sc_div_up(5 * heads, sck::TAKER_POOLS) + 1);
   if (st != SC_OK) {
     sc_trainer_free(ctx, tr);
     return st;
@@ -596,11 +625,10 @@ void sc_trainer_free(sc_ctx* ctx, sc_trainer* tr) {
   trainer_free_splat_arrays(tr);
   trainer_free_pairs(tr);
   trainer_free_items(tr);
-  cudaFree(tr->iranges);
   cudaFree(tr->takers.ids); cudaFree(tr->takers.prev); cudaFree(tr->takers.head);
-  cudaFree(tr->ranges); cudaFree(tr->image); cudaFree(tr->aux); cudaFree(tr->dl_dc);
-  cudaFree(tr->d_loss); cudaFree(tr->d_work); cudaFree(tr->d_total); cudaFree(tr->d_params); cudaFree(tr->d_out);
-  cudaFree(tr->ssim_terms); cudaFree(tr->d_ssim);
+  cudaFree(tr->zero); cudaFree(tr->image); cudaFree(tr->aux); cudaFree(tr->dl_dc);
+  cudaFree(tr->d_work); cudaFree(tr->d_params);
+  cudaFree(tr->ssim_terms);
   cudaFree(tr->d_host_targets);
   if (tr->copy_stream) cudaStreamDestroy(tr->copy_stream);
   if (tr->ev_fork) cudaEventDestroy(tr->ev_fork);
