@@ -136,7 +136,9 @@ __device__ __forceinline__ bool eval_alpha(const EntryGeom& e, float c, float dy
 }
 
 // The same for a thread's two pixels (rows fy.x, fy.y of one column) with
-// packed arithmetic; v0, v1 are the per-pixel results of eval_alpha.
+// packed arithmetic; v0, v1 are the per-pixel results of eval_alpha.  PLAIN:
+// the record is plain_record, whose other two tests cannot fail.
+template <bool PLAIN>
 __device__ __forceinline__ void eval_alpha2(const EntryGeom& e, float c, float2 fy, float ry, float op, float2& dy,
                                             float2& g, float2& alpha_raw, float2& alpha, bool& v0, bool& v1) {
   dy = __fadd2_rn(fy, f2(-ry));
@@ -144,9 +146,9 @@ __device__ __forceinline__ void eval_alpha2(const EntryGeom& e, float c, float2 
   const float2 ex = __fmul2_rn(quad, f2(NEG_HALF_LOG2E));
   g = make_float2(ex2_approx(ex.x), ex2_approx(ex.y));
   alpha_raw = __fmul2_rn(f2(op), g);
-  alpha = make_float2(fminf(alpha_raw.x, ALPHA_MAX), fminf(alpha_raw.y, ALPHA_MAX));
-  v0 = quad.x >= 0.0f && alpha.x >= ALPHA_MIN;
-  v1 = quad.y >= 0.0f && alpha.y >= ALPHA_MIN;
+  alpha = PLAIN ? alpha_raw : make_float2(fminf(alpha_raw.x, ALPHA_MAX), fminf(alpha_raw.y, ALPHA_MAX));
+  v0 = (PLAIN || quad.x >= 0.0f) && alpha.x >= ALPHA_MIN;
+  v1 = (PLAIN || quad.y >= 0.0f) && alpha.y >= ALPHA_MIN;
 }
 
 template <typename T>
@@ -220,6 +222,18 @@ __device__ __forceinline__ uint2 list_range(const ListArgs& l, const BlendArgs& 
   }
   bit = (ty % SC_SUPER) * SC_SUPER + tx % SC_SUPER;
   return l.ranges[(size_t)v * l.super_per_view + (ty / SC_SUPER) * l.super_x + tx / SC_SUPER];
+}
+
+// A record whose pairs need only the alpha >= 1/255 test: finite and of ordinary
+// size, its conic well away from singular (det > 2^-10 a c, so that the quadratic form,
+// at least 2^-11 of its terms' magnitudes, cannot round below zero), and its
+// opacity below 0.99, so that no alpha reaches the clamp.  The backward walks a
+// stage of such entries without the other tests (1M splats, 8 views of 1080p: 1.405 -> 1.355
+// ms with the 8 rows unrolled; the forward gained under 1 % and tests all).
+__device__ __forceinline__ bool plain_record(const float4 ra, const float4 rb, float op) {
+  const float det = rb.x * rb.z - rb.y * rb.y;
+  return fabsf(ra.x) < 1e6f && fabsf(ra.y) < 1e6f && rb.x > 0.0f && rb.z > 0.0f && rb.x < 1e6f && rb.z < 1e6f &&
+         det > 9.765625e-4f * (rb.x * rb.z) && op < ALPHA_MAX;
 }
 
 // How a warp gets its entries, in stages of up to 32: gather() starts the copies
@@ -585,7 +599,7 @@ __global__ void __launch_bounds__(256) k_composite(const float4* __restrict__ re
           // alpha 0, which leaves its colour and T bit for bit unchanged
           float2 dy, g, araw, al;
           bool v0, v1;
-          eval_alpha2(e, rb.z, fy2, ra.y, rc.w, dy, g, araw, al, v0, v1);
+          eval_alpha2<false>(e, rb.z, fy2, ra.y, rc.w, dy, g, araw, al, v0, v1);
           v0 &= T2.x >= 1e-4f;
           v1 &= T2.y >= 1e-4f;
           const float2 am = make_float2(v0 ? al.x : 0.0f, v1 ? al.y : 0.0f);
@@ -1002,6 +1016,12 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
       sm.red.rg[oq * 9 + oe] = make_float4(gr[0], gr[PPT - 1], gg[0], gg[PPT - 1]);
       sm.red.b[oq * 9 + oe] = make_float2(gb[0], gb[PPT - 1]);
     }
+    // the positions below lo0 are behind no pixel's last contributor; none with a
+    // pixel outside the image, whose walk must stay empty
+    uint32_t low = stop[0];
+#pragma unroll
+    for (int q = 1; q < PPT; ++q) low = min(low, stop[q]);
+    const uint32_t lo0 = MODE == SC_BWD_EXACT ? __reduce_min_sync(FULL_MASK, low) : 0u;
     FEED feed = [&]() {
       if constexpr (LIST == LIST_TAKERS) return TakerFeed(sm.feed, takers, vrec, head);
       else return ListFeed<LIST, true>(sm.feed, l, vrec, begin, hi0, bit, STAGE);
@@ -1038,15 +1058,20 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
     // pixel skips it).  Alpha is carried negated, which needs no negations in
     // the packed operations; a skipping pixel gets alpha 0, so it keeps its T
     // (1 / 1 is exact) and its sums.
-    auto entry2 = [&](uint32_t i, const float4* r) -> float4 {
-      const uint32_t j = feed.pos(i);
+    // `plain`: the stage's records are plain and no pixel of the warp stops
+    // behind its entries, which leaves the alpha >= 1/255 test alone.
+    auto entry2 = [&](auto plain, uint32_t i, const float4* r) -> float4 {
+      constexpr bool PLAIN = decltype(plain)::value;
       const float4 ra = r[0], rb = r[1], rc = r[2];
       const EntryGeom e = entry_geom(fx, ra, rb);
       float2 dy, g, araw, al;
       bool v0, v1;
-      eval_alpha2(e, rb.z, fy2, ra.y, rc.w, dy, g, araw, al, v0, v1);
-      v0 &= (MODE == SC_BWD_EXACT || !done[0]) && j < stop[0];
-      v1 &= (MODE == SC_BWD_EXACT || !done[PPT - 1]) && j < stop[PPT - 1];
+      eval_alpha2<PLAIN>(e, rb.z, fy2, ra.y, rc.w, dy, g, araw, al, v0, v1);
+      const uint32_t j = PLAIN ? 0u : feed.pos(i);
+      if (!PLAIN) {
+        v0 &= (MODE == SC_BWD_EXACT || !done[0]) && j < stop[0];
+        v1 &= (MODE == SC_BWD_EXACT || !done[PPT - 1]) && j < stop[PPT - 1];
+      }
       float2 am = make_float2(v0 ? -al.x : 0.0f, v1 ? -al.y : 0.0f);
       const float2 oma = __fadd2_rn(f2(1.0f), am);
       const float2 inv = make_float2(rcp_approx(oma.x), rcp_approx(oma.y));
@@ -1055,7 +1080,8 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
         if (v0 && Tn.x > 1.0001f) { done[0] = true; v0 = false; am.x = 0.0f; Tn.x = T2.x; }
         if (v1 && Tn.y > 1.0001f) { done[PPT - 1] = true; v1 = false; am.y = 0.0f; Tn.y = T2.y; }
       }
-      const float2 gm = make_float2(v0 && araw.x < ALPHA_MAX ? g.x : 0.0f, v1 && araw.y < ALPHA_MAX ? g.y : 0.0f);
+      const float2 gm = make_float2(v0 && (PLAIN || araw.x < ALPHA_MAX) ? g.x : 0.0f,
+                                    v1 && (PLAIN || araw.y < ALPHA_MAX) ? g.y : 0.0f);
       const float2 ta = __fmul2_rn(Tn, am);
       // dC/dalpha = T_i c - S / (1 - alpha) = (T_{i+1} c - S) / (1 - alpha)
       const float2 dc = make_float2(fmaf(gb2.x, rc.z, fmaf(gg2.x, rc.y, gr2.x * rc.x)),
@@ -1146,17 +1172,26 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
       uint32_t i = 0;
       if constexpr (OCT) {
         float4* row = sm.red.row + lane;
-        for (; i + OCT_E <= n && !stopped; i += OCT_E) {
-#pragma unroll 4
-          for (int e = 0; e < OCT_E; ++e) row[e * OCT_ROW] = entry2(i + e, sr + 3 * (i + e));
-          turn(i, OCT_E);
-          if (MODE == SC_BWD_REF) stopped = __all_sync(FULL_MASK, all_done);
+        auto walk = [&](auto plain) {
+          for (; i + OCT_E <= n && !stopped; i += OCT_E) {
+#pragma unroll
+            for (int e = 0; e < OCT_E; ++e) row[e * OCT_ROW] = entry2(plain, i + e, sr + 3 * (i + e));
+            turn(i, OCT_E);
+            if (MODE == SC_BWD_REF) stopped = __all_sync(FULL_MASK, all_done);
+          }
+          if (i < n && !stopped) {
+            for (uint32_t e = 0; i + e < n; ++e) row[e * OCT_ROW] = entry2(plain, i + e, sr + 3 * (i + e));
+            turn(i, n - i);
+            if (MODE == SC_BWD_REF) stopped = __all_sync(FULL_MASK, all_done);
+          }
+        };
+        bool plain = MODE == SC_BWD_EXACT && n > 0 && feed.pos(0) < lo0;
+        if (plain) {
+          const float4* r = sr + 3 * lane;
+          plain = __all_sync(FULL_MASK, lane >= (int)n || plain_record(r[0], r[1], r[2].w));
         }
-        if (i < n && !stopped) {
-          for (uint32_t e = 0; i + e < n; ++e) row[e * OCT_ROW] = entry2(i + e, sr + 3 * (i + e));
-          turn(i, n - i);
-          if (MODE == SC_BWD_REF) stopped = __all_sync(FULL_MASK, all_done);
-        }
+        if (plain) walk(std::true_type{});
+        else walk(std::false_type{});
       } else {
         // two entries together: one 18-value reduce-scatter
         for (; i < n && !stopped; i += 2) {
