@@ -322,6 +322,22 @@ sc_status sc_ctx_set_fp64_det(sc_ctx* ctx, int enabled);
 /* tonemap.wgsl:27-41 into a headless RGBA8 buffer (viewer path). */
 sc_status sc_tonemap(sc_ctx* ctx, const float* image, uint32_t width, uint32_t height, uint8_t* rgba8);
 
+/* The viewer's whole compute pass (crates/nano-view/src/lib.rs:762-795) as one
+ * blocking call: project -> bin -> composite -> tonemap, without the pair
+ * count's readback and with the binning of the trainer (the blended splats and
+ * their order, and so the image, are those of sc_bin's REF32 keys with depth_max).
+ * A view holds the working arrays of one tiling; at most 65536 tiles. */
+typedef struct sc_view sc_view;
+sc_status sc_view_create(sc_ctx* ctx, const sc_tiling* tiling, sc_view** out);
+void sc_view_free(sc_ctx* ctx, sc_view* v);
+/* records of `projected` that a frame of this store writes (at least its capacity) */
+uint32_t sc_view_records(const sc_splats* s);
+/* projected (sc_view_records records), image (width * height float4) and rgba8
+ * (nullable, width * height RGBA8) are device buffers; rgba8_host (nullable)
+ * receives a copy of rgba8. */
+sc_status sc_view_frame(sc_view* v, const sc_splats* s, const sc_camera* cam, float depth_max,
+                        sc_projected_splat* projected, float* image, uint8_t* rgba8, uint8_t* rgba8_host);
+
 /* ------------------------------------------------------------- optimiser
  * replaces AdamGpu (crates/nano-optimize/src/adam_gpu.rs:31-547) */
 sc_status sc_adam_step(sc_ctx* ctx, float* params, const float* grads, float* m, float* v, uint64_t n,

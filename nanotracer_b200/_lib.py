@@ -132,6 +132,10 @@ _PROTOS = {
     "sc_composite_backward_ex": (ST, [P, P, U32, U32, P, C.POINTER(sc_tiling), P, P, I32, P, P, U32]),
     "sc_project_backward": (ST, [P, P, P, P, P, I32]),
     "sc_tonemap": (ST, [P, P, U32, U32, P]),
+    "sc_view_create": (ST, [P, C.POINTER(sc_tiling), C.POINTER(P)]),
+    "sc_view_free": (None, [P, P]),
+    "sc_view_records": (U32, [P]),
+    "sc_view_frame": (ST, [P, P, C.POINTER(sc_camera), F32, P, P, P, P]),
     "sc_adam_step": (ST, [P, P, P, P, P, U64, F32, U64, C.POINTER(sc_adam_config)]),
     "sc_adam_step_all": (ST, [P, P, P, P, U64, C.POINTER(sc_adam_groups)]),
     "sc_apply_constraints": (ST, [P, P, F32, F32, F32]),

@@ -27,6 +27,8 @@
 // pair in 0.49 ms instead of 0.83 ms at 1M splats and 8 views.
 #include "sc_internal.cuh"
 
+#include <algorithm>
+
 namespace sck {
 
 // SH constants, project_gaussians.wgsl:47-61
@@ -51,10 +53,9 @@ struct Cam {
   float near_plane, focal, width, height;
 };
 
-__device__ __forceinline__ Cam load_cam(const sc_camera* c) {
+__device__ __forceinline__ Cam cam_of(const float4 a, const float4 b, const float4 cc, const float4 d, const float4 e,
+                                      const float4 f) {
   Cam k;
-  const float4* p = reinterpret_cast<const float4*>(c);
-  float4 a = __ldg(p + 0), b = __ldg(p + 1), cc = __ldg(p + 2), d = __ldg(p + 3), e = __ldg(p + 4), f = __ldg(p + 5);
   k.v[0] = a.x; k.v[1] = a.y; k.v[2] = a.z; k.v[3] = a.w;
   k.v[4] = b.x; k.v[5] = b.y; k.v[6] = b.z; k.v[7] = b.w;
   k.v[8] = cc.x; k.v[9] = cc.y; k.v[10] = cc.z; k.v[11] = cc.w;
@@ -63,6 +64,28 @@ __device__ __forceinline__ Cam load_cam(const sc_camera* c) {
   k.focal = f.x; k.width = f.y; k.height = f.z;
   return k;
 }
+__device__ __forceinline__ Cam load_cam(const sc_camera* c) {
+  const float4* p = reinterpret_cast<const float4*>(c);
+  return cam_of(__ldg(p + 0), __ldg(p + 1), __ldg(p + 2), __ldg(p + 3), __ldg(p + 4), __ldg(p + 5));
+}
+
+// Where a kernel's cameras come from: device memory (the trainer's step
+// parameters), or the launch's own parameters (the stage calls: staging them in
+// an allocation of the stream's pool cost a call up to 250 us of host time,
+// since the pool gives its memory back at every synchronize).
+struct CamPtr {
+  const sc_camera* p;
+  __device__ __forceinline__ Cam get(uint32_t v) const { return load_cam(p + v); }
+};
+template <uint32_t N>
+struct CamArgs {
+  sc_camera c[N];
+  __device__ __forceinline__ Cam get(uint32_t v) const {
+    const float4* p = reinterpret_cast<const float4*>(c + v);
+    return cam_of(p[0], p[1], p[2], p[3], p[4], p[5]);
+  }
+};
+static_assert(sizeof(sc_camera) == 96, "camera layout");
 
 __device__ __forceinline__ void sh_basis15(float x, float y, float z, float b[15]) {
   const float xx = x * x, yy = y * y, zz = z * z;
@@ -211,7 +234,8 @@ __device__ __forceinline__ void proj_cp_async16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(sa), "l"(gmem) : "memory");
 }
 
-__global__ void __launch_bounds__(PROJ_THREADS, 8) k_project(DSplats s_all, const sc_camera* __restrict__ cams, uint32_t n_views,
+template <typename CAMS>
+__global__ void __launch_bounds__(PROJ_THREADS, 8) k_project(DSplats s_all, const __grid_constant__ CAMS cams, uint32_t n_views,
                                                  uint32_t stride, float4* __restrict__ rec, TileArgs ta,
                                                  uint32_t* __restrict__ depth_keys, uint32_t* __restrict__ ids,
                                                  uint32_t* __restrict__ counts, int precise,
@@ -263,7 +287,7 @@ __global__ void __launch_bounds__(PROJ_THREADS, 8) k_project(DSplats s_all, cons
     // ties only with splats at or beyond depth_max, and emits nothing)
     uint32_t key = 0xFFFFFFFFu, cnt = 0;
     if (live) {
-      const Cam c = load_cam(cams + v);
+      const Cam c = cams.get(v);
       Geo g;
       if (geometry<false>(c, px, py, pz, qw, qx, qy, qz, l0, l1, l2, precise, g)) {
         const float f = c.focal;
@@ -355,7 +379,8 @@ __global__ void __launch_bounds__(PROJ_THREADS, 8) k_project(DSplats s_all, cons
   }
 }
 
-sc_status launch_project(sc_ctx* ctx, const DSplats& s, const sc_camera* d_cams, uint32_t n_views, uint32_t stride,
+template <typename CAMS>
+static sc_status project_cams(sc_ctx* ctx, const DSplats& s, const CAMS& cams, uint32_t n_views, uint32_t stride,
                          float4* rec, const sc_tiling* tl, uint32_t* depth_keys, uint32_t* ids, uint32_t* counts,
                          int precise, int cull, float4* zero_grad, float4* zero_comp, const SceneDev* scenes) {
   if (stride == 0 || n_views == 0) return SC_OK;
@@ -366,9 +391,27 @@ sc_status launch_project(sc_ctx* ctx, const DSplats& s, const sc_camera* d_cams,
   const uint32_t bs = PROJ_THREADS;  // grid: (splats / bs) x views CTAs, views innermost
   const uint64_t blocks = sc_div_up(stride, bs) * (uint64_t)n_views;
   if (blocks > 0x7FFFFFFFull) return sc_fail(ctx, SC_ERR_INVALID_ARG, "too many splat views for one launch");
-  k_project<<<(unsigned)blocks, bs, 0, ctx->stream>>>(s, d_cams, n_views, stride, rec, ta, depth_keys, ids, counts,
-                                                      precise, zero_grad, zero_comp, scenes);
+  k_project<CAMS><<<(unsigned)blocks, bs, 0, ctx->stream>>>(s, cams, n_views, stride, rec, ta, depth_keys, ids, counts,
+                                                            precise, zero_grad, zero_comp, scenes);
   return sc_check_launch(ctx, "k_project");
+}
+
+sc_status launch_project(sc_ctx* ctx, const DSplats& s, const sc_camera* d_cams, uint32_t n_views, uint32_t stride,
+                         float4* rec, const sc_tiling* tl, uint32_t* depth_keys, uint32_t* ids, uint32_t* counts,
+                         int precise, int cull, float4* zero_grad, float4* zero_comp, const SceneDev* scenes) {
+  return project_cams(ctx, s, CamPtr{d_cams}, n_views, stride, rec, tl, depth_keys, ids, counts, precise, cull,
+                      zero_grad, zero_comp, scenes);
+}
+
+sc_status launch_project_host_cams(sc_ctx* ctx, const DSplats& s, const sc_camera* cams, uint32_t n_views,
+                                   float4* rec, int precise) {
+  auto run = [&](auto args) {
+    std::copy(cams, cams + n_views, args.c);
+    return project_cams(ctx, s, args, n_views, s.cap, rec, nullptr, nullptr, nullptr, nullptr, precise, 0, nullptr,
+                        nullptr, nullptr);
+  };
+  if (n_views <= 4) return run(CamArgs<4>{});
+  return run(CamArgs<SC_MAX_VIEWS>{});
 }
 
 // ---------------------------------------------------------------- backward
@@ -460,11 +503,12 @@ __device__ __forceinline__ bool splat_backward_view(const Cam& c, float px, floa
 }
 
 __global__ void __launch_bounds__(128) k_project_backward(DSplats s, const float4* __restrict__ pg,
-                                                          const sc_camera* __restrict__ cam, float* __restrict__ out,
-                                                          uint32_t gcap, int accumulate, int precise) {
+                                                          const __grid_constant__ CamArgs<1> cam,
+                                                          float* __restrict__ out, uint32_t gcap, int accumulate,
+                                                          int precise) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= s.n) return;
-  const Cam c = load_cam(cam);
+  const Cam c = cam.get(0);
   float gpos[3] = {0, 0, 0}, grot[4] = {0, 0, 0, 0}, gsc[3] = {0, 0, 0}, gop = 0, basis[15];
   const float4 p0 = pg[3 * (size_t)i], p1 = pg[3 * (size_t)i + 1], p2 = pg[3 * (size_t)i + 2];
   const float op = 1.0f / (1.0f + expf(-sp_row(s, 10, i)));
@@ -493,10 +537,10 @@ __global__ void __launch_bounds__(128) k_project_backward(DSplats s, const float
   }
 }
 
-sc_status launch_project_backward(sc_ctx* ctx, const DSplats& s, const float4* pg, const sc_camera* d_cam,
+sc_status launch_project_backward(sc_ctx* ctx, const DSplats& s, const float4* pg, const sc_camera& cam,
                                   float* grads, uint32_t gcap, int accumulate, int precise_det) {
   if (s.n == 0) return SC_OK;
-  k_project_backward<<<(unsigned)sc_div_up(s.n, 128), 128, 0, ctx->stream>>>(s, pg, d_cam, grads, gcap, accumulate,
+  k_project_backward<<<(unsigned)sc_div_up(s.n, 128), 128, 0, ctx->stream>>>(s, pg, CamArgs<1>{{cam}}, grads, gcap, accumulate,
                                                                              precise_det);
   return sc_check_launch(ctx, "k_project_backward");
 }

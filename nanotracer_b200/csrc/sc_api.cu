@@ -476,18 +476,6 @@ void sc_camera_from_pose(const float eye[3], const float target[3], const float 
   out->n_splats = n_splats;
 }
 
-// cameras are staged through the scratch-independent error buffer page
-static sc_status stage_cams(sc_ctx* ctx, const sc_camera* cams, uint32_t n_views, sc_camera** d_cams) {
-  // cameras live in a small dedicated slice right after the error word page
-  static_assert(sizeof(sc_camera) == 96, "camera layout");
-  if (n_views > SC_MAX_VIEWS) return sc_fail(ctx, SC_ERR_INVALID_ARG, "too many views");
-  void* p;
-  SC_CUDA_TRY(ctx, cudaMallocAsync(&p, (size_t)n_views * sizeof(sc_camera), ctx->stream), "camera alloc");
-  SC_CUDA_TRY(ctx, cudaMemcpyAsync(p, cams, (size_t)n_views * sizeof(sc_camera), cudaMemcpyHostToDevice, ctx->stream), "camera upload");
-  *d_cams = reinterpret_cast<sc_camera*>(p);
-  return SC_OK;
-}
-
 static bool tiling_ok(const sc_tiling* t) {
   return t && t->width > 0 && t->height > 0 && t->tile_w > 0 && t->tile_h > 0;
 }
@@ -497,12 +485,9 @@ sc_status sc_project(sc_ctx* ctx, const sc_splats* s, const sc_camera* cams, uin
                      sc_projected_splat* projected) {
   if (!ctx || !s || !cams || (!projected && s->n)) return SC_ERR_INVALID_ARG;
   if (n_views == 0) return SC_OK;
-  sc_camera* d_cams;
-  SC_TRY(stage_cams(ctx, cams, n_views, &d_cams));
-  sc_status st = sck::launch_project(ctx, dview(s), d_cams, n_views, s->cap, reinterpret_cast<float4*>(projected),
-                                     nullptr, nullptr, nullptr, nullptr, ctx->fp64_det, 0);
-  cudaFreeAsync(d_cams, ctx->stream);
-  return st;
+  if (n_views > SC_MAX_VIEWS) return sc_fail(ctx, SC_ERR_INVALID_ARG, "too many views");
+  return sck::launch_project_host_cams(ctx, dview(s), cams, n_views, reinterpret_cast<float4*>(projected),
+                                       ctx->fp64_det);
 }
 
 }  // extern "C"
@@ -815,12 +800,8 @@ sc_status sc_project_backward(sc_ctx* ctx, const sc_splats* s, const sc_projecte
                               sc_grads* g, int accumulate) {
   if (!ctx || !s || !pg || !cam || !g) return SC_ERR_INVALID_ARG;
   if (g->cap < s->n) return sc_fail(ctx, SC_ERR_CAPACITY, "grads smaller than the splat count");
-  sc_camera* d_cam;
-  SC_TRY(stage_cams(ctx, cam, 1, &d_cam));
-  sc_status st = sck::launch_project_backward(ctx, dview(s), reinterpret_cast<const float4*>(pg), d_cam, g->slab,
-                                              g->cap, accumulate, ctx->fp64_det);
-  cudaFreeAsync(d_cam, ctx->stream);
-  return st;
+  return sck::launch_project_backward(ctx, dview(s), reinterpret_cast<const float4*>(pg), *cam, g->slab, g->cap,
+                                      accumulate, ctx->fp64_det);
 }
 
 sc_status sc_tonemap(sc_ctx* ctx, const float* image, uint32_t w, uint32_t h, uint8_t* rgba8) {

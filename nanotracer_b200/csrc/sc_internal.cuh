@@ -316,7 +316,12 @@ sc_status launch_project(sc_ctx* ctx, const DSplats& s, const sc_camera* d_cams,
                          float4* zero_grad = nullptr, float4* zero_comp = nullptr,
                          const SceneDev* scenes = nullptr);
 
-sc_status launch_project_backward(sc_ctx* ctx, const DSplats& s, const float4* proj_grad, const sc_camera* d_cam,
+// the records alone (no keys, no counts), one stride of s.cap per view, with
+// the cameras (host, at most SC_MAX_VIEWS) among the launch's parameters
+sc_status launch_project_host_cams(sc_ctx* ctx, const DSplats& s, const sc_camera* cams, uint32_t n_views,
+                                   float4* rec, int precise_det);
+
+sc_status launch_project_backward(sc_ctx* ctx, const DSplats& s, const float4* proj_grad, const sc_camera& cam,
                                   float* grads, uint32_t gcap, int accumulate, int precise_det);
 
 // Adam hyper-parameters, clamp limits and bias corrections of one step

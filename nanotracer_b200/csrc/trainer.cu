@@ -159,6 +159,8 @@ struct sc_trainer {
   SceneDev* d_scenes = nullptr;
   double* h_losses = nullptr;    // pinned: per-view squared-error sums of the last step
   uint32_t scene_max_cap = 0, scene_max_gstride = 0;
+  // a viewer's frame (sc_view): forward only, into the caller's records and image
+  bool forward_only = false;
   // graph
   cudaGraphExec_t exec = nullptr;
   const void* g_key[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
@@ -181,7 +183,8 @@ struct sc_trainer {
 };
 
 static void trainer_free_splat_arrays(sc_trainer* tr) {
-  cudaFree(tr->rec); cudaFree(tr->pgrad); cudaFree(tr->pcomp); cudaFree(tr->grads); cudaFree(tr->dkeys);
+  if (!tr->forward_only) cudaFree(tr->rec);
+  cudaFree(tr->pgrad); cudaFree(tr->pcomp); cudaFree(tr->grads); cudaFree(tr->dkeys);
   cudaFree(tr->dkeys_tmp);
   tr->pcomp = nullptr;
   cudaFree(tr->ids); cudaFree(tr->ids_tmp); cudaFree(tr->counts_by_id); cudaFree(tr->counts);
@@ -260,18 +263,20 @@ static sc_status ensure_splat_arrays(sc_trainer* tr, uint32_t cap) {
   SC_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "sync");
   trainer_free_splat_arrays(tr);
   const size_t nv = (size_t)tr->V * cap;
-  SC_CUDA_TRY(ctx, cudaMalloc(&tr->rec, nv * 48), "rec");
-  SC_CUDA_TRY(ctx, cudaMalloc(&tr->pgrad, nv * 48), "pgrad");
-  if (tr->cfg.compensated_sums) SC_CUDA_TRY(ctx, cudaMalloc(&tr->pcomp, nv * 48), "pcomp");
-  tr->grad_stride = (cap + 63u) & ~63u;
-  SC_CUDA_TRY(ctx, cudaMalloc(&tr->grads, (size_t)SC_NROWS * tr->grad_stride * 4), "grads");
+  if (!tr->forward_only) {
+    SC_CUDA_TRY(ctx, cudaMalloc(&tr->rec, nv * 48), "rec");
+    SC_CUDA_TRY(ctx, cudaMalloc(&tr->pgrad, nv * 48), "pgrad");
+    if (tr->cfg.compensated_sums) SC_CUDA_TRY(ctx, cudaMalloc(&tr->pcomp, nv * 48), "pcomp");
+    tr->grad_stride = (cap + 63u) & ~63u;
+    SC_CUDA_TRY(ctx, cudaMalloc(&tr->grads, (size_t)SC_NROWS * tr->grad_stride * 4), "grads");
+  }
   SC_CUDA_TRY(ctx, cudaMalloc(&tr->dkeys, nv * 4), "dkeys");
   SC_CUDA_TRY(ctx, cudaMalloc(&tr->dkeys_tmp, nv * 4), "dkeys");
   SC_CUDA_TRY(ctx, cudaMalloc(&tr->ids, nv * 4), "ids");
   SC_CUDA_TRY(ctx, cudaMalloc(&tr->ids_tmp, nv * 4), "ids");
   SC_CUDA_TRY(ctx, cudaMalloc(&tr->counts_by_id, nv * 4), "counts");
   SC_CUDA_TRY(ctx, cudaMalloc(&tr->counts, (nv + 1) * 4), "counts");
-  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->rec, 0, nv * 48, ctx->stream), "zero");
+  if (!tr->forward_only) SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->rec, 0, nv * 48, ctx->stream), "zero");
   tr->stride = cap;
   trainer_drop_graph(tr);
   const sc_status st = ensure_zero_block(tr);
@@ -328,7 +333,7 @@ static sc_status ensure_pairs(sc_trainer* tr, uint64_t K) {
 
 // taker chunks per pool
 static sc_status ensure_takers(sc_trainer* tr, uint64_t chunks) {
-  if (tr->cfg.bwd_mode != SC_BWD_EXACT || chunks <= tr->takers.pool_cap) return SC_OK;
+  if (tr->forward_only || tr->cfg.bwd_mode != SC_BWD_EXACT || chunks <= tr->takers.pool_cap) return SC_OK;
   sc_ctx* ctx = tr->ctx;
   const uint64_t cap = chunks + chunks / 4 + 64;
   if (cap * sck::TAKER_POOLS > 0xFFFFFFFFull) return sc_fail(ctx, SC_ERR_CAPACITY, "too many blended entries in one step");
@@ -460,7 +465,7 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
   // are needed only from the backward on (a host upload overlaps the forward)
   const bool mse_in_bwd = lam == 0.0f;
   const float* fwd_target = mse_in_bwd ? nullptr : tr->targets;
-  const sck::TakerChunks* takers = tr->cfg.bwd_mode == SC_BWD_EXACT ? &tr->takers : nullptr;
+  const sck::TakerChunks* takers = tr->cfg.bwd_mode == SC_BWD_EXACT && !tr->forward_only ? &tr->takers : nullptr;
   if (tr->h_targets && !mse_in_bwd)  // the copies run in order: the last view's event covers all
     SC_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->stream, tr->ev_view[V - 1], 0), "join");
   if (tr->two_level)
@@ -474,6 +479,7 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
     SC_TRY(sck::launch_ssim(ctx, tr->image, tr->targets, tr->cfg.tiling.width, tr->cfg.tiling.height, V,
                             weight * lam, tr->dl_dc, tr->d_ssim, tr->ssim_terms));
   }
+  if (tr->forward_only) return SC_OK;
   mark(tr, 7, capturing);
   const float* bwd_target = mse_in_bwd ? tr->targets : nullptr;
   // with host targets and the MSE formed here, one launch per view on its own
@@ -844,6 +850,103 @@ sc_status sc_trainer_blend_pairs(const sc_trainer* tr, uint64_t out[2]) {
   if (!tr || !out) return SC_ERR_INVALID_ARG;
   for (int i = 0; i < 2; ++i) out[i] = tr->prof_steps ? tr->work_acc[4 + i] / tr->prof_steps : 0;
   return SC_OK;
+}
+
+}  // extern "C"
+
+// ================================================================ viewer frame
+struct sc_view {
+  sc_trainer* tr = nullptr;
+};
+
+extern "C" {
+
+sc_status sc_view_create(sc_ctx* ctx, const sc_tiling* tl, sc_view** out) {
+  if (!ctx || !tl || !out || !tl->width || !tl->height || !tl->tile_w || !tl->tile_h) return SC_ERR_INVALID_ARG;
+  *out = nullptr;
+  sc_trainer* tr = new sc_trainer();
+  tr->ctx = ctx;
+  tr->forward_only = true;
+  tr->cfg.n_views = tr->V = 1;
+  tr->cfg.tiling = *tl;
+  tr->cfg.bwd_mode = SC_BWD_EXACT;
+  tr->cfg.tile_cull = 1;
+  tr->tiles_x = (tl->width + tl->tile_w - 1) / tl->tile_w;
+  tr->tiles_y = (tl->height + tl->tile_h - 1) / tl->tile_h;
+  tr->T = tr->tiles_x * tr->tiles_y;
+  tr->P = (uint64_t)tl->width * tl->height;
+  tr->ST = sck::super_tiles_per_view(tl);
+  tr->super_bits = bits_for(tr->ST);
+  tr->two_level = tr->super_bits <= 16;
+  cudaError_t e = (uint64_t)tr->tiles_x * tr->tiles_y > 65536 ? cudaErrorInvalidValue : cudaSuccess;
+  if (e != cudaSuccess) {
+    delete tr;
+    return sc_fail(ctx, SC_ERR_INVALID_ARG, "REF32 keys hold at most 65536 tiles (tile_emit.wgsl key layout)");
+  }
+  e = cudaMallocHost(&tr->h_params, sizeof(StepParams));
+  if (e == cudaSuccess) e = cudaMallocHost(&tr->h_out, sizeof(StepOut));
+  if (e == cudaSuccess) e = cudaMalloc(&tr->d_params, sizeof(StepParams));
+  if (e != cudaSuccess) {
+    sc_trainer_free(ctx, tr);
+    return sc_cuda_fail(ctx, e, "view alloc");
+  }
+  std::memset(tr->h_params, 0, sizeof(StepParams));
+  sc_view* v = new sc_view();
+  v->tr = tr;
+  *out = v;
+  return SC_OK;
+}
+
+void sc_view_free(sc_ctx* ctx, sc_view* v) {
+  if (!v) return;
+  sc_trainer_free(ctx, v->tr);
+  delete v;
+}
+
+uint32_t sc_view_records(const sc_splats* s) {
+  return s ? (uint32_t)sc_div_up(s->cap, sck::RADIX_SEG_TILE) * sck::RADIX_SEG_TILE : 0;
+}
+
+sc_status sc_view_frame(sc_view* v, const sc_splats* s, const sc_camera* cam, float depth_max,
+                        sc_projected_splat* projected, float* image, uint8_t* rgba8, uint8_t* rgba8_host) {
+  if (!v || !s || !cam || !projected || !image || (rgba8_host && !rgba8)) return SC_ERR_INVALID_ARG;
+  sc_trainer* tr = v->tr;
+  sc_ctx* ctx = tr->ctx;
+  tr->cfg.tiling.depth_max = depth_max;
+  tr->cfg.fp64_det = (uint32_t)ctx->fp64_det;
+  SC_TRY(ensure_splat_arrays(tr, s->cap));
+  tr->rec = reinterpret_cast<float4*>(projected);
+  tr->image = reinterpret_cast<float4*>(image);
+  sc_status st = SC_OK;
+  for (int attempt = 0; attempt < 4; ++attempt) {
+    const bool sizing = tr->two_level ? tr->icap == 0 : tr->kcap == 0;
+    tr->h_params->cams[0] = *cam;
+    st = enqueue_step(tr, const_cast<sc_splats*>(s), nullptr, nullptr, false, sizing);
+    if (st == SC_OK && rgba8)
+      st = sck::launch_tonemap(ctx, tr->image, tr->cfg.tiling.width, tr->cfg.tiling.height, rgba8);
+    if (st == SC_OK) {
+      k_finalize<<<1, 32, 0, ctx->stream>>>(tr->d_loss, nullptr, 0.0f, 1, 0.0, 0.0, tr->d_total, ctx->d_error,
+                                            tr->takers.drawn, tr->h_out, nullptr);
+      st = sc_check_launch(ctx, "k_finalize");
+    }
+    cudaError_t e = cudaSuccess;
+    if (st == SC_OK && rgba8_host)
+      e = cudaMemcpyAsync(rgba8_host, rgba8, 4 * (size_t)tr->P, cudaMemcpyDeviceToHost, ctx->stream);
+    const cudaError_t es = cudaStreamSynchronize(ctx->stream);  // also before a failure: h_params is read until then
+    if (st == SC_OK && (e != cudaSuccess || es != cudaSuccess)) st = sc_cuda_fail(ctx, e != cudaSuccess ? e : es, "frame");
+    if (st != SC_OK) break;
+    const StepOut o = *tr->h_out;
+    if (!(o.err & (SC_DEVERR_TIMEOUT | SC_DEVERR_SKIP))) break;
+    if (cudaMemsetAsync(ctx->d_error, 0, 4, ctx->stream) != cudaSuccess) st = sc_fail(ctx, SC_ERR_CUDA, "clear error");
+    else if (o.err & SC_DEVERR_TIMEOUT) st = sc_fail(ctx, SC_ERR_TIMEOUT, "a bounded device wait gave up during the frame");
+    if (st == SC_OK) st = ensure_items(tr, o.items);
+    if (st == SC_OK) st = ensure_pairs(tr, o.pairs);
+    if (st != SC_OK) break;
+    if (attempt == 3) st = sc_fail(ctx, SC_ERR_CAPACITY, "item capacity kept overflowing");
+  }
+  tr->rec = nullptr;  // the caller's
+  tr->image = nullptr;
+  return st;
 }
 
 }  // extern "C"

@@ -5,12 +5,13 @@ composite, tonemap — into an RGBA8 device buffer instead of a swapchain
 texture.  There is no window here; frame() returns the pixels."""
 from __future__ import annotations
 
+import ctypes as C
 import math
 from dataclasses import dataclass, field
 
 import numpy as np
 
-from ._lib import SC_KEYS_REF32
+from ._lib import check, lib, ptr
 from .gpu import CudaCtx
 from .raster import CameraUniform, Rasterizer
 from .splat_gpu import GpuSplatBuffer
@@ -49,9 +50,10 @@ class HeadlessView:
         self.width, self.height = int(width), int(height)
         self.rasterizer = Rasterizer(ctx)
         self.binner = TileBinner(ctx)
-        self.projected = self.rasterizer.alloc_projected(self.splats, 1)
+        self.projected = ctx.storage_buffer_zeroed("projected", 48 * lib().sc_view_records(self.splats.handle))
         self.image = self.rasterizer.alloc_image(self.width, self.height, 1)
         self.rgba8 = ctx.storage_buffer_zeroed("rgba8", 4 * self.width * self.height)
+        self._view = None  # the library's frame state, made by the first frame
 
     def tiling(self, orbit: OrbitCamera) -> TilingParams:
         return TilingParams(self.width, self.height, self.TILE, max(orbit.distance * 4.0, 50.0))
@@ -61,14 +63,24 @@ class HeadlessView:
         n = self.splats.n
         cam = CameraUniform.from_pose(orbit.position(), np.asarray(orbit.target, np.float32), (0.0, 1.0, 0.0),
                                       orbit.fov_y, self.width, self.height, n)
-        self.rasterizer.project(self.splats, [cam], self.projected)
         params = self.tiling(orbit)
-        bins = self.binner.bin(self.projected, n, params, stride=self.splats.capacity, n_views=1,
-                               key_mode=SC_KEYS_REF32)
-        self.rasterizer.composite(self.projected, bins, self.image, params, self.splats.capacity, 1)
-        self.rasterizer.tonemap(self.image, self.width, self.height, self.rgba8)
-        return self.rgba8.readback(np.uint8).reshape(self.height, self.width, 4)
+        if self._view is None:
+            t, h = params.struct(), C.c_void_p()
+            check(lib().sc_view_create(self.ctx.handle, C.byref(t), C.byref(h)), self.ctx.handle)
+            self._view = h
+        out = np.empty((self.height, self.width, 4), np.uint8)
+        check(lib().sc_view_frame(self._view, self.splats.handle, C.byref(cam.c), float(params.depth_max),
+                                  self.projected.cptr, self.image.cptr, self.rgba8.cptr, ptr(out)), self.ctx.handle)
+        return out
 
     def hdr(self) -> np.ndarray:
         """The last frame before tonemapping: (height, width, 4) float32 (rgb, 1 - T)."""
         return self.image.readback(np.float32).reshape(self.height, self.width, 4)
+
+    def __del__(self):
+        try:
+            if self._view and self.ctx.handle:
+                lib().sc_view_free(self.ctx.handle, self._view)
+                self._view = None
+        except Exception:
+            pass

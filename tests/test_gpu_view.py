@@ -43,3 +43,35 @@ def test_frame_matches_oracle_forward(ctx, oracle, azimuth, elevation):
     want, _, _ = oracle.composite(rec, pay, ranges, tl)
     assert np.mean(np.abs(hdr - want) <= 1e-4) > 0.999
     assert (hdr[..., 3] > 0).mean() > 0.05  # something was drawn
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n,size,distance", [(1, (16, 16), 4.0), (300, (33, 17), 1.5), (20000, (333, 211), 2.2),
+                                             (20000, (64, 800), 30.0)])
+def test_frame_equals_the_stage_calls_bit_for_bit(ctx, n, size, distance):
+    """The one-call frame blends the splats of sc_bin's REF32 lists in their
+    order: the image before and after tonemapping, and the records, are those of
+    project -> bin -> composite -> tonemap, from one frame to the next (the
+    item buffers grow on the way) and with the store's FP64 determinant option."""
+    from nanotracer_b200 import CameraUniform, TilingParams
+    from tests.util import GpuPipe
+    W, H = size
+    scene = random_scene(n, n + 3)
+    view = HeadlessView(ctx, scene, W, H)
+    try:
+        for k, (az, el) in enumerate([(0.3, 0.2), (2.5, -0.5), (4.0, 0.9)]):
+            ctx.set_fp64_det(k == 2)
+            orbit = OrbitCamera(distance=distance, azimuth=az, elevation=el)
+            px = view.frame(orbit)
+            cam = CameraUniform.from_pose(orbit.position(), orbit.target, (0.0, 1.0, 0.0), orbit.fov_y, W, H, n)
+            pipe = GpuPipe(ctx, scene, cam, TilingParams(W, H, 16, max(4.0 * distance, 50.0)))
+            rec = pipe.project()[0]
+            pipe.bin()
+            img, _ = pipe.composite()
+            assert np.array_equal(view.hdr(), img[0])
+            assert np.array_equal(view.projected.readback(np.float32).reshape(-1, 12)[:n], rec)
+            out = ctx.storage_buffer_zeroed("rgba8", 4 * W * H)
+            pipe.r.tonemap(pipe.img, W, H, out)
+            assert np.array_equal(px, out.readback(np.uint8).reshape(H, W, 4))
+    finally:
+        ctx.set_fp64_det(False)
