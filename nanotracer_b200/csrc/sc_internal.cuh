@@ -306,14 +306,12 @@ namespace sck {
 // writes per (view, splat) a depth sort key (float bits, 0xFFFFFFFF when the
 // splat emits no pairs; one segment of stride keys per view) and a count for
 // the native pipeline: (tile, splat) pairs, or with bit 1 of `cull` two-level
-// binning items.  Bit 0 of `cull`: exact tile culling.  zero_grad (nullable):
-// per-(view, splat) gradient records of the same layout set to zero.
+// binning items.  Bit 0 of `cull`: exact tile culling.
 // scenes (nullable, n_views entries): view v projects scene v's own store
 // (its first scene.s.n splats; the rest of the view's stride is culled).
 sc_status launch_project(sc_ctx* ctx, const DSplats& s, const sc_camera* d_cams, uint32_t n_views,
                          uint32_t stride, float4* rec, const sc_tiling* tiling, uint32_t* depth_keys,
                          uint32_t* splat_ids, uint32_t* counts, int precise_det, int cull,
-                         float4* zero_grad = nullptr, float4* zero_comp = nullptr,
                          const SceneDev* scenes = nullptr);
 
 // the records alone (no keys, no counts), one stride of s.cap per view, with
@@ -420,9 +418,9 @@ __device__ __forceinline__ void constrain_geometry(float np[14], const AdamParam
 // ---- many scenes in one step (one view per scene), each with its own store
 // gradient rows of every scene from its view's records (grid.y = scene)
 sc_status launch_project_backward_scenes(sc_ctx* ctx, const SceneDev* d_scenes, uint32_t n_scenes,
-                                         uint32_t max_gstride, const float4* proj_grad, uint32_t stride,
+                                         uint32_t max_gstride, float4* proj_grad, uint32_t stride,
                                          const sc_camera* d_cams, const uint32_t* d_skip, int precise_det,
-                                         const float4* proj_comp);
+                                         float4* proj_comp);
 // Adam + constraints + densify statistic of every scene's splats (grid.z = scene;
 // gstride and the stores' capacities multiples of 8)
 sc_status launch_adam_rows_scenes(sc_ctx* ctx, const SceneDev* d_scenes, uint32_t n_scenes, uint32_t max_count,
@@ -432,11 +430,12 @@ sc_status launch_adam_rows_scenes(sc_ctx* ctx, const SceneDev* d_scenes, uint32_
 // Shard-major gradient layout: element (row r, splat i) of a buffer cut into
 // chunks of `shard` splats sits at ((i / shard) * SC_NROWS + r) * shard + i % shard.
 // Per-splat gradient summed over this rank's views, written shard-major; rows
-// of splats in [n, n_shards*shard) are zero.
-sc_status launch_project_backward_shards(sc_ctx* ctx, const DSplats& s, const float4* proj_grad, uint32_t stride,
+// of splats in [n, n_shards*shard) are zero.  The projected gradients (and
+// compensation records) come back zeroed.
+sc_status launch_project_backward_shards(sc_ctx* ctx, const DSplats& s, float4* proj_grad, uint32_t stride,
                                          const sc_camera* d_cams, uint32_t n_views, float* grads, uint32_t n_shards,
                                          uint32_t shard, const uint32_t* d_skip_flag, int precise_det,
-                                         const float4* proj_comp = nullptr);
+                                         float4* proj_comp = nullptr);
 // Adam + constraints + densify statistic for splats [lo, lo+count) from one
 // reduce-scattered chunk g[r * shard + j]
 // Adam + constraints + densify statistic over splats [lo, lo+count) from

@@ -254,6 +254,17 @@ static sc_status ensure_zero_block(sc_trainer* tr) {
   return SC_OK;
 }
 
+// The blend backward adds to the gradient records and the projection backward
+// clears what it read, so they are zero between steps; a step that breaks off
+// between the two calls this.
+static sc_status zero_gradient_records(sc_trainer* tr) {
+  sc_ctx* ctx = tr->ctx;
+  const size_t bytes = (size_t)tr->V * tr->stride * 48;
+  if (tr->pgrad) SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->pgrad, 0, bytes, ctx->stream), "zero");
+  if (tr->pcomp) SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->pcomp, 0, bytes, ctx->stream), "zero");
+  return SC_OK;
+}
+
 // Per-view arrays hold stride = cap rounded up to whole sort tiles, so each
 // view's depth keys are one segment of the segmented depth sort.
 static sc_status ensure_splat_arrays(sc_trainer* tr, uint32_t cap) {
@@ -278,6 +289,7 @@ static sc_status ensure_splat_arrays(sc_trainer* tr, uint32_t cap) {
   SC_CUDA_TRY(ctx, cudaMalloc(&tr->counts, (nv + 1) * 4), "counts");
   if (!tr->forward_only) SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->rec, 0, nv * 48, ctx->stream), "zero");
   tr->stride = cap;
+  SC_TRY(zero_gradient_records(tr));
   trainer_drop_graph(tr);
   const sc_status st = ensure_zero_block(tr);
   if (st != SC_OK) {
@@ -393,7 +405,7 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
   mark(tr, 0, capturing);
   SC_TRY(sck::launch_project(ctx, ds, d_cams, V, tr->stride, tr->rec, &tr->cfg.tiling, tr->dkeys, tr->ids,
                              tr->counts_by_id, tr->cfg.fp64_det ? 1 : 0,
-                             (tr->cfg.tile_cull ? 1 : 0) | (tr->two_level ? 2 : 0), tr->pgrad, tr->pcomp,
+                             (tr->cfg.tile_cull ? 1 : 0) | (tr->two_level ? 2 : 0),
                              tr->scenes_mode ? tr->d_scenes : nullptr));
   mark(tr, 1, capturing);
   bool in_tmp = false;
@@ -743,7 +755,11 @@ static sc_status run_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, float* a
       SC_CUDA_TRY(ctx, cudaGraphLaunch(tr->exec, ctx->stream), "graph launch");
       ctx->launches += tr->kernels_per_step;
     } else {
-      SC_TRY(enqueue_step(tr, s, mo, acc, false, sizing));
+      const sc_status st = enqueue_step(tr, s, mo, acc, false, sizing);
+      if (st != SC_OK) {
+        zero_gradient_records(tr);
+        return st;
+      }
     }
     SC_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "step sync");
     const StepOut o = *tr->h_out;
@@ -751,6 +767,7 @@ static sc_status run_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, float* a
     tr->last_items = o.items;
     if (o.err & SC_DEVERR_TIMEOUT) {
       cudaMemsetAsync(ctx->d_error, 0, 4, ctx->stream);
+      zero_gradient_records(tr);
       return sc_fail(ctx, SC_ERR_TIMEOUT, "a bounded device wait gave up during the step");
     }
     if (o.err & SC_DEVERR_SKIP) {
