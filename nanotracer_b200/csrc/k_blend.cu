@@ -761,6 +761,29 @@ sc_status launch_composite_items(sc_ctx* ctx, const float4* rec, uint32_t stride
 // warps per (view, tile) of a blend launch: one takers' head each
 uint32_t blend_warps_per_tile(const sc_tiling* tl) { return tl->tile_w * tl->tile_h / pick_ppt(tl) / 32; }
 
+// Classes from 1024, 512 and 192 takers up, 256 tiles each: four classes of 128
+// from 2048, 1024, 512 and 256 left the 3M-splat step at 1.67 ms, a last class from
+// 256 the 200k-splat one at 134 us.
+__global__ void __launch_bounds__(256) k_heavy_tiles(TakerChunks t, uint32_t tiles, uint32_t warps,
+                                                     const uint32_t* __restrict__ skip) {
+  const uint32_t vt = blockIdx.x * 256 + threadIdx.x;
+  if (vt >= tiles || (skip && (*skip & SC_DEVERR_SKIP))) return;
+  uint32_t most = 0;
+  for (uint32_t w = 0; w < warps; ++w) most = max(most, t.head[(size_t)vt * warps + w].y);
+  const uint32_t c = most >= 1024 ? 0 : most >= 512 ? 1 : 2;
+  uint32_t at = HEAVY_CAP;
+  if (most >= 192) at = atomicAdd(t.n_heavy + c, 1u);
+  if (at < HEAVY_CAP) t.heavy[c * HEAVY_CAP + at] = vt;
+  t.is_heavy[vt] = at < HEAVY_CAP;
+}
+
+sc_status launch_heavy_tiles(sc_ctx* ctx, const TakerChunks& takers, uint32_t tiles, uint32_t warps_per_tile,
+                             const uint32_t* d_skip) {
+  if (tiles == 0) return SC_OK;
+  k_heavy_tiles<<<(tiles + 255) / 256, 256, 0, ctx->stream>>>(takers, tiles, warps_per_tile, d_skip);
+  return sc_check_launch(ctx, "k_heavy_tiles");
+}
+
 // ---------------------------------------------------------------- MSE (standalone)
 __global__ void k_mse_views(const float4* __restrict__ pred, const float* __restrict__ target, uint64_t P,
                             float gscale, float4* __restrict__ dl_dc, double* __restrict__ loss) {
@@ -916,6 +939,11 @@ __device__ __forceinline__ void twosum_atomic_add4(float4* s, float4* c, float4 
 // LIST_TAKERS: exact mode over the entries that the forward wrote down per warp.
 // A warp sends its sums of an entry to global memory itself, one float4 atomic
 // per part of the entry's record.
+// The tiles with the longest walks (at silhouettes, where pixels never saturate:
+// thousands of takers against some 60 on average) start first: in tile order the
+// last of them began half-way, and a one-view step waited for it alone (1M
+// splats, one 1080p view: 272 -> 208 us; 200k splats at 1024x1024: 142 -> 127 us;
+// 3M splats, 4 views: 1.62 -> 1.50 ms; 8 views of 1M 1.372 -> 1.369 ms).
 template <int PPT, int MODE, int LIST, bool COMP, bool COUNT, bool OCT>
 __global__ void __launch_bounds__(256) k_composite_backward(const float4* __restrict__ rec, ListArgs l, BlendArgs a,
                                                             const float4* __restrict__ fwd,
@@ -936,7 +964,17 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
   if (skip && (*skip & SC_DEVERR_SKIP)) return;
   const uint32_t warp = threadIdx.x >> 5;
   BwdSmem<FEED, OCT>& sm = reinterpret_cast<BwdSmem<FEED, OCT>*>(sbuf)[warp];
-  const uint32_t vt = blockIdx.x;
+  uint32_t vt = blockIdx.x;
+  if (LIST == LIST_TAKERS && takers.heavy) {  // the heavy tiles' blocks come first
+    constexpr uint32_t H = HEAVY_CLASSES * HEAVY_CAP;
+    if (vt < H) {
+      if (vt % HEAVY_CAP >= takers.n_heavy[vt / HEAVY_CAP]) return;
+      vt = takers.heavy[vt];
+    } else {
+      vt -= H;
+      if (takers.is_heavy[vt]) return;
+    }
+  }
   const uint32_t v = vt / a.num_tiles, tile = vt - v * a.num_tiles;
   const uint32_t ty = tile / a.tiles_x, tx = tile - ty * a.tiles_x;
   uint32_t px, py0;
@@ -1234,6 +1272,7 @@ static sc_status backward_ppt(sc_ctx* ctx, const BlendArgs& a, uint32_t grid, ui
   const size_t smem = threads / 32 * sizeof(BwdSmem<FEED, OCT>);
   if (smem > 48 * 1024)
     SC_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
+  if (LIST == LIST_TAKERS && takers.heavy) grid += HEAVY_CLASSES * HEAVY_CAP;
   kern<<<grid, threads, smem, ctx->stream>>>(rec, l, a, fwd, dl_dc, target, gscale, loss, aux, proj_grad, d_skip,
                                              reinterpret_cast<unsigned long long*>(work), proj_comp, takers);
   return sc_check_launch(ctx, "k_composite_backward");

@@ -513,14 +513,24 @@ uint32_t super_tiles_per_view(const sc_tiling* tl);
 // holding chunks [p pool_cap, (p + 1) pool_cap); a pool that runs out raises
 // SC_DEVERR_TAKERS and goes on counting.
 constexpr uint32_t TAKER_POOLS = 64;  // a power of two
+constexpr uint32_t HEAVY_CLASSES = 3, HEAVY_CAP = 256;
 struct TakerChunks {
   uint32_t* ids;    // TAKER_POOLS x pool_cap x 32
   uint32_t* prev;   // TAKER_POOLS x pool_cap
   uint2* head;
   uint32_t* drawn;  // TAKER_POOLS
+  // the (view, tile)s that the backward starts first (null: tile order), in
+  // HEAVY_CLASSES lists of HEAVY_CAP by their longest warp's takers, how many
+  // there are (zeroed by the caller), and for every (view, tile) whether it is in one
+  uint32_t* heavy;
+  uint32_t* n_heavy;
+  uint8_t* is_heavy;
   uint32_t pool_cap;
 };
 uint32_t blend_warps_per_tile(const sc_tiling* tl);
+// fills the heavy lists of `tiles` (view, tile)s from their heads
+sc_status launch_heavy_tiles(sc_ctx* ctx, const TakerChunks& takers, uint32_t tiles, uint32_t warps_per_tile,
+                             const uint32_t* d_skip);
 sc_status launch_composite(sc_ctx* ctx, const float4* rec, uint32_t stride, uint32_t n_views,
                            const uint32_t* payloads, const uint32_t* ranges, const sc_tiling* tl, float4* image,
                            uint2* aux, const float* target, float mse_scale, float4* dl_dc, double* loss,

@@ -233,7 +233,7 @@ static sc_status ensure_zero_block(sc_trainer* tr) {
   size_t off = 0;
   auto take = [&](size_t b) { const size_t o = off; off += (b + 255) & ~(size_t)255; return o; };
   const size_t o_loss = take(8 * (size_t)tr->V), o_ssim = take(8 * (size_t)tr->V), o_total = take(16),
-               o_drawn = take(sck::TAKER_POOLS * 4),
+               o_drawn = take((sck::TAKER_POOLS + sck::HEAVY_CLASSES) * 4),
                o_ranges = take((size_t)tr->V * (tr->two_level ? tr->ST : tr->T) * 8),
                o_scan = take(sck::scan_scratch_bytes(nsp + 1)),
                o_seg = take(sck::radix_seg_scratch_bytes(tr->stride, tr->V, 16));
@@ -246,6 +246,7 @@ static sc_status ensure_zero_block(sc_trainer* tr) {
   tr->d_ssim = reinterpret_cast<double*>(z + o_ssim);
   tr->d_total = reinterpret_cast<uint64_t*>(z + o_total);
   tr->takers.drawn = reinterpret_cast<uint32_t*>(z + o_drawn);
+  tr->takers.n_heavy = tr->takers.drawn + sck::TAKER_POOLS;
   (tr->two_level ? tr->iranges : tr->ranges) = reinterpret_cast<uint32_t*>(z + o_ranges);
   tr->scan_scratch = z + o_scan;
   tr->scan_bytes = o_seg - o_scan;
@@ -500,6 +501,12 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
   // (tiles with long lists) overlap each other
   const bool per_view = tr->h_targets && mse_in_bwd;
   if (per_view) SC_CUDA_TRY(ctx, cudaEventRecord(tr->ev_fwd, ctx->stream), "forward done");
+  // the longest walks first, unless all tiles start at once anyway (6 CTAs per
+  // SM) or the views go one by one
+  const bool heavy_first = takers && !per_view && (uint64_t)V * tr->T > 6 * (uint64_t)ctx->sm_count;
+  if (heavy_first)
+    SC_TRY(sck::launch_heavy_tiles(ctx, tr->takers, V * tr->T, sck::blend_warps_per_tile(&tr->cfg.tiling),
+                                   ctx->d_error));
   for (uint32_t v0 = 0; v0 < V; v0 += per_view ? 1 : V) {
     const uint32_t nv = per_view ? 1 : V;
     cudaStream_t main_stream = ctx->stream;
@@ -512,6 +519,7 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
     const float* tg = bwd_target ? bwd_target + 3 * po : nullptr;
     sck::TakerChunks vt = tr->takers;  // the views' heads
     if (takers) vt.head += (size_t)v0 * tr->T * sck::blend_warps_per_tile(&tr->cfg.tiling);
+    if (!heavy_first) vt.heavy = nullptr;
     sc_status st;
     if (tr->two_level)
       st = (sck::launch_composite_backward_items(ctx, tr->rec + so, tr->stride, nv, item_keys, item_ids,
@@ -617,6 +625,9 @@ sc_status sc_trainer_create(sc_ctx* ctx, const sc_train_config* cfg, sc_trainer*
   if (e == cudaSuccess) e = cudaMalloc(&tr->dl_dc, pix * 16);
   const size_t heads = (size_t)tr->V * tr->T * sck::blend_warps_per_tile(&t);
   if (e == cudaSuccess && cfg->bwd_mode == SC_BWD_EXACT) e = cudaMalloc(&tr->takers.head, heads * sizeof(uint2));
+  if (e == cudaSuccess && cfg->bwd_mode == SC_BWD_EXACT)
+    e = cudaMalloc(&tr->takers.heavy, sck::HEAVY_CLASSES * sck::HEAVY_CAP * 4);
+  if (e == cudaSuccess && cfg->bwd_mode == SC_BWD_EXACT) e = cudaMalloc(&tr->takers.is_heavy, (size_t)tr->V * tr->T);
   if (e == cudaSuccess) e = cudaMalloc(&tr->d_work, 6 * sck::BLEND_WORK_SLOTS * 8);
   if (e == cudaSuccess && cfg->ssim_lambda > 0.0f) e = cudaMalloc(&tr->ssim_terms, sck::ssim_terms_bytes(tr->P, tr->V));
   for (int i = 0; i <= kStages && e == cudaSuccess; ++i) e = cudaEventCreate(&tr->ev[i]);
@@ -644,6 +655,7 @@ void sc_trainer_free(sc_ctx* ctx, sc_trainer* tr) {
   trainer_free_pairs(tr);
   trainer_free_items(tr);
   cudaFree(tr->takers.ids); cudaFree(tr->takers.prev); cudaFree(tr->takers.head);
+  cudaFree(tr->takers.heavy); cudaFree(tr->takers.is_heavy);
   cudaFree(tr->zero); cudaFree(tr->image); cudaFree(tr->aux); cudaFree(tr->dl_dc);
   cudaFree(tr->d_work); cudaFree(tr->d_params);
   cudaFree(tr->ssim_terms);

@@ -109,3 +109,24 @@ def test_list_backward_against_the_oracle_for_every_warp_layout(ctx, oracle, til
                                             dl.reshape(-1, 4), mode, np.ascontiguousarray(aux[0, ..., 1]).reshape(-1),
                                             tfin.reshape(-1), want_abs=True)
     check_pg_explained(pg, want, absum, flags, label=f"tile {tile} mode {mode}")
+
+
+@pytest.mark.parametrize("n,size", [(1200, (480, 320)), (2500, (640, 480))])
+def test_trainer_backward_starts_heavy_tiles_first(ctx, n, size):
+    """Images of more tiles than start at once, whose silhouette tiles take a
+    few hundred faint splats and fall into the lists that the backward starts with:
+    every tile is still walked exactly once."""
+    W, H = size
+    scene = _scene(n)
+    scene.scales[:] = np.log(0.25)
+    scene.opacities[:] = -3.0
+    cam = CameraUniform.from_pose(*orbit_pose(20.0), FOV_Y, W, H, n)
+    tl = TilingParams(W, H, 8, 8.0)
+    tgt = _targets(W, H)
+    want, img = _stage_grads(ctx, scene, cam, tl, tgt, W, H)
+    cfg = TrainConfig(n_views=1, width=W, height=H, tile_w=8, tile_h=8, depth_max=8.0, tile_cull=False)
+    got, timg = _trainer_grads(ctx, scene, cam, cfg, tgt)
+    assert np.array_equal(img, timg)
+    for lo, hi in [(0, 3), (3, 7), (7, 10), (10, 11), (11, 14), (14, 59)]:
+        d = np.linalg.norm((got[lo:hi] - want[lo:hi]).astype(np.float64))
+        assert d <= 1e-5 * np.linalg.norm(want[lo:hi].astype(np.float64)), (lo, d)
