@@ -309,6 +309,7 @@ __global__ void __launch_bounds__(256, GEOM ? 3 : 4) k_adam_rows(DSplats s, DMom
                                                    const float* __restrict__ g, uint32_t lo, uint32_t count,
                                                    uint32_t gstride, AdamParams ap, const float* __restrict__ d_bc,
                                                    const uint32_t* __restrict__ skip) {
+  sc_after_previous();
   adam_rows<GEOM>(s, mo, acc, g, lo, count, gstride, ap, d_bc, skip);
 }
 
@@ -318,6 +319,7 @@ template <bool GEOM>
 __global__ void __launch_bounds__(256, GEOM ? 3 : 4) k_adam_rows_scenes(const SceneDev* __restrict__ scenes,
                                                           AdamParams ap, const float* __restrict__ d_bc,
                                                           const uint32_t* __restrict__ skip) {
+  sc_after_previous();
   const SceneDev sd = scenes[blockIdx.z];
   adam_rows<GEOM>(sd.s, sd.mo, sd.acc, sd.grads, 0, sd.s.n, sd.gstride, ap, d_bc, skip);
 }
@@ -326,9 +328,9 @@ sc_status launch_adam_rows_scenes(sc_ctx* ctx, const SceneDev* d_scenes, uint32_
                                   const AdamParams& ap, const float* d_bc, const uint32_t* d_skip) {
   if (n_scenes == 0 || max_count == 0) return SC_OK;
   const unsigned gx = (unsigned)sc_div_up(sc_div_up(max_count, ADAM_SPT), 256);
-  k_adam_rows_scenes<true><<<dim3(gx, 9, n_scenes), 256, 0, ctx->stream>>>(d_scenes, ap, d_bc, d_skip);
+  sc_launch(ctx, k_adam_rows_scenes<true>, dim3(gx, 9, n_scenes), 256, 0, d_scenes, ap, d_bc, d_skip);
   SC_TRY(sc_check_launch(ctx, "k_adam_rows_scenes"));
-  k_adam_rows_scenes<false><<<dim3(gx, ADAM_GROUPS - 9, n_scenes), 256, 0, ctx->stream>>>(d_scenes, ap, d_bc, d_skip);
+  sc_launch(ctx, k_adam_rows_scenes<false>, dim3(gx, ADAM_GROUPS - 9, n_scenes), 256, 0, d_scenes, ap, d_bc, d_skip);
   return sc_check_launch(ctx, "k_adam_rows_scenes");
 }
 
@@ -339,10 +341,10 @@ sc_status launch_adam_rows(sc_ctx* ctx, const DSplats& s, const DMoments& mo, fl
   if (lo % ADAM_SPT || gstride % ADAM_SPT || s.cap % ADAM_SPT || mo.cap % ADAM_SPT)
     return sc_fail(ctx, SC_ERR_INVALID_ARG, "Adam rows: offsets and strides must be multiples of 8");
   const unsigned gx = (unsigned)sc_div_up(sc_div_up(count, ADAM_SPT), 256);
-  k_adam_rows<true><<<dim3(gx, 9), 256, 0, ctx->stream>>>(s, mo, acc, g, lo, count, gstride, ap, d_bc, d_skip);
+  sc_launch(ctx, k_adam_rows<true>, dim3(gx, 9), 256, 0, s, mo, acc, g, lo, count, gstride, ap, d_bc, d_skip);
   SC_TRY(sc_check_launch(ctx, "k_adam_rows"));
-  k_adam_rows<false><<<dim3(gx, ADAM_GROUPS - 9), 256, 0, ctx->stream>>>(s, mo, acc, g, lo, count, gstride, ap, d_bc,
-                                                                          d_skip);
+  sc_launch(ctx, k_adam_rows<false>, dim3(gx, ADAM_GROUPS - 9), 256, 0, s, mo, acc, g, lo, count, gstride, ap, d_bc,
+            d_skip);
   return sc_check_launch(ctx, "k_adam_rows");
 }
 

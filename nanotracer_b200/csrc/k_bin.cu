@@ -187,6 +187,7 @@ __global__ void __launch_bounds__(256) k_tile_ranges_u32x4(const uint32_t* __res
                                                            uint32_t tile_bits, uint32_t key_mask,
                                                            uint32_t* __restrict__ ranges,
                                                            unsigned long long* __restrict__ high_popc) {
+  sc_after_previous();
   const uint64_t K = min(*d_total, cap);
   const uint64_t nq = (K + 3) >> 2;
   const uint32_t lane = threadIdx.x & 31;
@@ -257,11 +258,10 @@ sc_status launch_tile_ranges(sc_ctx* ctx, const void* keys, int key_mode, const 
                                                  key_bits >= 32 ? ~0u : (1u << key_bits) - 1u, ranges,
                                                  reinterpret_cast<unsigned long long*>(high_popc));
   else
-    k_tile_ranges_u32x4<<<(unsigned)std::min<uint64_t>(sc_div_up(sc_div_up(cap, 4), 256), (uint64_t)ctx->sm_count * 8),
-                          256, 0, ctx->stream>>>(static_cast<const uint32_t*>(keys), d_total, cap, num_tiles,
-                                                 tiles_per_view, tile_bits,
-                                                 key_bits >= 32 ? ~0u : (1u << key_bits) - 1u, ranges,
-                                                 reinterpret_cast<unsigned long long*>(high_popc));
+    sc_launch(ctx, k_tile_ranges_u32x4, (unsigned)std::min<uint64_t>(sc_div_up(sc_div_up(cap, 4), 256),
+              (uint64_t)ctx->sm_count * 8), 256, 0, static_cast<const uint32_t*>(keys), d_total, cap, num_tiles,
+              tiles_per_view, tile_bits, key_bits >= 32 ? ~0u : (1u << key_bits) - 1u, ranges,
+              reinterpret_cast<unsigned long long*>(high_popc));
   return sc_check_launch(ctx, "k_tile_ranges");
 }
 
@@ -423,6 +423,7 @@ __global__ void __launch_bounds__(SE_THREADS) k_super_emit(
     const uint32_t* __restrict__ offsets, const uint32_t* __restrict__ counts_by_id, BinArgs a, uint32_t super_x,
     uint32_t super_bits, uint32_t* __restrict__ keys, uint32_t* __restrict__ payloads, uint64_t cap,
     uint32_t* __restrict__ err, int cull) {
+  sc_after_previous();
   __shared__ uint32_t sk[SE_CHUNK], sp[SE_CHUNK];
   __shared__ uint32_t s_class[SE_CLASSES];
   __shared__ uint16_t s_perm[SE_THREADS];
@@ -521,8 +522,8 @@ sc_status launch_super_emit(sc_ctx* ctx, const float4* rec, uint32_t stride, uin
   const BinArgs a = bin_args(tl);
   const uint32_t sx = (a.tiles_x + SC_SUPER - 1) / SC_SUPER;
   const uint32_t bits = super_bits_for(super_tiles_per_view(tl));
-  k_super_emit<<<(unsigned)sc_div_up(total, SE_THREADS), SE_THREADS, 0, ctx->stream>>>(
-      rec, stride, n_views, sorted_ids, offsets, counts_by_id, a, sx, bits, keys, payloads, cap, d_error, cull);
+  sc_launch(ctx, k_super_emit, (unsigned)sc_div_up(total, SE_THREADS), SE_THREADS, 0, rec, stride, n_views,
+            sorted_ids, offsets, counts_by_id, a, sx, bits, keys, payloads, cap, d_error, cull);
   return sc_check_launch(ctx, "k_super_emit");
 }
 

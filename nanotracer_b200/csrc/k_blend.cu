@@ -539,6 +539,7 @@ __global__ void __launch_bounds__(256) k_composite(const float4* __restrict__ re
                                                    float4* __restrict__ dl_dc, double* __restrict__ loss,
                                                    uint32_t* __restrict__ skip, unsigned long long* __restrict__ work,
                                                    TakerChunks takers) {
+  sc_after_previous();
   extern __shared__ float4 sbuf[];  // one ListSmem per warp, then one TakerRing per warp
   __shared__ double sred[8];
   __shared__ uint32_t s_work[2];
@@ -699,8 +700,8 @@ static sc_status composite_ppt(sc_ctx* ctx, const BlendArgs& a, uint32_t grid, u
   const size_t smem = threads / 32 * (sizeof(ListSmem) + (takers.head ? sizeof(TakerRing) : 0));
   if (smem > 48 * 1024)
     SC_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
-  kern<<<grid, threads, smem, ctx->stream>>>(rec, l, a, image, aux, target, gscale, dl_dc, loss, d_skip,
-                                             reinterpret_cast<unsigned long long*>(work), takers);
+  sc_launch(ctx, kern, grid, threads, smem, rec, l, a, image, aux, target, gscale, dl_dc, loss, d_skip,
+            reinterpret_cast<unsigned long long*>(work), takers);
   return sc_check_launch(ctx, "k_composite");
 }
 
@@ -766,6 +767,7 @@ uint32_t blend_warps_per_tile(const sc_tiling* tl) { return tl->tile_w * tl->til
 // 256 the 200k-splat one at 134 us.
 __global__ void __launch_bounds__(256) k_heavy_tiles(TakerChunks t, uint32_t tiles, uint32_t warps,
                                                      const uint32_t* __restrict__ skip) {
+  sc_after_previous();
   const uint32_t vt = blockIdx.x * 256 + threadIdx.x;
   if (vt >= tiles || (skip && (*skip & SC_DEVERR_SKIP))) return;
   uint32_t most = 0;
@@ -780,7 +782,7 @@ __global__ void __launch_bounds__(256) k_heavy_tiles(TakerChunks t, uint32_t til
 sc_status launch_heavy_tiles(sc_ctx* ctx, const TakerChunks& takers, uint32_t tiles, uint32_t warps_per_tile,
                              const uint32_t* d_skip) {
   if (tiles == 0) return SC_OK;
-  k_heavy_tiles<<<(tiles + 255) / 256, 256, 0, ctx->stream>>>(takers, tiles, warps_per_tile, d_skip);
+  sc_launch(ctx, k_heavy_tiles, (tiles + 255) / 256, 256, 0, takers, tiles, warps_per_tile, d_skip);
   return sc_check_launch(ctx, "k_heavy_tiles");
 }
 
@@ -955,6 +957,7 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
                                                             const uint32_t* __restrict__ skip,
                                                             unsigned long long* __restrict__ work,
                                                             float4* __restrict__ proj_comp, TakerChunks takers) {
+  sc_after_previous();
   static_assert(!OCT || PPT == 2, "the octet reduction takes two pixels per thread");
   static_assert(LIST != LIST_TAKERS || MODE == SC_BWD_EXACT, "the takers are the exact mode's entries");
   using FEED = typename std::conditional<LIST == LIST_TAKERS, TakerFeed, ListFeed<LIST, true>>::type;
@@ -1273,8 +1276,8 @@ static sc_status backward_ppt(sc_ctx* ctx, const BlendArgs& a, uint32_t grid, ui
   if (smem > 48 * 1024)
     SC_CUDA_TRY(ctx, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "smem attr");
   if (LIST == LIST_TAKERS && takers.heavy) grid += HEAVY_CLASSES * HEAVY_CAP;
-  kern<<<grid, threads, smem, ctx->stream>>>(rec, l, a, fwd, dl_dc, target, gscale, loss, aux, proj_grad, d_skip,
-                                             reinterpret_cast<unsigned long long*>(work), proj_comp, takers);
+  sc_launch(ctx, kern, grid, threads, smem, rec, l, a, fwd, dl_dc, target, gscale, loss, aux, proj_grad, d_skip,
+            reinterpret_cast<unsigned long long*>(work), proj_comp, takers);
   return sc_check_launch(ctx, "k_composite_backward");
 }
 

@@ -73,6 +73,7 @@ struct TermsSmem {
 __global__ void __launch_bounds__(256, 3) k_ssim_terms(const float4* __restrict__ pred,
                                                        const float* __restrict__ target, SsimArgs a,
                                                        float* __restrict__ terms, double* __restrict__ ssim_sum) {
+  sc_after_previous();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   TermsSmem& sm = *reinterpret_cast<TermsSmem*>(smem_raw);
   __shared__ double red[8];
@@ -223,6 +224,7 @@ __device__ __forceinline__ float reflected_taps(const float* src, int i, int n, 
 __global__ void __launch_bounds__(256, 4) k_ssim_grad(const float4* __restrict__ pred,
                                                       const float* __restrict__ target, SsimArgs a,
                                                       const float* __restrict__ terms, float4* __restrict__ dl_dc) {
+  sc_after_previous();
   extern __shared__ __align__(16) unsigned char smem_raw[];
   GradSmem& sm = *reinterpret_cast<GradSmem*>(smem_raw);
   const uint32_t v = blockIdx.z;
@@ -377,9 +379,9 @@ sc_status launch_ssim(sc_ctx* ctx, const float4* pred, const float* target, uint
     attr_set[dev] = true;
   }
   const dim3 grid((w + SS_T - 1) / SS_T, (h + SS_T - 1) / SS_T, n_views);
-  k_ssim_terms<<<grid, 256, sizeof(TermsSmem), ctx->stream>>>(pred, target, a, terms, ssim_sum);
+  sc_launch(ctx, k_ssim_terms, grid, 256, sizeof(TermsSmem), pred, target, a, terms, ssim_sum);
   SC_TRY(sc_check_launch(ctx, "k_ssim_terms"));
-  k_ssim_grad<<<grid, 256, sizeof(GradSmem), ctx->stream>>>(pred, target, a, terms, dl_dc);
+  sc_launch(ctx, k_ssim_grad, grid, 256, sizeof(GradSmem), pred, target, a, terms, dl_dc);
   return sc_check_launch(ctx, "k_ssim_grad");
 }
 

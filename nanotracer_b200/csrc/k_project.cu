@@ -240,6 +240,7 @@ __global__ void __launch_bounds__(PROJ_THREADS, 8) k_project(DSplats s_all, cons
                                                  uint32_t* __restrict__ depth_keys, uint32_t* __restrict__ ids,
                                                  uint32_t* __restrict__ counts, int precise,
                                                  const SceneDev* __restrict__ scenes) {
+  sc_after_previous();
   // the chunk's 14 geometric / opacity / DC rows (and, in the BF16 form, its 45
   // SH-rest rows) are staged in shared memory by 16-byte cp.async copies issued
   // together at the start, so their latency is paid once, not once per
@@ -382,8 +383,8 @@ static sc_status project_cams(sc_ctx* ctx, const DSplats& s, const CAMS& cams, u
   const uint32_t bs = PROJ_THREADS;  // grid: (splats / bs) x views CTAs, views innermost
   const uint64_t blocks = sc_div_up(stride, bs) * (uint64_t)n_views;
   if (blocks > 0x7FFFFFFFull) return sc_fail(ctx, SC_ERR_INVALID_ARG, "too many splat views for one launch");
-  k_project<CAMS><<<(unsigned)blocks, bs, 0, ctx->stream>>>(s, cams, n_views, stride, rec, ta, depth_keys, ids, counts,
-                                                            precise, scenes);
+  sc_launch(ctx, k_project<CAMS>, (unsigned)blocks, bs, 0, s, cams, n_views, stride, rec, ta, depth_keys, ids, counts,
+            precise, scenes);
   return sc_check_launch(ctx, "k_project");
 }
 
@@ -647,6 +648,7 @@ __global__ void __launch_bounds__(PB_THREADS, 5) k_project_backward_shards(DSpla
                                                                      uint32_t n_shards, uint32_t shard,
                                                                      const uint32_t* __restrict__ skip, int precise,
                                                                      float4* __restrict__ pc) {
+  sc_after_previous();
   project_backward_rows(s, pg, stride, cams, n_views, out, n_shards, shard, skip, precise, pc);
 }
 
@@ -657,6 +659,7 @@ __global__ void __launch_bounds__(PB_THREADS, 5) k_project_backward_scenes(const
                                                                      const sc_camera* __restrict__ cams,
                                                                      const uint32_t* __restrict__ skip, int precise,
                                                                      float4* __restrict__ pc) {
+  sc_after_previous();
   const uint32_t v = blockIdx.y;
   const SceneDev sd = scenes[v];
   const size_t off = (size_t)3 * v * stride;
@@ -670,8 +673,8 @@ sc_status launch_project_backward_scenes(sc_ctx* ctx, const SceneDev* d_scenes, 
                                          float4* pc) {
   if (n_scenes == 0 || max_gstride == 0) return SC_OK;
   const dim3 grid((unsigned)sc_div_up(max_gstride, PB_THREADS), n_scenes);
-  k_project_backward_scenes<<<grid, PB_THREADS, 0, ctx->stream>>>(d_scenes, pg, stride, d_cams, d_skip, precise_det,
-                                                                  pc);
+  sc_launch(ctx, k_project_backward_scenes, grid, PB_THREADS, 0, d_scenes, pg, stride, d_cams, d_skip, precise_det,
+            pc);
   return sc_check_launch(ctx, "k_project_backward_scenes");
 }
 
@@ -681,8 +684,8 @@ sc_status launch_project_backward_shards(sc_ctx* ctx, const DSplats& s, float4* 
                                          float4* pc) {
   const uint64_t total = (uint64_t)n_shards * shard;
   if (total == 0) return SC_OK;
-  k_project_backward_shards<<<(unsigned)sc_div_up(total, PB_THREADS), PB_THREADS, 0, ctx->stream>>>(
-      s, pg, stride, d_cams, n_views, grads, n_shards, shard, d_skip, precise_det, pc);
+  sc_launch(ctx, k_project_backward_shards, (unsigned)sc_div_up(total, PB_THREADS), PB_THREADS, 0, s, pg, stride,
+            d_cams, n_views, grads, n_shards, shard, d_skip, precise_det, pc);
   return sc_check_launch(ctx, "k_project_backward_shards");
 }
 

@@ -87,6 +87,7 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan(uint32_t* __restrict__ da
                                                        unsigned long long* __restrict__ status,
                                                        unsigned* __restrict__ ticket, uint64_t* __restrict__ total,
                                                        uint32_t* __restrict__ err, ScanGather gather) {
+  sc_after_previous();
   __shared__ unsigned s_tile;
   __shared__ unsigned long long s_warp[SCAN_THREADS / 32];
   __shared__ unsigned long long s_excl;
@@ -204,7 +205,7 @@ static sc_status scan_u32_impl(sc_ctx* ctx, uint32_t* data, uint64_t n, uint64_t
   unsigned long long* status = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(scratch) + 256);
   if (!clean)
     SC_CUDA_TRY(ctx, cudaMemsetAsync(scratch, 0, scan_scratch_bytes(n), ctx->stream), "memset scan status");
-  k_scan<<<(unsigned)tiles, SCAN_THREADS, 0, ctx->stream>>>(data, n, status, ticket, d_total, ctx->d_error, gather);
+  sc_launch(ctx, k_scan, (unsigned)tiles, SCAN_THREADS, 0, data, n, status, ticket, d_total, ctx->d_error, gather);
   return sc_check_launch(ctx, "k_scan");
 }
 
@@ -273,8 +274,8 @@ extern "C" sc_status sc_exclusive_scan_u32_noalloc(sc_ctx* ctx, uint32_t* data, 
   SC_CUDA_TRY(ctx, cudaMemsetAsync(scratch, 0, 256 + tiles * 8, ctx->stream), "clear scan scratch");
   unsigned* ticket = reinterpret_cast<unsigned*>(scratch);
   unsigned long long* status = reinterpret_cast<unsigned long long*>(reinterpret_cast<char*>(scratch) + 256);
-  sck::k_scan<<<(unsigned)tiles, SCAN_THREADS, 0, ctx->stream>>>(data, n, status, ticket, total, ctx->d_error,
-                                                                 sck::ScanGather{nullptr, nullptr, 1, 0});
+  sc_launch(ctx, sck::k_scan, (unsigned)tiles, SCAN_THREADS, 0, data, n, status, ticket, total, ctx->d_error,
+            sck::ScanGather{nullptr, nullptr, 1, 0});
   return sc_check_launch(ctx, "k_scan");
 }
 
@@ -349,6 +350,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_hist(const K* __restrict__ ke
                                                         const uint64_t* __restrict__ d_n, int passes,
                                                         uint32_t key_bits, uint32_t* __restrict__ hist /* passes x RADIX */,
                                                         unsigned* __restrict__ done) {
+  sc_after_previous();
   constexpr int RADIX = Rdx<RB>::RADIX;
   __shared__ uint32_t sh[RS_MAX_PASSES * RADIX];
   for (int t = threadIdx.x; t < passes * RADIX; t += RS_THREADS) sh[t] = 0;
@@ -612,6 +614,7 @@ __global__ void __launch_bounds__(RS_THREADS, RB == 8 ? 4 : 3) k_rs_pass(const K
                                                         const uint32_t* __restrict__ digit_base,
                                                         unsigned* __restrict__ lookback, unsigned* __restrict__ ticket,
                                                         uint32_t* __restrict__ err, int dbits) {
+  sc_after_previous();
   constexpr int IPT = RsCfg<K>::IPT;
   constexpr int TILE = RS_THREADS * IPT;
   constexpr int RADIX = Rdx<RB>::RADIX;
@@ -656,8 +659,8 @@ static sc_status radix_passes(sc_ctx* ctx, K* keys, uint32_t* vals, K* keys_tmp,
   SC_CUDA_TRY(ctx, cudaMemsetAsync(scratch, 0, need, ctx->stream), "memset radix scratch");
   const unsigned hist_blocks = (unsigned)std::min<uint64_t>(sc_div_up(n_cap, RS_THREADS),
                                                             (uint64_t)ctx->sm_count * RS_HIST_BLOCKS_PER_SM);
-  k_rs_hist<K, RB><<<hist_blocks, RS_THREADS, 0, ctx->stream>>>(keys, n_cap, d_n, passes, key_bits, hist,
-                                                                tickets + RS_DONE);
+  sc_launch(ctx, k_rs_hist<K, RB>, hist_blocks, RS_THREADS, 0, keys, n_cap, d_n, passes, key_bits, hist, tickets +
+            RS_DONE);
   SC_TRY(sc_check_launch(ctx, "k_rs_hist"));
   const size_t smem = sizeof(RsSmem<K, RB>);
   static bool attr_set = false;
@@ -672,13 +675,11 @@ static sc_status radix_passes(sc_ctx* ctx, K* keys, uint32_t* vals, K* keys_tmp,
   for (int p = 0; p < passes; ++p) {
     const int dbits = std::min(RB, (int)key_bits - RB * p);
     if (dbits == RB)
-      k_rs_pass<K, false, RB><<<(unsigned)tiles, RS_THREADS, smem, ctx->stream>>>(
-          kin, vin, kout, vout, n_cap, d_n, RB * p, hist + p * RADIX, lookback + (size_t)p * tiles * RADIX,
-          tickets + p, ctx->d_error, RB);
+      sc_launch(ctx, k_rs_pass<K, false, RB>, (unsigned)tiles, RS_THREADS, smem, kin, vin, kout, vout, n_cap, d_n, RB
+                * p, hist + p * RADIX, lookback + (size_t)p * tiles * RADIX, tickets + p, ctx->d_error, RB);
     else
-      k_rs_pass<K, true, RB><<<(unsigned)tiles, RS_THREADS, smem, ctx->stream>>>(
-          kin, vin, kout, vout, n_cap, d_n, RB * p, hist + p * RADIX, lookback + (size_t)p * tiles * RADIX,
-          tickets + p, ctx->d_error, dbits);
+      sc_launch(ctx, k_rs_pass<K, true, RB>, (unsigned)tiles, RS_THREADS, smem, kin, vin, kout, vout, n_cap, d_n, RB *
+                p, hist + p * RADIX, lookback + (size_t)p * tiles * RADIX, tickets + p, ctx->d_error, dbits);
     SC_TRY(sc_check_launch(ctx, "k_rs_pass"));
     std::swap(kin, kout);
     std::swap(vin, vout);
@@ -727,6 +728,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_rs_hist_seg(const uint32_t* __re
                                                             uint32_t n_segs, int passes, uint32_t key_bits,
                                                             uint32_t* __restrict__ hist /* [passes][n_segs][RADIX] */,
                                                             unsigned* __restrict__ done) {
+  sc_after_previous();
   constexpr int RADIX = Rdx<RB>::RADIX;
   __shared__ uint32_t sh[4 * RADIX];
   for (int t = threadIdx.x; t < passes * RADIX; t += RS_THREADS) sh[t] = 0;
@@ -765,6 +767,7 @@ __global__ void __launch_bounds__(RS_THREADS, 4) k_rs_pass_seg(const uint32_t* _
                                                             unsigned* __restrict__ lookback,
                                                             unsigned* __restrict__ ticket, uint32_t* __restrict__ err,
                                                             int dbits) {
+  sc_after_previous();
   constexpr int RADIX = Rdx<8>::RADIX;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   RsSmem<uint32_t, 8>& sm = *reinterpret_cast<RsSmem<uint32_t, 8>*>(smem_raw);
@@ -808,8 +811,8 @@ sc_status radix_sort_segments(sc_ctx* ctx, uint32_t* keys, uint32_t* vals, uint3
   if (!clean) SC_CUDA_TRY(ctx, cudaMemsetAsync(scratch, 0, need, ctx->stream), "memset radix scratch");
   const unsigned bx = (unsigned)std::max<uint64_t>(
       1, std::min<uint64_t>(sc_div_up(seg_len, RS_THREADS), (uint64_t)ctx->sm_count * RS_HIST_BLOCKS_PER_SM / n_segs));
-  k_rs_hist_seg<RB><<<dim3(bx, n_segs), RS_THREADS, 0, ctx->stream>>>(keys, seg_len, n_segs, passes, key_bits, hist,
-                                                                      tickets + RS_DONE);
+  sc_launch(ctx, k_rs_hist_seg<RB>, dim3(bx, n_segs), RS_THREADS, 0, keys, seg_len, n_segs, passes, key_bits, hist,
+            tickets + RS_DONE);
   SC_TRY(sc_check_launch(ctx, "k_rs_hist_seg"));
   const size_t smem = sizeof(RsSmem<uint32_t, RB>);
   static bool attr_set = false;
@@ -826,11 +829,11 @@ sc_status radix_sort_segments(sc_ctx* ctx, uint32_t* keys, uint32_t* vals, uint3
     const uint32_t* db = hist + (size_t)p * n_segs * RADIX;
     unsigned* lb = lookback + (size_t)p * tiles * RADIX;
     if (dbits == RB)
-      k_rs_pass_seg<false><<<(unsigned)tiles, RS_THREADS, smem, ctx->stream>>>(kin, vin, kout, vout, n, tps, RB * p,
-                                                                             db, lb, tickets + p, ctx->d_error, RB);
+      sc_launch(ctx, k_rs_pass_seg<false>, (unsigned)tiles, RS_THREADS, smem, kin, vin, kout, vout, n, tps, RB * p,
+                db, lb, tickets + p, ctx->d_error, RB);
     else
-      k_rs_pass_seg<true><<<(unsigned)tiles, RS_THREADS, smem, ctx->stream>>>(kin, vin, kout, vout, n, tps, RB * p,
-                                                                            db, lb, tickets + p, ctx->d_error, dbits);
+      sc_launch(ctx, k_rs_pass_seg<true>, (unsigned)tiles, RS_THREADS, smem, kin, vin, kout, vout, n, tps, RB * p, db,
+                lb, tickets + p, ctx->d_error, dbits);
     SC_TRY(sc_check_launch(ctx, "k_rs_pass_seg"));
     std::swap(kin, kout);
     std::swap(vin, vout);
@@ -868,8 +871,8 @@ sc_status selftest_lookback_timeout(sc_ctx* ctx) {
   const size_t smem = sizeof(RsSmem<K, 8>);
   SC_CUDA_TRY(ctx, cudaFuncSetAttribute(k_rs_pass<K, false, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                         (int)smem), "smem attr");
-  k_rs_pass<K, false, 8><<<2, RS_THREADS, smem, ctx->stream>>>(keys, vals, kout, vout, n, nullptr, 0, hist, lookback,
-                                                               ticket, ctx->d_error, 8);
+  sc_launch(ctx, k_rs_pass<K, false, 8>, 2, RS_THREADS, smem, keys, vals, kout, vout, n, nullptr, 0, hist, lookback,
+            ticket, ctx->d_error, 8);
   SC_TRY(sc_check_launch(ctx, "k_rs_pass (timeout self-test)"));
   return sc_check_device_error(ctx);
 }

@@ -15,6 +15,7 @@
 #include <stdint.h>
 
 #include <string>
+#include <utility>
 
 #include "../../include/splat_cuda.h"
 
@@ -51,6 +52,9 @@ struct sc_ctx {
   // sc_ctx_set_fp64_det: near-degenerate splats get an FP64 determinant and
   // inverse in sc_project and sc_project_backward
   int fp64_det = 0;
+  // the trainer's chains of kernels launch with programmatic stream
+  // serialization (sc_launch)
+  bool overlap_launches = false;
   // grow-only scratch arena for temporaries of the reference-shaped calls
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
@@ -295,6 +299,31 @@ sc_status sc_check_device_error(sc_ctx* ctx);
     cudaError_t _e = (expr);                              \
     if (_e != cudaSuccess) return sc_cuda_fail(ctx, _e, what); \
   } while (0)
+
+// Launch of a kernel that begins with sc_after_previous().  With
+// ctx->overlap_launches its launch overlaps the end of the kernel before it on
+// the stream: its blocks become resident as that one's last blocks leave, and
+// wait in sc_after_previous() until it has completed and its writes are
+// visible, so nothing else changes.  A step of 5k splats falls from 0.198 to
+// 0.175 ms, of 200k from 0.479 to 0.449, of 1M from 1.154 to 1.115, 8 views of 1M from 4.22 to 4.18
+// ms.  Letting the next kernel's blocks in from the start (launch_dependents
+// first of all) costs what they hold while they wait: 0.193, 0.496, 1.302, 4.28 ms.
+template <typename... P, typename... A>
+static inline void sc_launch(sc_ctx* ctx, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, A&&... args) {
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = dim3(threads);
+  c.dynamicSmemBytes = smem;
+  c.stream = ctx->stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  c.attrs = &at;
+  c.numAttrs = ctx->overlap_launches ? 1 : 0;
+  cudaLaunchKernelEx(&c, kernel, std::forward<A>(args)...);  // sc_check_launch reads the error
+}
+// First statement of such a kernel: waits for the kernel before.
+__device__ __forceinline__ void sc_after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 static inline uint64_t sc_div_up(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 

@@ -54,6 +54,7 @@ __global__ void k_finalize(const double* __restrict__ loss_sums, const double* _
                            uint32_t n_views, double inv_count, double weight, const uint64_t* __restrict__ d_total,
                            const uint32_t* __restrict__ err, const uint32_t* __restrict__ drawn,
                            StepOut* __restrict__ out, double* __restrict__ losses) {
+  sc_after_previous();
   uint32_t most = 0;
   for (uint32_t p = threadIdx.x; p < sck::TAKER_POOLS; p += 32) most = max(most, drawn[p]);
   most = __reduce_max_sync(0xffffffffu, most);
@@ -374,6 +375,12 @@ static void mark(sc_trainer* tr, int i, bool capturing) {
 // (re)size the pair buffers before emitting (eager runs only).
 static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, float* acc, bool capturing, bool sizing) {
   sc_ctx* ctx = tr->ctx;
+  // host targets fork the step over several streams, which keeps plain launches
+  struct Overlap {
+    sc_ctx* ctx;
+    ~Overlap() { ctx->overlap_launches = false; }
+  } overlap{ctx};
+  ctx->overlap_launches = !tr->h_targets;
   const sc_camera* d_cams = reinterpret_cast<const sc_camera*>(tr->d_params);  // cams is the first member
   const float* d_bc = reinterpret_cast<const float*>(reinterpret_cast<const char*>(tr->d_params) +
                                                      offsetof(StepParams, bc));
@@ -564,10 +571,9 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
     SC_TRY(sck::launch_adam_rows(ctx, ds, dm, acc, tr->grads, 0, ds.n, tr->grad_stride, ap, d_bc, ctx->d_error));
   }
   mark(tr, 9, capturing);
-  k_finalize<<<1, 32, 0, ctx->stream>>>(tr->d_loss, lam > 0.0f ? tr->d_ssim : nullptr, lam, V,
-                                        1.0 / (3.0 * (double)tr->P), tr->grads_mode ? (double)tr->loss_weight : 0.0,
-                                        tr->d_total, ctx->d_error, tr->takers.drawn, tr->h_out,
-                                        tr->scenes_mode ? tr->h_losses : nullptr);
+  sc_launch(ctx, k_finalize, 1, 32, 0, tr->d_loss, lam > 0.0f ? tr->d_ssim : nullptr, lam, V, 1.0 / (3.0 *
+            (double)tr->P), tr->grads_mode ? (double)tr->loss_weight : 0.0, tr->d_total, ctx->d_error,
+            tr->takers.drawn, tr->h_out, tr->scenes_mode ? tr->h_losses : nullptr);
   SC_TRY(sc_check_launch(ctx, "k_finalize"));
   tr->kernels_per_step = (uint32_t)(ctx->launches - launches0);
   return SC_OK;
@@ -954,8 +960,8 @@ sc_status sc_view_frame(sc_view* v, const sc_splats* s, const sc_camera* cam, fl
     if (st == SC_OK && rgba8)
       st = sck::launch_tonemap(ctx, tr->image, tr->cfg.tiling.width, tr->cfg.tiling.height, rgba8);
     if (st == SC_OK) {
-      k_finalize<<<1, 32, 0, ctx->stream>>>(tr->d_loss, nullptr, 0.0f, 1, 0.0, 0.0, tr->d_total, ctx->d_error,
-                                            tr->takers.drawn, tr->h_out, nullptr);
+      sc_launch(ctx, k_finalize, 1, 32, 0, tr->d_loss, nullptr, 0.0f, 1, 0.0, 0.0, tr->d_total, ctx->d_error,
+                tr->takers.drawn, tr->h_out, nullptr);
       st = sc_check_launch(ctx, "k_finalize");
     }
     cudaError_t e = cudaSuccess;
