@@ -26,7 +26,10 @@
 // (2.25 with 8 rows), a thread slides over 12 or 14 staged values for 2 or 4
 // outputs (8 or 4 in the adjoint) instead of 11 loads each, and the moments of
 // x and y go as packed pairs.  2 views of 1237x822: terms 158 -> 79 us, gradient 422 ->
-// 113 us.
+// 113 us.  The gradient's planes come by cp.async, the next channel's during the
+// horizontal pass of this one, the prediction and target ahead of both passes, and the
+// reflected taps are at most five, unrolled: 113 -> 98 us (103 without the last;
+// two buffers of planes, with 3 CTAs per SM instead of 4, 111 us).
 // Reflect-101 with a 5-pixel radius folds at most once for images of 6 or more
 // pixels per side, which the host requires.
 #include "sc_internal.cuh"
@@ -207,18 +210,42 @@ template <int STRIDE>
 __device__ __forceinline__ float reflected_taps(const float* src, int i, int n, int base, const float* g) {
   float acc = 0.f;
   if (i <= SS_R && i >= 1) {
-    for (int k = 0; k < SS_W; ++k) {
-      const int j = -i - k + SS_R;
-      if (j >= 0) acc += g[k] * src[(j - base) * STRIDE];
-    }
+#pragma unroll
+    for (int k = 0; k < SS_R; ++k)
+      if (k <= SS_R - i) acc += g[k] * src[(SS_R - i - k - base) * STRIDE];
   }
   if (i >= n - 1 - SS_R && i <= n - 2) {
-    for (int k = 0; k < SS_W; ++k) {
+#pragma unroll
+    for (int k = SS_R + 1; k < SS_W; ++k) {
       const int j = 2 * (n - 1) - i - k + SS_R;
       if (j <= n - 1) acc += g[k] * src[(j - base) * STRIDE];
     }
   }
   return acc;
+}
+
+// Copies one channel's planes to shared memory (cp.async, zeros outside the image): a
+// warp takes whole rows, 32 columns and then 10.
+__device__ __forceinline__ void stage_planes(float (*f)[SS_H][SS_S], const float* __restrict__ tc, uint64_t P, int x0,
+                                             int y0, int W, int H) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int rx = (threadIdx.x & 31) + 32 * h, gx = x0 - SS_R + rx;
+    if (rx >= SS_H) break;
+    const bool in_x = gx >= 0 && gx < W;
+#pragma unroll 3
+    for (int ry = threadIdx.x >> 5; ry < SS_H; ry += 8) {
+      const int gy = y0 - SS_R + ry;
+      const bool in = in_x && gy >= 0 && gy < H;
+      const float* t = in ? tc + ((int64_t)gy * W + gx) : tc;  // nothing is read with a size of 0
+#pragma unroll
+      for (int pl = 0; pl < 3; ++pl)
+        asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(
+                         (uint32_t)__cvta_generic_to_shared(&f[pl][ry][rx])),
+                     "l"(t + pl * P), "r"(in ? 4 : 0)
+                     : "memory");
+    }
+  }
 }
 
 __global__ void __launch_bounds__(256, 4) k_ssim_grad(const float4* __restrict__ pred,
@@ -234,26 +261,20 @@ __global__ void __launch_bounds__(256, 4) k_ssim_grad(const float4* __restrict__
   const bool y_edge = y0 == 0 || y0 + SS_T + SS_R >= H, x_edge = x0 == 0 || x0 + SS_T + SS_R >= W;
   const int ty = threadIdx.x >> 3, tx = 4 * (threadIdx.x & 7);  // horizontal pass: row, 4 columns
   const int y = y0 + ty;
+  stage_planes(sm.f, tv, a.P, x0, y0, W, H);
   float gout[3][4];
 #pragma unroll
   for (int c = 0; c < 3; ++c) {
-    // a warp stages whole rows, 32 columns and then 10
-    const float* tc = tv + (uint64_t)(3 * c) * a.P;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int rx = (threadIdx.x & 31) + 32 * h, gx = x0 - SS_R + rx;
-      if (rx >= SS_H) break;
-      const bool in_x = gx >= 0 && gx < W;
-#pragma unroll 3
-      for (int ry = threadIdx.x >> 5; ry < SS_H; ry += 8) {
-        const int gy = y0 - SS_R + ry;
-        const bool in = in_x && gy >= 0 && gy < H;
-        const float* t = tc + ((int64_t)gy * W + gx);
-#pragma unroll
-        for (int pl = 0; pl < 3; ++pl) sm.f[pl][ry][rx] = in ? t[pl * a.P] : 0.f;
-      }
-    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
+    float xs[4], tg[4];  // this channel's prediction and target, on their way during both passes
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const bool in = x0 + tx + q < W && y < H;
+      const uint64_t p = (uint64_t)v * a.P + (uint64_t)y * W + x0 + tx + q;
+      xs[q] = in ? reinterpret_cast<const float*>(pred + p)[c] : 0.f;
+      tg[q] = in ? target[3 * p + c] : 0.f;
+    }
     // vertical adjoint: 8 rows of a staged column per task (sources outside the image are staged as zeros)
     for (int t = threadIdx.x; t < (SS_T / 8) * 3 * SS_H; t += 256) {
       const int strip = t / (3 * SS_H), rem = t - strip * (3 * SS_H);
@@ -271,6 +292,7 @@ __global__ void __launch_bounds__(256, 4) k_ssim_grad(const float4* __restrict__
         }
       }
       if (y_edge) {
+#pragma unroll
         for (int q = 0; q < 8; ++q)
           if (y0 + 8 * strip + q < H)
             o[q] += reflected_taps<SS_S>(&sm.f[pl][0][rx], y0 + 8 * strip + q, H, y0 - SS_R, a.g);
@@ -279,6 +301,8 @@ __global__ void __launch_bounds__(256, 4) k_ssim_grad(const float4* __restrict__
       for (int q = 0; q < 8; ++q) sm.vt[pl][8 * strip + q][rx] = o[q];
     }
     __syncthreads();
+    // the next channel's planes travel during the horizontal pass
+    if (c < 2) stage_planes(sm.f, tv + (uint64_t)(3 * (c + 1)) * a.P, a.P, x0, y0, W, H);
     // horizontal adjoint of this channel's planes at 4 pixels
     float s[3][4];
 #pragma unroll
@@ -295,20 +319,15 @@ __global__ void __launch_bounds__(256, 4) k_ssim_grad(const float4* __restrict__
         }
       }
       if (x_edge) {
+#pragma unroll
         for (int q = 0; q < 4; ++q)
           if (x0 + tx + q < W) s[pl][q] += reflected_taps<1>(&sm.vt[pl][ty][0], x0 + tx + q, W, x0 - SS_R, a.g);
       }
     }
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
-      const int x = x0 + tx + q;
-      gout[c][q] = 0.f;
-      if (x < W && y < H) {
-        const uint64_t p = (uint64_t)v * a.P + (uint64_t)y * W + x;
-        const float xs = reinterpret_cast<const float*>(pred + p)[c], tg = target[3 * p + c];
-        const float dssim = s[0][q] + 2.0f * (xs * s[1][q]) + tg * s[2][q];
-        gout[c][q] = (-a.inv_n * dssim) / 3.0f * a.scale;
-      }
+      const float dssim = s[0][q] + 2.0f * (xs[q] * s[1][q]) + tg[q] * s[2][q];
+      gout[c][q] = (-a.inv_n * dssim) / 3.0f * a.scale;
     }
   }
   if (y >= H) return;
