@@ -433,10 +433,11 @@ def stage_bytes(N: int, V: int, P: int, K: int, items: int, bw: dict, bf16: bool
     rest_b = 90 if bf16 else 180
     mom_b = 59 * 2 * (2 if bf16 else 4)
     fwd_list = bw.get("fwd_scanned", 0) * 8 + bw.get("fwd_blended", 0) * 48  # item words + blended records
-    bwd_list = bw.get("bwd_scanned", 0) * 8 + bw.get("bwd_blended", 0) * 48
+    bwd_list = bw.get("bwd_scanned", 0) * 8 + bw.get("bwd_blended", 0) * 48  # list entry, written and read + record
     tile_passes = max(1, math.ceil(max(1, (tiles - 1).bit_length()) / 8))
     return {
-        # records, zeroed gradient records, depth key, id, item count
+        # records, cleared gradient records (by the projection backward, as
+        # far as they are nonzero), depth key, id, item count
         "project": N * (56 + rest_b) + V * N * (48 + 48 + 4 + 4 + 4),
         # segmented onesweep over the 16-bit depth keys: a histogram read, then 2 passes
         # of 8-bit digits each reading and writing key + id
@@ -484,7 +485,7 @@ def run_ours(args):
         from nanotracer_b200.autotune import autotune
         cfg, trials = autotune(ctx, scene, cams0, tbuf, cfg)
         tune = {"choice": f"{cfg.tile_w}x{cfg.tile_h} tiles, sort_mode {cfg.sort_mode}, blend batch "
-                          f"{cfg.blend_batch or 'all threads'}, sort digits {cfg.sort_digit_bits or 'auto'}",
+                          f"{cfg.blend_batch or 128}, sort digits {cfg.sort_digit_bits or 'auto'}",
                 "trial_ms": {t.label: (round(t.ms, 3) if t.ms is not None else t.error) for t in trials},
                 "identical_images_per_tile_shape": all(
                     len({t.digest for t in trials if t.digest and (t.tile_w, t.tile_h) == s}) <= 1

@@ -431,9 +431,10 @@ sc_status sc_trainer_stats(const sc_trainer* tr, uint64_t* pairs, uint32_t* n_ke
  * Each call resets the accumulated stage times and counters. */
 sc_status sc_trainer_set_profiling(sc_trainer* tr, int enabled);
 /* Blend work per step, averaged over the steps since profiling was enabled
- * (two-level binning only; zeros otherwise): out[0] list positions the
- * forward's batches covered, out[1] entries it blended, out[2], out[3] the
- * same for the backward.  No counterpart in the reference. */
+ * (two-level binning only; zeros otherwise), summed over the tiles and of a
+ * tile its furthest warp's: out[0] list positions the forward covered, out[1]
+ * entries it blended, out[2], out[3] the same for the backward.  No counterpart
+ * in the reference. */
 sc_status sc_trainer_blend_work(const sc_trainer* tr, uint64_t out[4]);
 /* Contributing (pixel, entry) pairs per step with profiling level 2, averaged
  * like sc_trainer_blend_work: out[0] pixels that took an entry's alpha in the

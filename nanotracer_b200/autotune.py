@@ -12,7 +12,7 @@ Tuned axes:
   * binning path: two-level super-tile item lists, or the stable sort of the
     (tile, splat) pairs (TrainConfig.sort_mode);
   * blend batch depth: list positions the blend forward takes per stage
-    (TrainConfig.blend_batch: a quarter, half or all of the tile's threads);
+    (TrainConfig.blend_batch: 128, or a quarter or half of the tile's threads);
   * sort radix width: 8- or 9-bit digits in the binning sort's onesweep
     passes (TrainConfig.sort_digit_bits).
 The search is coordinate-wise: tile shape x binning path first (with the
@@ -50,7 +50,7 @@ from .train import TrainConfig, Trainer
 
 TILE_SHAPES = ((16, 16), (8, 8), (32, 8))
 SORT_MODES = (0, 1)        # TrainConfig.sort_mode: two-level item lists, stable pair sort
-BATCH_FRACTIONS = (4, 2)   # blend batch = threads / f, besides the default (all threads)
+BATCH_FRACTIONS = (4, 2)   # blend batch = threads / f, besides the default (128)
 DIGIT_BITS = (8, 9)        # TrainConfig.sort_digit_bits, besides the default (fewer passes wins)
 
 
@@ -79,7 +79,7 @@ def blend_threads(tile_w: int, tile_h: int) -> int:
 
 
 def batch_choices(tile_w: int, tile_h: int) -> list[int]:
-    """Blend batch depths worth trying for a tile shape (0 = all threads)."""
+    """Blend batch depths worth trying for a tile shape (0 = the default, 128)."""
     th = blend_threads(tile_w, tile_h)
     return [0] + sorted({th // f for f in BATCH_FRACTIONS if th // f >= 32 and (th // f) % 32 == 0}, reverse=True)
 

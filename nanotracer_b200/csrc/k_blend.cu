@@ -175,7 +175,7 @@ __device__ __forceinline__ float3 mse_pixel(float cr, float cg, float cb, const 
 }
 
 // Work counters of one blend launch (when given): per CTA, the list positions
-// its batches covered and the entries it staged, added into one of
+// its furthest warp covered and the entries that one kept, added into one of
 // BLEND_WORK_SLOTS (scanned, staged) pairs so that the atomics spread.
 __device__ __forceinline__ void add_work(unsigned long long* work, uint32_t scanned, uint32_t staged) {
   if (work && threadIdx.x == 0 && scanned) {

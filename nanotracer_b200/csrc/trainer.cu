@@ -10,18 +10,25 @@
 //   items (mask | view, super tile; splat) in depth order    k_super_emit (two-level binning)
 //   stable sort of the items by super tile                   onesweep u32 (super tile bits)
 //   per-super-tile ranges (+ pair count from the masks)      k_tile_ranges_u32x4
-//   alpha-blend forward over the super-tile item lists       k_composite (item lists)
-//   alpha-blend backward, MSE dL/dC in its prologue          k_composite_backward (item lists)
-//   project backward over all views -> gradient rows         k_project_backward_shards (one shard)
+//   alpha-blend forward over the super-tile item lists;
+//     writes down each warp's takers (exact backward)        k_composite (item lists)
+//   tiles with the longest walks (one launch for all views)  k_heavy_tiles
+//   alpha-blend backward over the takers, MSE dL/dC in its
+//     prologue                                               k_composite_backward
+//   project backward over all views -> gradient rows;
+//     clears the projected gradients it read                 k_project_backward_shards (one shard)
 //   Adam + constraints + densify statistic over the rows     k_adam_rows
-//   loss / pair count / error word -> pinned host            finalize + memcpy node
+//   loss / pair count / error word -> pinned host            k_finalize (writes the host memory itself)
+// One fill clears what a step counts in (ensure_zero_block).  With the reference's
+// backward mode both blends walk the item lists.
 // (sort_mode 1 keeps the pair path: emission of (view*T + tile, splat) pairs,
 // their stable tile sort, per-tile ranges and pair-list blends.)
 //
 // The item (or pair) buffers have a device-side capacity.  When a step emits
 // more than fit, the emit kernel raises SC_DEVERR_CAPACITY, the blend and Adam
 // kernels of that step skip their work (parameters are untouched), and the host
-// grows the buffers and runs the step again.
+// grows the buffers and runs the step again.  The forward's taker chunks are bounded
+// the same way (SC_DEVERR_TAKERS: backward and Adam are skipped).
 #include "sc_internal.cuh"
 
 #include <algorithm>
