@@ -88,7 +88,6 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-#define ALPHA_MIN (1.0f / 255.0f)
 #define ALPHA_MAX 0.99f
 #define FULL_MASK 0xffffffffu
 
@@ -278,7 +277,7 @@ __device__ __forceinline__ bool reaches(const float4 ra, const float4 rb, float 
   const float wr = fminf(fmaxf(-s.kx, a0), a1), wl = fminf(fmaxf(s.kx, a0), a1);
   const float ur = (-s.b * wr + cull_sqrt(fmaxf(s.L * s.a - wr * wr * s.det, 0.0f))) * s.inv_a;
   const float ul = (-s.b * wl - cull_sqrt(fmaxf(s.L * s.a - wl * wl * s.det, 0.0f))) * s.inv_a;
-  const bool out = op * 255.0f <= 1.0f ||
+  const bool out = op < ALPHA_MIN ||
                    (!s.keep && op == op &&
                     (w1 < -s.yh || w0 > s.yh || s.mx + ur + 1e-2f < w.x0 || s.mx + ul - 1e-2f > w.x1));
   return !out;

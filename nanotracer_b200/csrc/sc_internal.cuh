@@ -119,6 +119,9 @@ __device__ __forceinline__ void sp_set(const DSplats& s, int r, uint32_t i, floa
   s.slab[(size_t)r * s.cap + i] = v;
 }
 
+// the blend skips a pixel whose alpha is below this
+#define ALPHA_MIN (1.0f / 255.0f)
+
 // ---------------------------------------------------------------- tile culling
 // A pixel reaches alpha = op exp(-q/2) >= 1/255 only inside the ellipse
 // q(u, w) = a u^2 + 2 b u w + c w^2 <= L, L = 2 ln(255 op) (u, w: offsets from
@@ -132,6 +135,8 @@ __device__ __forceinline__ void sp_set(const DSplats& s, int r, uint32_t i, floa
 // and the interval by 1e-3 px, so float rounding in the blend can never
 // accept a pixel this test rejects; the same margins cover the SFU
 // approximations used here (relative errors near 1e-7, i.e. below 1e-5 px).
+// The opacity itself is compared as the blend compares alpha: op == ALPHA_MIN
+// is taken at the splat's centre, although 255 op rounds to 1.
 // Counting (projection) and emission call the same functions, so they agree.
 __device__ __forceinline__ float cull_sqrt(float x) {
   float r;
@@ -140,7 +145,7 @@ __device__ __forceinline__ float cull_sqrt(float x) {
 }
 struct CullShape {
   float mx, my, a, b, det, L, xh, yh, kx, inv_a;
-  bool any;   // op > 1/255 and the conic is positive definite
+  bool any;   // op >= ALPHA_MIN: some alpha may pass
   bool keep;  // not positive definite: keep the reference rectangle whole
 };
 
@@ -153,7 +158,7 @@ __device__ __forceinline__ CullShape cull_shape(float mx, float my, float a, flo
   // margins below, and the blend's own evaluation of the quadratic form is
   // noisy along the needle: such a splat keeps its whole rectangle.
   s.keep = !(a > 0.0f && c > 0.0f && s.det > 9.765625e-4f * a * c);
-  s.any = op * 255.0f > 1.0f;
+  s.any = op >= ALPHA_MIN;
   const float q = 2.0f * __logf(fmaxf(op * 255.0f, 1.0f));
   s.L = q + 1e-3f * q + 1e-3f;
   s.xh = cull_sqrt(__fdividef(s.L * c, s.det));

@@ -16,8 +16,8 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from nanotracer_b200 import CameraUniform, GpuSplatBuffer, GradSplatBuffers, TilingParams
-from nanotracer_b200._lib import SC_BWD_EXACT, SC_BWD_REF, check, lib
+from nanotracer_b200 import CameraUniform, GpuSplatBuffer, GradSplatBuffers, Rasterizer, TileBinner, TilingParams
+from nanotracer_b200._lib import SC_BWD_EXACT, SC_BWD_REF, SC_KEYS_REF32, check, lib
 from nanotracer_b200.raster import cameras_array
 from nanotracer_b200.scene import FOV_Y, orbit_pose, random_scene
 from nanotracer_b200.train import TrainConfig, Trainer
@@ -130,3 +130,34 @@ def test_trainer_backward_starts_heavy_tiles_first(ctx, n, size):
     for lo, hi in [(0, 3), (3, 7), (7, 10), (10, 11), (11, 14), (14, 59)]:
         d = np.linalg.norm((got[lo:hi] - want[lo:hi]).astype(np.float64))
         assert d <= 1e-5 * np.linalg.norm(want[lo:hi].astype(np.float64)), (lo, d)
+
+
+@pytest.mark.parametrize("mode", [SC_BWD_EXACT, SC_BWD_REF])
+def test_a_splat_at_the_alpha_threshold_is_blended_at_its_centre(ctx, oracle, mode):
+    """The blend takes alpha >= 1/255; a splat of exactly that opacity reaches
+    it at a pixel on its centre (g = 1), one float below it nowhere."""
+    W, H = 33, 19
+    at = np.float32(1.0) / np.float32(255.0)
+    rec = np.zeros((2, 12), np.float32)
+    for k, (x, op) in enumerate([(8.5, at), (24.5, np.nextafter(at, np.float32(0)))]):
+        rec[k] = [x, 9.5, 1.0, 6.0, 0.4, 0.1, 0.3, 1.0, 0.9, 0.5, 0.2, op]
+    tl = TilingParams(W, H, 16, 8.0)
+    r, binner = Rasterizer(ctx), TileBinner(ctx)
+    proj = ctx.storage_buffer("rec", rec)
+    bins = binner.bin(proj, 2, tl, stride=2, n_views=1, key_mode=SC_KEYS_REF32)
+    img, aux = r.alloc_image(W, H), r.alloc_aux(W, H)
+    r.composite(proj, bins, img, tl, 2, 1, aux=aux)
+    got = img.readback(np.float32).reshape(H, W, 4)
+    otl = oracle.tiling(W, H, 16, 16, 8.0)
+    _, pay, ranges = oracle.bin_ref(rec, otl)
+    want, _, _ = oracle.composite(rec, pay, ranges, otl)
+    want = np.asarray(want).reshape(H, W, 4)
+    assert want[9, 8, 3] > 0 and (want[..., 3] > 0).sum() == 1
+    assert np.allclose(got, want, rtol=0, atol=1e-7)
+    dl = np.full((H, W, 4), 0.5, np.float32)
+    pg = ctx.storage_buffer_zeroed("pg", rec.nbytes)
+    r.composite_backward(proj, bins, img, ctx.storage_buffer("dl", dl), pg, tl, 2, 1, mode=mode, aux=aux)
+    g = pg.readback(np.float32).reshape(2, 12)
+    # one pixel at T = 1, dx = dy = 0: dcolor = alpha dL/dC, dopacity = dL/dC . colour
+    assert np.allclose(g[0, 8:11], 0.5 * at, rtol=1e-6) and abs(g[0, 2] - 0.5 * 1.6) <= 1e-5
+    assert not g[1].any()
