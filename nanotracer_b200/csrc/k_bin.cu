@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(EMIT_WARPS * 32) k_presorted_emit(
       const float4 ra = rec[3 * o], rb = rec[3 * o + 1], rc = rec[3 * o + 2];
       if (!rect_of(ra, rb, a, x0, y0, x1, y1)) { x0 = 0; y0 = 0; x1 = -1; y1 = -1; }
       cs = cull_shape(ra.x, ra.y, rb.x, rb.y, rb.z, rc.w);
-      test = cull && !cs.keep;
+      test = cull_test(cs, cull, rc.w);
       vbase = v << a.tile_bits;
     }
   }
@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(SE_THREADS) k_super_emit(
       const float4 ra = rec[3 * o], rb = rec[3 * o + 1], rc = rec[3 * o + 2];
       if (!rect_of(ra, rb, a, x0, y0, x1, y1)) { x0 = 0; y0 = 0; x1 = -1; y1 = -1; }
       cs = cull_shape(ra.x, ra.y, rb.x, rb.y, rb.z, rc.w);
-      test = (cull & 1) && !cs.keep;
+      test = cull_test(cs, cull, rc.w);
       vkey = v << super_bits;
     }
   }

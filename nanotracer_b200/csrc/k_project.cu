@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(PROJ_THREADS, 8) k_project(DSplats s_all, cons
             int x0, y0, x1, y1;
             if (tile_rect(mx, my, radius, 1.0f, ta.tw, ta.th, ta.tiles_x, ta.tiles_y, x0, y0, x1, y1)) {
               const CullShape cs = cull_shape(mx, my, g.ca, g.cb, g.cc, opacity);
-              const bool test = ta.cull && !cs.keep;
+              const bool test = cull_test(cs, (int)ta.cull, opacity);
               if (ta.super) {
                 for (int sy = y0 / SC_SUPER; sy <= y1 / SC_SUPER; ++sy) {
                   int sx0, sx1;
@@ -378,7 +378,7 @@ static sc_status project_cams(sc_ctx* ctx, const DSplats& s, const CAMS& cams, u
   if (stride == 0 || n_views == 0) return SC_OK;
   TileArgs ta{1, 1, 1, 1, 0, 0, 1.0f};
   if (tl) ta = TileArgs{tl->tile_w, tl->tile_h, (tl->width + tl->tile_w - 1) / tl->tile_w,
-                        (tl->height + tl->tile_h - 1) / tl->tile_h, (cull & 1) ? 1u : 0u, (cull & 2) ? 1u : 0u,
+                        (tl->height + tl->tile_h - 1) / tl->tile_h, (uint32_t)(cull & 5), (cull & 2) ? 1u : 0u,
                         tl->depth_max};
   const uint32_t bs = PROJ_THREADS;  // grid: (splats / bs) x views CTAs, views innermost
   const uint64_t blocks = sc_div_up(stride, bs) * (uint64_t)n_views;

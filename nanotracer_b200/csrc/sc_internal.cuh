@@ -168,6 +168,13 @@ __device__ __forceinline__ CullShape cull_shape(float mx, float my, float a, flo
   return s;
 }
 
+// Whether the ellipse decides the splat's tiles (bit 0 of cull), or its whole
+// rectangle is listed.  Bit 2, the viewer's frame, lists a splat of NaN opacity
+// too, as sc_bin does: the blend clamps its alpha to 0.99.
+__device__ __forceinline__ bool cull_test(const CullShape& s, int cull, float op) {
+  return (cull & 1) && !s.keep && !((cull & 4) && op != op);
+}
+
 // Tiles [tlo, thi] of row ty (tile width tw, height th) that the ellipse can
 // reach; false when the row misses it.  Caller clamps to the 3-sigma rectangle.
 __device__ __forceinline__ bool cull_row_span(const CullShape& s, int ty, uint32_t tw, uint32_t th, int& tlo,
@@ -340,7 +347,7 @@ namespace sck {
 // writes per (view, splat) a depth sort key (float bits, 0xFFFFFFFF when the
 // splat emits no pairs; one segment of stride keys per view) and a count for
 // the native pipeline: (tile, splat) pairs, or with bit 1 of `cull` two-level
-// binning items.  Bit 0 of `cull`: exact tile culling.
+// binning items.  Bits 0 and 2 of `cull`: exact tile culling (cull_test).
 // scenes (nullable, n_views entries): view v projects scene v's own store
 // (its first scene.s.n splats; the rest of the view's stride is culled).
 sc_status launch_project(sc_ctx* ctx, const DSplats& s, const sc_camera* d_cams, uint32_t n_views,

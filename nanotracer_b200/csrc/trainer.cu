@@ -417,10 +417,11 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
   uint64_t* work_bwd = tr->profiling ? tr->d_work + 3 * sck::BLEND_WORK_SLOTS : nullptr;
   if (tr->profiling)
     SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->d_work, 0, 6 * sck::BLEND_WORK_SLOTS * 8, ctx->stream), "zero work");
+  const int cull = tr->cfg.tile_cull ? (tr->forward_only ? 5 : 1) : 0;
   mark(tr, 0, capturing);
   SC_TRY(sck::launch_project(ctx, ds, d_cams, V, tr->stride, tr->rec, &tr->cfg.tiling, tr->dkeys, tr->ids,
                              tr->counts_by_id, tr->cfg.fp64_det ? 1 : 0,
-                             (tr->cfg.tile_cull ? 1 : 0) | (tr->two_level ? 2 : 0),
+                             cull | (tr->two_level ? 2 : 0),
                              tr->scenes_mode ? tr->d_scenes : nullptr));
   mark(tr, 1, capturing);
   bool in_tmp = false;
@@ -436,7 +437,6 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
     // items (member mask | view, super tile; splat) in depth order, grouped
     // per super tile by a stable sort; each tile then blends the items of its
     // super tile whose mask holds it
-    const int cull = tr->cfg.tile_cull ? 1 : 0;
     uint64_t* d_items = tr->d_total + 1;
     // item counts in depth order (gathered through the sorted ids) -> offsets
     SC_TRY(sck::scan_u32_gather(ctx, tr->counts, nsp + 1, tr->counts_by_id, sorted_ids, tr->stride, nsp, d_items,
@@ -470,8 +470,7 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
   }
   mark(tr, 3, capturing);
   SC_TRY(sck::launch_presorted_emit(ctx, tr->rec, tr->stride, V, sorted_ids, tr->counts, tr->counts_by_id,
-                                    &tr->cfg.tiling, tr->keys, tr->vals, tr->kcap, ctx->d_error,
-                                    (int)tr->cfg.tile_cull));
+                                    &tr->cfg.tiling, tr->keys, tr->vals, tr->kcap, ctx->d_error, cull));
   mark(tr, 4, capturing);
   // keys are (view << tile_bits) | tile: the stable sort on the tile bits alone
   // groups the pairs by tile, then view (the emission is view-major), then depth

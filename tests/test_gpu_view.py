@@ -75,3 +75,24 @@ def test_frame_equals_the_stage_calls_bit_for_bit(ctx, n, size, distance):
             assert np.array_equal(px, out.readback(np.uint8).reshape(H, W, 4))
     finally:
         ctx.set_fp64_det(False)
+
+
+@pytest.mark.gpu
+def test_frame_shows_a_splat_of_nan_opacity_as_the_stage_calls_do(ctx):
+    """A NaN alpha is clamped to 0.99 by the blend: such a splat covers its
+    rectangle's pixels in the stage calls, and so it does in the frame."""
+    from nanotracer_b200 import CameraUniform, TilingParams
+    from tests.util import GpuPipe
+    W, H, n = 120, 75, 40
+    scene = random_scene(n, 5)
+    scene.opacities[::9] = np.nan
+    view = HeadlessView(ctx, scene, W, H)
+    orbit = OrbitCamera(distance=3.0, azimuth=0.7, elevation=0.1)
+    view.frame(orbit)
+    cam = CameraUniform.from_pose(orbit.position(), orbit.target, (0.0, 1.0, 0.0), orbit.fov_y, W, H, n)
+    pipe = GpuPipe(ctx, scene, cam, TilingParams(W, H, 16, 50.0))
+    rec = pipe.project()[0]
+    pipe.bin()
+    img, _ = pipe.composite()
+    assert (np.isnan(rec[:, 11]) & (rec[:, 7] != 0)).any()
+    assert np.array_equal(view.hdr(), img[0])
