@@ -1094,13 +1094,27 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
     const float2 gr2 = make_float2(gr[0], gr[PPT - 1]), gg2 = make_float2(gg[0], gg[PPT - 1]);
     const float2 gb2 = make_float2(gb[0], gb[PPT - 1]), fy2 = make_float2(fy[0], fy[PPT - 1]);
     bool stopped = false;
+    // An entry of a list need not be taken by a pixel of the warp, and one that
+    // no pixel takes sends nothing; nor does a pixel add to an entry that it
+    // skips.  Both matter where zeros would not do: a pixel whose dL/dC is not
+    // finite (odd: the warp has one), an entry whose record is not.  The takers
+    // are taken by definition.
+    constexpr bool GATED = LIST != LIST_TAKERS;
+    uint32_t took = 0;  // octet path: the rows that this thread's pixels took
+    bool odd = false;
+    if constexpr (GATED && OCT) {
+      float s = 0.0f;
+#pragma unroll
+      for (int q = 0; q < PPT; ++q) s += fabsf(gr[q]) + fabsf(gg[q]) + fabsf(gb[q]);
+      odd = __any_sync(FULL_MASK, !(s < INFINITY));
+    }
     // octet path: a thread's two pixels' (h, -T alpha) of entry i (zeros where a
     // pixel skips it).  Alpha is carried negated, which needs no negations in
     // the packed operations; a skipping pixel gets alpha 0, so it keeps its T
     // (1 / 1 is exact) and its sums.
     // `plain`: the stage's records are plain and no pixel of the warp stops
     // behind its entries, which leaves the alpha >= 1/255 test alone.
-    auto entry2 = [&](auto plain, uint32_t i, const float4* r) -> float4 {
+    auto entry2 = [&](auto plain, uint32_t i, uint32_t row, const float4* r) -> float4 {
       constexpr bool PLAIN = decltype(plain)::value;
       const float4 ra = r[0], rb = r[1], rc = r[2];
       const EntryGeom e = entry_geom(fx, ra, rb);
@@ -1126,8 +1140,14 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
       // dC/dalpha = T_i c - S / (1 - alpha) = (T_{i+1} c - S) / (1 - alpha)
       const float2 dc = make_float2(fmaf(gb2.x, rc.z, fmaf(gg2.x, rc.y, gr2.x * rc.x)),
                                     fmaf(gb2.y, rc.z, fmaf(gg2.y, rc.y, gr2.y * rc.x)));
-      const float2 h = __fmul2_rn(__fmul2_rn(inv, __ffma2_rn(T2, dc, NG2)), gm);
-      NG2 = __ffma2_rn(ta, dc, NG2);
+      float2 h = __fmul2_rn(__fmul2_rn(inv, __ffma2_rn(T2, dc, NG2)), gm);
+      float2 ng = __ffma2_rn(ta, dc, NG2);
+      if constexpr (GATED) {
+        if (!v0) { h.x = 0.0f; ng.x = NG2.x; }
+        if (!v1) { h.y = 0.0f; ng.y = NG2.y; }
+        if (v0 || v1) took |= 1u << row;
+      }
+      NG2 = ng;
       T2 = Tn;
       if constexpr (COUNT) w_pix += (uint32_t)v0 + (uint32_t)v1;
       if (MODE == SC_BWD_REF) all_done = (done[0] || j == 0) && (done[PPT - 1] || j == 0);
@@ -1136,14 +1156,25 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
     // turn round: the sums of entries i0 .. i0 + rows - 1 over the warp's pixels, and out
     auto turn = [&](uint32_t i0, uint32_t rows) {
       if constexpr (OCT) {
+        uint32_t taken = 0xFFFFFFFFu;
+        if constexpr (GATED) {
+          taken = __reduce_or_sync(FULL_MASK, took);
+          took = 0;
+        }
         __syncwarp();
         const float4* w = sm.red.row + oe * OCT_ROW + oq * 8;
         const float4 m = feed.rec()[3 * (i0 + oe)];
         float2 sh = f2(0.f), shx = sh, shxx = sh, cr = sh, cg = sh, cb = sh;
 #pragma unroll
         for (int j = 0; j < 8; ++j) {
-          const float4 x = w[j], rg = sm.red.rg[oq * 9 + j];
-          const float2 b = sm.red.b[oq * 9 + j], h = make_float2(x.x, x.y), ta = make_float2(x.z, x.w);
+          const float4 x = w[j];
+          const float2 h = make_float2(x.x, x.y), ta = make_float2(x.z, x.w);
+          float4 rg = sm.red.rg[oq * 9 + j];
+          float2 b = sm.red.b[oq * 9 + j];
+          if (GATED && odd) {  // T alpha is 0 where the pixel skips the entry only
+            if (ta.x == 0.0f) rg.x = rg.z = b.x = 0.0f;
+            if (ta.y == 0.0f) rg.y = rg.w = b.y = 0.0f;
+          }
           const float2 dx = f2(__fadd_rn(fx_oct + (float)j, -m.x));
           const float2 hx = __fmul2_rn(h, dx);
           sh = __fadd2_rn(sh, h);
@@ -1161,14 +1192,15 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
         float c6[6], c3[3];
         rs_half<12, 16>(c, c6, lane);
         rs_half<6, 8>(c6, c3, lane);
-        if (oe < rows && oq < 3) send(i0 + oe, oq, make_float3(c3[0], c3[1], c3[2]));
+        if (oe < rows && oq < 3 && (taken >> oe & 1u)) send(i0 + oe, oq, make_float3(c3[0], c3[1], c3[2]));
         __syncwarp();  // the rows may be written again
       }
     };
     // general path: this thread's raw sums of entry i over its pixels into
     // c[0..8]: h = dL/dalpha * gauss (the opacity gradient), its first and second
-    // moments in (dx, dy), and the colour gradient
-    auto entry = [&](uint32_t i, const float4* r, float* c) {
+    // moments in (dx, dy), and the colour gradient; whether one of them took it
+    auto entry = [&](uint32_t i, const float4* r, float* c) -> bool {
+      bool contrib = false;
       const uint32_t j = feed.pos(i);
       const float4 ra = r[0], rb = r[1], rc = r[2];
       const EntryGeom e = entry_geom(fx, ra, rb);
@@ -1196,12 +1228,14 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
               c[3] += hx * e.dx; c[4] += hx * dy; c[5] += hy * dy;
               ng -= ta * dc;
               Tq = Tn;
+              contrib = true;
               if constexpr (COUNT) ++w_pix;
             }
           }
         }
         if (MODE == SC_BWD_REF) all_done &= done[q] || j == 0;
       }
+      return contrib;
     };
     const WarpRect rect = LIST == LIST_TAKERS ? WarpRect{} : warp_rect(px, py0, PPT);
     for (uint32_t n_raw = feed.gather(); n_raw > 0 && !stopped;) {
@@ -1215,12 +1249,12 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
         auto walk = [&](auto plain) {
           for (; i + OCT_E <= n && !stopped; i += OCT_E) {
 #pragma unroll
-            for (int e = 0; e < OCT_E; ++e) row[e * OCT_ROW] = entry2(plain, i + e, sr + 3 * (i + e));
+            for (int e = 0; e < OCT_E; ++e) row[e * OCT_ROW] = entry2(plain, i + e, e, sr + 3 * (i + e));
             turn(i, OCT_E);
             if (MODE == SC_BWD_REF) stopped = __all_sync(FULL_MASK, all_done);
           }
           if (i < n && !stopped) {
-            for (uint32_t e = 0; i + e < n; ++e) row[e * OCT_ROW] = entry2(plain, i + e, sr + 3 * (i + e));
+            for (uint32_t e = 0; i + e < n; ++e) row[e * OCT_ROW] = entry2(plain, i + e, e, sr + 3 * (i + e));
             turn(i, n - i);
             if (MODE == SC_BWD_REF) stopped = __all_sync(FULL_MASK, all_done);
           }
@@ -1239,12 +1273,12 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
           float c[9 * RS_E];
 #pragma unroll
           for (int q = 0; q < 9 * RS_E; ++q) c[q] = 0.0f;
-          entry(i, sr + 3 * i, c);
-          if (two) entry(i + 1, sr + 3 * i + 3, c + 9);
+          const bool any0 = __any_sync(FULL_MASK, entry(i, sr + 3 * i, c));
+          const bool any1 = two && __any_sync(FULL_MASK, entry(i + 1, sr + 3 * i + 3, c + 9));
           const float w = warp_reduce_scatter<9 * RS_E>(c, lane);
           if (rs_idx >= 0) sm.red.sum[rs_idx] = w;
           __syncwarp();
-          if (lane < (two ? 6 : 3)) {
+          if (lane < 3 ? any0 : lane < 6 && any1) {
             const float* m = sm.red.sum + 3 * lane;
             send(i + lane / 3, lane % 3, make_float3(m[0], m[1], m[2]));
           }

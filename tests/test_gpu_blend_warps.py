@@ -161,3 +161,42 @@ def test_a_splat_at_the_alpha_threshold_is_blended_at_its_centre(ctx, oracle, mo
     # one pixel at T = 1, dx = dy = 0: dcolor = alpha dL/dC, dopacity = dL/dC . colour
     assert np.allclose(g[0, 8:11], 0.5 * at, rtol=1e-6) and abs(g[0, 2] - 0.5 * 1.6) <= 1e-5
     assert not g[1].any()
+
+
+@pytest.mark.parametrize("mode", [SC_BWD_EXACT, SC_BWD_REF])
+@pytest.mark.parametrize("tile", TILES)
+def test_a_gradient_that_is_not_finite_reaches_the_splats_of_its_pixel_only(ctx, tile, mode):
+    """A pixel skips a splat by adding nothing to it: with dL/dC of NaN or
+    infinity at two pixels, the projected gradients that are not finite are those
+    of the splats that these pixels take, and the others are what they are with
+    zeros there.  A splat whose record is NaN, which no pixel takes, gets zeros."""
+    n, W, H = 900, 61, 45
+    cam = CameraUniform.from_pose(*orbit_pose(35.0), FOV_Y, W, H, n)
+    pipe = GpuPipe(ctx, _scene(n), cam, TilingParams(W, H, tile[0], 8.0, tile_h_override=tile[1]))
+    rec = pipe.project()[0].copy()
+    broken = np.arange(n) % 100 == 0
+    rec[broken, :4] = np.nan, 20.0, 3.0, 40.0  # listed in tile column 0
+    rec[broken, 7] = 1.0
+    pipe.proj.upload(rec)
+    _, pay, _ = pipe.bin()
+    assert np.isin(np.flatnonzero(broken), pay).all()
+    img, aux = pipe.composite()
+    assert np.isfinite(img).all()
+    dl = np.zeros((1, H, W, 4), np.float32)
+    dl[..., :3] = np.random.default_rng(3).normal(0, 1e-3, (1, H, W, 3))
+    spots = [(20, 30), (33, 17)]
+    only = np.zeros_like(dl)
+    for y, x in spots:
+        dl[0, y, x, :3] = 0.0
+        only[0, y, x, :3] = 1.0
+    base = pipe.backward(dl, mode)[0]
+    taken = pipe.backward(only, mode)[0][:, 8:11].any(axis=1)  # dcolor = sum T alpha dL/dC
+    assert 0 < taken.sum() < n // 2
+    for (y, x), bad in zip(spots, (np.nan, np.inf)):
+        dl[0, y, x, :3] = bad
+    got = pipe.backward(dl, mode)[0]
+    assert not got[broken].any()
+    assert not np.isfinite(got[taken]).all(axis=1).any()
+    # the atomics' order differs between the runs
+    scale = np.abs(base).max(axis=0)
+    assert np.allclose(got[~taken], base[~taken], rtol=1e-4, atol=1e-6 * scale.max())
