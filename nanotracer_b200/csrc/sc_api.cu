@@ -18,6 +18,7 @@ sc_status sc_fail(sc_ctx* ctx, sc_status st, const std::string& msg) {
 
 sc_status sc_cuda_fail(sc_ctx* ctx, cudaError_t e, const char* what) {
   if (ctx) ctx->last_error = std::string(what) + ": " + cudaGetErrorString(e);
+  cudaGetLastError();  // reported here: the next launch's check must not find it again
   return e == cudaErrorMemoryAllocation ? SC_ERR_OOM : SC_ERR_CUDA;
 }
 

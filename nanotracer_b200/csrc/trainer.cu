@@ -352,21 +352,29 @@ static sc_status ensure_pairs(sc_trainer* tr, uint64_t K) {
   return ensure_scratch(tr);
 }
 
-// taker chunks per pool
+// Taker chunks per pool.  The chunks that are there go only once the larger
+// ones have been had: every step's forward writes into them, so there is no
+// state without any.
 static sc_status ensure_takers(sc_trainer* tr, uint64_t chunks) {
   if (tr->forward_only || tr->cfg.bwd_mode != SC_BWD_EXACT || chunks <= tr->takers.pool_cap) return SC_OK;
   sc_ctx* ctx = tr->ctx;
   const uint64_t cap = chunks + chunks / 4 + 64;
   if (cap * sck::TAKER_POOLS > 0xFFFFFFFFull) return sc_fail(ctx, SC_ERR_CAPACITY, "too many blended entries in one step");
-  SC_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream), "sync");
+  uint32_t *ids = nullptr, *prev = nullptr;
+  cudaError_t e = cudaMalloc(&ids, cap * sck::TAKER_POOLS * 32 * 4);
+  if (e == cudaSuccess) e = cudaMalloc(&prev, cap * sck::TAKER_POOLS * 4);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+  if (e != cudaSuccess) {
+    cudaFree(ids);
+    cudaFree(prev);
+    return sc_cuda_fail(ctx, e, "takers");
+  }
+  trainer_drop_graph(tr);
   cudaFree(tr->takers.ids);
   cudaFree(tr->takers.prev);
-  tr->takers.ids = tr->takers.prev = nullptr;
-  tr->takers.pool_cap = 0;
-  SC_CUDA_TRY(ctx, cudaMalloc(&tr->takers.ids, cap * sck::TAKER_POOLS * 32 * 4), "takers");
-  SC_CUDA_TRY(ctx, cudaMalloc(&tr->takers.prev, cap * sck::TAKER_POOLS * 4), "takers");
+  tr->takers.ids = ids;
+  tr->takers.prev = prev;
   tr->takers.pool_cap = (uint32_t)cap;
-  trainer_drop_graph(tr);
   return SC_OK;
 }
 

@@ -1,0 +1,86 @@
+"""Host paths that a GPU test must not bring about: allocations that fail in
+the middle of a step, and the sizes of arrays that kernels read.  The library's
+own objects are linked with a CUDA runtime whose device memory is host memory
+(fake_cudart.cpp) and run in a child process; no kernel runs."""
+import os
+import subprocess
+import sys
+from pathlib import Path
+
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+
+PRELUDE = """
+import numpy as np
+from nanotracer_b200 import AdamMomentBuffers, CameraUniform, CudaCtx, GpuSplatBuffer, TilingParams
+from nanotracer_b200._lib import SplatCudaError, lib
+from nanotracer_b200.scene import FOV_Y, orbit_pose, random_scene
+from nanotracer_b200.train import TrainConfig, Trainer
+import ctypes as C
+L = lib()
+for f in (L.fake_bad, L.fake_composites, L.fake_replays, L.fake_pool_cap):
+    f.restype = C.c_uint64
+L.fake_step.argtypes = [C.c_uint64, C.c_uint64, C.c_uint32, C.c_uint32]
+L.fake_scan_total.argtypes = [C.c_uint64]
+CAPACITY, TAKERS = 2, 4
+ctx = CudaCtx(0)
+scene = random_scene(300, 1)
+W, H = 64, 48
+cam = CameraUniform.from_pose(*orbit_pose(10.0), FOV_Y, W, H, 300)
+
+def trainer(**kw):
+    cfg = TrainConfig(n_views=1, width=W, height=H, depth_max=8.0, **kw)
+    g = GpuSplatBuffer.upload(ctx, scene)
+    mo = AdamMomentBuffers(ctx, g.capacity)
+    acc = ctx.storage_buffer_zeroed("acc", 4 * g.capacity)
+    tr = Trainer(ctx, cfg)
+    tr.set_targets(ctx.storage_buffer_zeroed("targets", 12 * W * H))
+    n = [0]
+    def step():
+        n[0] += 1
+        return tr.step(g, mo, acc, [cam], n[0])
+    return tr, step
+"""
+
+
+@pytest.fixture(scope="module")
+def fake_lib(tmp_path_factory):
+    from nanotracer_b200 import build
+    build.build()
+    out = tmp_path_factory.mktemp("fake") / "libsplatcuda_fake.so"
+    cuda = Path(build._nvcc()).resolve().parents[1] / "include"
+    subprocess.run(["g++", "-std=c++17", "-O1", "-shared", "-fPIC", "-Wl,-Bsymbolic", "-I", str(cuda),
+                    str(Path(__file__).with_name("fake_cudart.cpp")), *map(str, sorted(build.BUILD.glob("*.o"))),
+                    "-o", str(out)], check=True)
+    return out
+
+
+def run(fake_lib, body):
+    r = subprocess.run([sys.executable, "-c", PRELUDE + body], cwd=ROOT, capture_output=True, text=True, timeout=300,
+                       env={**os.environ, "SPLATCUDA_LIB": str(fake_lib), "PYTHONPATH": str(ROOT)})
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+@pytest.mark.parametrize("sort_mode", [0, 1])
+@pytest.mark.parametrize("nth", [1, 2])
+def test_a_step_after_a_failed_growth_of_the_takers_runs_on_live_chunks(fake_lib, sort_mode, nth):
+    """A step draws more chunks than there are, and the larger arrays cannot be
+    had (the first or the second of them): the call fails, and the next steps
+    blend into chunks that are there and grow them as soon as they can."""
+    run(fake_lib, f"""
+tr, step = trainer(sort_mode={sort_mode})
+step(), step()
+L.fake_step(0, 0, TAKERS, 5000)
+L.fake_fail({nth})
+try:
+    step()
+    raise SystemExit("the failed allocation was not reported")
+except SplatCudaError as e:
+    assert e.status == 2, e
+step()
+assert L.fake_bad() == 0, "a blend ran without its chunks"
+L.fake_step(0, 0, TAKERS, 5000)
+step()
+assert L.fake_bad() == 0 and L.fake_pool_cap() >= 5000
+""")
