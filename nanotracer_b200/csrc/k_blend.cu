@@ -332,8 +332,8 @@ struct ListFeed {
   __device__ __forceinline__ bool mine() const {
     return REV ? at > begin + 4 * (threadIdx.x & 31) : first() < end;
   }
-  // the lists' arrays are 16-byte aligned and go on past their last entry, so a
-  // group of four holding a walked position is readable whole
+  // the lists' arrays are 16-byte aligned and hold whole groups of four words
+  // (sc_list_bytes), so a group holding a walked position is readable whole
   __device__ __forceinline__ void load() {
     if (mine()) {
       if (LIST == LIST_ITEMS) key = __ldg(reinterpret_cast<const uint4*>(keys + first()));

@@ -593,8 +593,8 @@ sc_status sc_bin(sc_ctx* ctx, const sc_projected_splat* projected, uint32_t n, u
     const uint64_t cap = K + K / 8 + 1024;
     SC_CUDA_TRY(ctx, cudaMalloc(&b->keys, cap * kb), "keys alloc");
     SC_CUDA_TRY(ctx, cudaMalloc(&b->keys_tmp, cap * kb), "keys alloc");
-    SC_CUDA_TRY(ctx, cudaMalloc(&b->vals, cap * 4), "vals alloc");
-    SC_CUDA_TRY(ctx, cudaMalloc(&b->vals_tmp, cap * 4), "vals alloc");
+    SC_CUDA_TRY(ctx, cudaMalloc(&b->vals, sc_list_bytes(cap)), "vals alloc");
+    SC_CUDA_TRY(ctx, cudaMalloc(&b->vals_tmp, sc_list_bytes(cap)), "vals alloc");
     b->cap = cap;
   }
   if (K == 0) {

@@ -337,6 +337,10 @@ static inline void sc_launch(sc_ctx* ctx, void (*kernel)(P...), dim3 grid, unsig
 // First statement of such a kernel: waits for the kernel before.
 __device__ __forceinline__ void sc_after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// Bytes of a list array of n words (ids, keys, payloads): the blends read lists
+// in aligned groups of four words, the last of which may go past the list's end.
+static inline size_t sc_list_bytes(uint64_t n) { return (size_t)((n + 3) / 4) * 16; }
+
 static inline uint64_t sc_div_up(uint64_t a, uint64_t b) { return (a + b - 1) / b; }
 
 // ---------------------------------------------------------------- kernel entry points

@@ -316,15 +316,15 @@ static sc_status ensure_items(sc_trainer* tr, uint64_t I) {
   uint64_t cap = I + I / 4 + 65536;
   if (cap > (1ull << 30) - 1) cap = (1ull << 30) - 1;
   if (I > cap) return sc_fail(ctx, SC_ERR_CAPACITY, "more than 2^30 binning items in one step");
-  SC_CUDA_TRY(ctx, cudaMalloc(&tr->ikeys, cap * 4), "items");
-  SC_CUDA_TRY(ctx, cudaMalloc(&tr->ikeys_tmp, cap * 4), "items");
-  SC_CUDA_TRY(ctx, cudaMalloc(&tr->ivals, cap * 4), "items");
-  SC_CUDA_TRY(ctx, cudaMalloc(&tr->ivals_tmp, cap * 4), "items");
+  SC_CUDA_TRY(ctx, cudaMalloc(&tr->ikeys, sc_list_bytes(cap)), "items");
+  SC_CUDA_TRY(ctx, cudaMalloc(&tr->ikeys_tmp, sc_list_bytes(cap)), "items");
+  SC_CUDA_TRY(ctx, cudaMalloc(&tr->ivals, sc_list_bytes(cap)), "items");
+  SC_CUDA_TRY(ctx, cudaMalloc(&tr->ivals_tmp, sc_list_bytes(cap)), "items");
   // zero-filled so a step whose emission overflowed still reads valid ids
-  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->ivals, 0, cap * 4, ctx->stream), "zero");
-  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->ivals_tmp, 0, cap * 4, ctx->stream), "zero");
-  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->ikeys, 0, cap * 4, ctx->stream), "zero");
-  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->ikeys_tmp, 0, cap * 4, ctx->stream), "zero");
+  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->ivals, 0, sc_list_bytes(cap), ctx->stream), "zero");
+  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->ivals_tmp, 0, sc_list_bytes(cap), ctx->stream), "zero");
+  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->ikeys, 0, sc_list_bytes(cap), ctx->stream), "zero");
+  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->ikeys_tmp, 0, sc_list_bytes(cap), ctx->stream), "zero");
   tr->icap = cap;
   trainer_drop_graph(tr);
   return ensure_scratch(tr);
@@ -338,15 +338,15 @@ static sc_status ensure_pairs(sc_trainer* tr, uint64_t K) {
   uint64_t cap = K + K / 4 + 65536;
   if (cap > (1ull << 30) - 1) cap = (1ull << 30) - 1;
   if (K > cap) return sc_fail(ctx, SC_ERR_CAPACITY, "more than 2^30 tile/splat pairs in one step");
-  SC_CUDA_TRY(ctx, cudaMalloc(&tr->vals, cap * 4), "vals");
-  SC_CUDA_TRY(ctx, cudaMalloc(&tr->keys, cap * 4), "keys");
-  SC_CUDA_TRY(ctx, cudaMalloc(&tr->keys_tmp, cap * 4), "keys");
-  SC_CUDA_TRY(ctx, cudaMalloc(&tr->vals_tmp, cap * 4), "vals");
+  SC_CUDA_TRY(ctx, cudaMalloc(&tr->vals, sc_list_bytes(cap)), "vals");
+  SC_CUDA_TRY(ctx, cudaMalloc(&tr->keys, sc_list_bytes(cap)), "keys");
+  SC_CUDA_TRY(ctx, cudaMalloc(&tr->keys_tmp, sc_list_bytes(cap)), "keys");
+  SC_CUDA_TRY(ctx, cudaMalloc(&tr->vals_tmp, sc_list_bytes(cap)), "vals");
   // zero-filled so a step whose emission overflowed still reads valid ids
-  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->vals, 0, cap * 4, ctx->stream), "zero");
-  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->keys, 0, cap * 4, ctx->stream), "zero");
-  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->keys_tmp, 0, cap * 4, ctx->stream), "zero");
-  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->vals_tmp, 0, cap * 4, ctx->stream), "zero");
+  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->vals, 0, sc_list_bytes(cap), ctx->stream), "zero");
+  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->keys, 0, sc_list_bytes(cap), ctx->stream), "zero");
+  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->keys_tmp, 0, sc_list_bytes(cap), ctx->stream), "zero");
+  SC_CUDA_TRY(ctx, cudaMemsetAsync(tr->vals_tmp, 0, sc_list_bytes(cap), ctx->stream), "zero");
   tr->kcap = cap;
   trainer_drop_graph(tr);
   return ensure_scratch(tr);

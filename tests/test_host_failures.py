@@ -84,3 +84,31 @@ L.fake_step(0, 0, TAKERS, 5000)
 step()
 assert L.fake_bad() == 0 and L.fake_pool_cap() >= 5000
 """)
+
+
+@pytest.mark.parametrize("sort_mode", [0, 1])
+def test_list_arrays_end_on_a_whole_group_of_four_words_in_the_trainer(fake_lib, sort_mode):
+    """The blends read their lists in 16-byte groups, the last of which may reach
+    beyond the list: into the array's own bytes, whatever count sized it."""
+    run(fake_lib, f"""
+tr, step = trainer(sort_mode={sort_mode})
+step()
+for n in (65537, 200002, 700003):
+    L.fake_step(n, n, CAPACITY, 0)  # sizes the arrays for n + n / 4 + 65536 words
+    step()
+assert L.fake_composites() >= 4 and L.fake_bad() == 0
+""")
+
+
+def test_list_arrays_end_on_a_whole_group_of_four_words_in_the_binner(fake_lib):
+    run(fake_lib, """
+from nanotracer_b200 import Rasterizer, TileBinner
+g = GpuSplatBuffer.upload(ctx, scene)
+r, tl = Rasterizer(ctx), TilingParams(W, H, 16, 8.0)
+proj, img = r.alloc_projected(g), r.alloc_image(W, H)
+for n in (1, 101, 4002, 70003):
+    L.fake_scan_total(n)  # sizes the arrays for n + n / 8 + 1024 words
+    bins = TileBinner(ctx).bin(proj, 300, tl, stride=g.capacity)
+    r.composite(proj, bins, img, tl, g.capacity)
+assert L.fake_composites() == 4 and L.fake_bad() == 0
+""")
