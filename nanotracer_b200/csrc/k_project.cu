@@ -78,7 +78,7 @@ struct CamPtr {
   __device__ __forceinline__ Cam get(uint32_t v) const { return load_cam(p + v); }
 };
 template <uint32_t N>
-struct CamArgs {
+struct __align__(16) CamArgs {  // read as float4, wherever it stands among the parameters
   sc_camera c[N];
   __device__ __forceinline__ Cam get(uint32_t v) const {
     const float4* p = reinterpret_cast<const float4*>(c + v);
@@ -86,6 +86,7 @@ struct CamArgs {
   }
 };
 static_assert(sizeof(sc_camera) == 96, "camera layout");
+static_assert(alignof(CamArgs<1>) == 16 && sizeof(CamArgs<1>) == sizeof(sc_camera), "read as float4");
 
 __device__ __forceinline__ void sh_basis15(float x, float y, float z, float b[15]) {
   const float xx = x * x, yy = y * y, zz = z * z;
