@@ -82,6 +82,24 @@ __global__ void k_finalize(const double* __restrict__ loss_sums, const double* _
   out->chunks = most;
 }
 
+// What a captured step holds of its call: the stores whole (an array that took
+// another's place in memory may have another capacity or form).
+struct StepInputs {
+  DSplats s;
+  DMoments mo;
+  const void *acc, *targets, *h_targets, *gout;
+  uint32_t scene_max_cap, scene_max_gstride, shards, shard;
+  float weight;
+  bool grads;
+  bool operator==(const StepInputs& o) const {
+    return s.slab == o.s.slab && s.rest16 == o.s.rest16 && s.n == o.s.n && s.cap == o.s.cap && s.bf16 == o.s.bf16 &&
+           mo.m == o.mo.m && mo.v == o.mo.v && mo.m16 == o.mo.m16 && mo.v16 == o.mo.v16 && mo.cap == o.mo.cap &&
+           mo.bf16 == o.mo.bf16 && acc == o.acc && targets == o.targets && h_targets == o.h_targets &&
+           gout == o.gout && scene_max_cap == o.scene_max_cap && scene_max_gstride == o.scene_max_gstride &&
+           shards == o.shards && shard == o.shard && weight == o.weight && grads == o.grads;
+  }
+};
+
 // stage names of the two-level binning step (the pair-sort step uses kStageNames)
 const char* kStageNames2[] = {"project", "depth_sort", "count_scan", "item_emit", "item_sort", "item_ranges",
                               "blend_fwd", "blend_bwd", "bwd_adam"};
@@ -169,13 +187,10 @@ struct sc_trainer {
   uint32_t scene_max_cap = 0, scene_max_gstride = 0;
   // a viewer's frame (sc_view): forward only, into the caller's records and image
   bool forward_only = false;
-  // graph
+  // the captured step, and the last step's inputs; whatever replaces one of the
+  // trainer's own arrays drops the graph
   cudaGraphExec_t exec = nullptr;
-  const void* g_key[8] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-  uint64_t g_key_n = 0, g_key_kcap = 0, g_key_icap = 0;
-  bool g_key_grads = false;
-  float g_key_w = 0.0f;
-  uint32_t g_key_shards = 0, g_key_shard = 0;
+  StepInputs inputs{};
   // results of the last step
   uint64_t last_pairs = 0, last_items = 0;
   uint32_t kernels_per_step = 0;
@@ -753,18 +768,18 @@ static sc_status run_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, float* a
   // many scenes: the table (stores, counts, rows) is copied by the step's first
   // node, so the graph depends only on the capacities that size its grids
   SC_TRY(ensure_splat_arrays(tr, tr->scenes_mode ? tr->scene_max_cap : s->cap));
+  // A step whose inputs are those of the step before is captured and replayed;
+  // one with others (stores taken in turn, a densified store) is launched
+  // kernel by kernel, which costs less than a capture used once.
+  const StepInputs in{s ? dview(s) : DSplats{}, mo ? dview(mo) : DMoments{}, acc, tr->targets, tr->h_targets, tr->gout,
+                      tr->scenes_mode ? tr->scene_max_cap : 0u, tr->scenes_mode ? tr->scene_max_gstride : 0u,
+                      tr->g_shards, tr->g_shard, tr->loss_weight, tr->grads_mode};
+  const bool again = tr->inputs == in;
+  if (!again) trainer_drop_graph(tr);
+  tr->inputs = in;
   for (int attempt = 0; attempt < 4; ++attempt) {
-    const bool sizing = tr->kcap == 0 || (tr->two_level && tr->icap == 0);
-    const void* mkey = mo ? (mo->m ? (const void*)mo->m : (const void*)mo->m16) : nullptr;
-    const void* key[8] = {s ? s->slab : nullptr, s ? s->rest16 : nullptr, mkey, acc, tr->targets, tr->scratch,
-                          tr->gout, tr->h_targets};
-    const uint64_t key_n = s ? s->n : ((uint64_t)tr->scene_max_cap << 32 | tr->scene_max_gstride);
-    const bool key_ok = tr->exec && std::equal(key, key + 8, tr->g_key) && tr->g_key_n == key_n &&
-                        tr->g_key_kcap == tr->kcap && tr->g_key_icap == tr->icap && tr->g_key_grads == tr->grads_mode &&
-                        tr->g_key_w == tr->loss_weight && tr->g_key_shards == tr->g_shards &&
-                        tr->g_key_shard == tr->g_shard;
-    if (!key_ok) trainer_drop_graph(tr);
-    if (tr->cfg.use_graph && !sizing) {
+    const bool sizing = tr->two_level ? tr->icap == 0 : tr->kcap == 0;
+    if (tr->cfg.use_graph && again && !sizing) {
       if (!tr->exec) {
         cudaGraph_t g = nullptr;
         SC_CUDA_TRY(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed), "begin capture");
@@ -775,14 +790,6 @@ static sc_status run_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, float* a
         ce = cudaGraphInstantiate(&tr->exec, g, 0);
         cudaGraphDestroy(g);
         if (ce != cudaSuccess) { tr->exec = nullptr; return sc_cuda_fail(ctx, ce, "graph instantiate"); }
-        std::copy(key, key + 8, tr->g_key);
-        tr->g_key_n = key_n;
-        tr->g_key_kcap = tr->kcap;
-        tr->g_key_icap = tr->icap;
-        tr->g_key_grads = tr->grads_mode;
-        tr->g_key_w = tr->loss_weight;
-        tr->g_key_shards = tr->g_shards;
-        tr->g_key_shard = tr->g_shard;
       }
       SC_CUDA_TRY(ctx, cudaGraphLaunch(tr->exec, ctx->stream), "graph launch");
       ctx->launches += tr->kernels_per_step;

@@ -19,7 +19,8 @@
 #include <vector>
 
 namespace {
-std::map<const void*, size_t> g_live;
+std::map<const void*, size_t> g_live, g_room;
+std::multimap<size_t, void*> g_free;
 std::map<const void*, std::string> g_names;
 using Graph = std::vector<std::function<void()>>;
 Graph* g_capture = nullptr;
@@ -45,12 +46,20 @@ void enqueue(std::function<void()> f) {
 cudaError_t alloc(void** p, size_t n) {
   *p = nullptr;
   if (g_fail > 0 && --g_fail == 0) return g_last = cudaErrorMemoryAllocation;
-  *p = std::calloc(1, n ? n : 1);
+  // a freed array's memory goes to the next one that fits, as a device's does
+  auto it = g_free.lower_bound(n);
+  if (it != g_free.end()) {
+    *p = it->second;
+    g_free.erase(it);
+  } else {
+    g_room[*p = std::malloc(n + (1u << 20))] = n + (1u << 20);
+  }
+  std::memset(*p, 0, n);
   g_live[*p] = n;
   return cudaSuccess;
 }
 cudaError_t release(void* p) {
-  if (p && g_live.erase(p)) std::free(p);
+  if (p && g_live.erase(p)) g_free.emplace(g_room[p], p);
   return cudaSuccess;
 }
 cudaError_t launch(const void* func, void** args) {

@@ -112,3 +112,56 @@ for n in (1, 101, 4002, 70003):
     r.composite(proj, bins, img, tl, g.capacity)
 assert L.fake_composites() == 4 and L.fake_bad() == 0
 """)
+
+
+@pytest.mark.parametrize("sort_mode", [0, 1])
+def test_steps_of_the_same_inputs_replay_a_graph_and_others_do_not(fake_lib, sort_mode):
+    """The first step sizes the arrays, the second is captured, and the graph is
+    launched from then on; a store that takes a freed one's place in memory with
+    another capacity, and stores taken in turn, are launched afresh."""
+    run(fake_lib, f"""
+tr, step = trainer(sort_mode={sort_mode})
+for k in range(5):
+    step()
+    assert L.fake_replays() == k, (k, L.fake_replays())
+def arrays(capacity):
+    g = GpuSplatBuffer.upload(ctx, scene, capacity=capacity)
+    mo = AdamMomentBuffers(ctx, 4096)
+    return g, mo
+acc, far = ctx.storage_buffer_zeroed("acc", 4 * 4096), arrays(2048)
+g, mo = arrays(512)
+r0 = L.fake_replays()
+for t in (1, 2):
+    tr.step(g, mo, acc, [cam], t)
+assert L.fake_replays() == r0 + 1
+g.free()
+again = GpuSplatBuffer.upload(ctx, scene, capacity=1024)
+tr.step(again, mo, acc, [cam], 3)
+assert L.fake_replays() == r0 + 1, "a graph of another capacity was replayed"
+for t in range(4, 8):
+    tr.step(*((again, mo) if t % 2 else far), acc, [cam], t)
+assert L.fake_replays() == r0 + 1
+# an overflow in a replayed step: the arrays grow, and the step runs again
+tr.step(*far, acc, [cam], 8), tr.step(*far, acc, [cam], 9)
+r1, c1 = L.fake_replays(), L.fake_composites()
+L.fake_step(300001, 300001, CAPACITY, 0)
+L.fake_step(300001, 300001, TAKERS, 3000)
+L.fake_step(300001, 300001, 0, 3000)
+tr.step(*far, acc, [cam], 10)
+assert (L.fake_replays() - r1, L.fake_composites() - c1) == (3, 3) and L.fake_pool_cap() >= 3000
+assert L.fake_bad() == 0
+""")
+
+
+def test_many_scenes_replay_a_graph(fake_lib):
+    run(fake_lib, """
+from nanotracer_b200.scenes import Scene, ScenesTrainer
+tr = ScenesTrainer(ctx, 2, W, H)
+for i in range(2):
+    g = GpuSplatBuffer.upload(ctx, scene)
+    tr.set_scene(i, Scene(g, AdamMomentBuffers(ctx, g.capacity), ctx.storage_buffer_zeroed("a", 4 * g.capacity),
+                          W, H, ctx.storage_buffer_zeroed("t", 12 * W * H)))
+for t in range(1, 6):
+    tr.step([cam, cam], t)
+assert L.fake_replays() == 4 and L.fake_bad() == 0
+""")
