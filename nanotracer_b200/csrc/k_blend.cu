@@ -235,6 +235,13 @@ __device__ __forceinline__ bool plain_record(const float4 ra, const float4 rb, f
          det > 9.765625e-4f * (rb.x * rb.z) && op < ALPHA_MAX;
 }
 
+// Values whose products and sums over a list stay finite.
+constexpr float ORDINARY = 1e15f;
+__device__ __forceinline__ bool ordinary_record(const float4 ra, const float4 rb, const float4 rc) {
+  return fabsf(ra.x) + fabsf(ra.y) + fabsf(rb.x) + fabsf(rb.y) + fabsf(rb.z) + fabsf(rc.x) + fabsf(rc.y) +
+         fabsf(rc.z) + fabsf(rc.w) < ORDINARY;
+}
+
 // How a warp gets its entries, in stages of up to 32: gather() starts the copies
 // of the next stage's records (3 float4 each, cp.async) and returns its size, 0
 // at the end; ready() waits for them and returns how many of them are left to
@@ -316,11 +323,12 @@ struct ListFeed {
   uint32_t at;            // next chunk: [at, at + 128), REV: [at - 128, at); a multiple of 4
   uint32_t qtail, qhead;  // entries queued and gathered
   uint4 key, wid;         // this lane's four words of the next chunk
+  bool odd;               // REV: the landed stage has a record that is not ordinary
 
   __device__ __forceinline__ ListFeed(ListSmem& smem, const ListArgs& l, const float4* rec, uint32_t b, uint32_t n,
                                       uint32_t bit, uint32_t stage)
       : sm(smem), ids(l.ids), keys(l.keys), vrec(rec), mask(0x10000u << bit), begin(b), end(b + n), most(stage),
-        at(REV ? (b + n + 3u) & ~3u : b & ~3u), qtail(0), qhead(0), key(make_uint4(0, 0, 0, 0)), wid(key) {
+        at(REV ? (b + n + 3u) & ~3u : b & ~3u), qtail(0), qhead(0), key(make_uint4(0, 0, 0, 0)), wid(key), odd(false) {
     load();
   }
   __device__ __forceinline__ bool more() const { return REV ? at > begin : at < end; }
@@ -383,6 +391,7 @@ struct ListFeed {
     const uint32_t id = sm.st.id[lane], pos = sm.st.pos[lane];
     const bool keep = lane < n && reaches(ra, rb, rc.w, w);
     const uint32_t bal = __ballot_sync(FULL_MASK, keep);
+    if constexpr (REV) odd = __any_sync(FULL_MASK, keep && !ordinary_record(ra, rb, rc));
     if (keep) {
       const uint32_t slot = STAGE + __popc(bal & ((1u << lane) - 1u));
       float4* d = sm.st.rec + 3 * slot;
@@ -1094,19 +1103,21 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
     const float2 gr2 = make_float2(gr[0], gr[PPT - 1]), gg2 = make_float2(gg[0], gg[PPT - 1]);
     const float2 gb2 = make_float2(gb[0], gb[PPT - 1]), fy2 = make_float2(fy[0], fy[PPT - 1]);
     bool stopped = false;
-    // An entry of a list need not be taken by a pixel of the warp, and one that
-    // no pixel takes sends nothing; nor does a pixel add to an entry that it
-    // skips.  Both matter where zeros would not do: a pixel whose dL/dC is not
-    // finite (odd: the warp has one), an entry whose record is not.  The takers
-    // are taken by definition.
-    constexpr bool GATED = LIST != LIST_TAKERS;
-    uint32_t took = 0;  // octet path: the rows that this thread's pixels took
-    bool odd = false;
-    if constexpr (GATED && OCT) {
+    // A pixel that skips an entry carries zeros for it, which add nothing unless
+    // they meet a value that is not finite: a pixel's dL/dC or T, or the entry's
+    // record.  The entries of a list that some pixel need not have taken are then
+    // walked with `gate`: a skipping pixel leaves its state alone and adds an
+    // exact zero, and an entry that no pixel of the warp takes sends nothing.
+    // (On every entry the gate cost a stage-by-stage step of 100k splats at 800x600
+    // 12 us of 508, apart 1; one of 61k at 1013x571, 3 views, in the reference's
+    // mode 6 of 798 either way.)
+    uint32_t took = 0;  // with gate: the rows that this thread's pixels took
+    bool odd = false;   // the warp has such a pixel
+    if constexpr (LIST != LIST_TAKERS && OCT) {
       float s = 0.0f;
 #pragma unroll
-      for (int q = 0; q < PPT; ++q) s += fabsf(gr[q]) + fabsf(gg[q]) + fabsf(gb[q]);
-      odd = __any_sync(FULL_MASK, !(s < INFINITY));
+      for (int q = 0; q < PPT; ++q) s += fabsf(gr[q]) + fabsf(gg[q]) + fabsf(gb[q]) + fabsf(T[q]);
+      odd = __any_sync(FULL_MASK, !(s < ORDINARY));
     }
     // octet path: a thread's two pixels' (h, -T alpha) of entry i (zeros where a
     // pixel skips it).  Alpha is carried negated, which needs no negations in
@@ -1114,7 +1125,7 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
     // (1 / 1 is exact) and its sums.
     // `plain`: the stage's records are plain and no pixel of the warp stops
     // behind its entries, which leaves the alpha >= 1/255 test alone.
-    auto entry2 = [&](auto plain, uint32_t i, uint32_t row, const float4* r) -> float4 {
+    auto entry2 = [&](auto plain, auto gate, uint32_t i, uint32_t row, const float4* r) -> float4 {
       constexpr bool PLAIN = decltype(plain)::value;
       const float4 ra = r[0], rb = r[1], rc = r[2];
       const EntryGeom e = entry_geom(fx, ra, rb);
@@ -1136,15 +1147,15 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
       }
       const float2 gm = make_float2(v0 && (PLAIN || araw.x < ALPHA_MAX) ? g.x : 0.0f,
                                     v1 && (PLAIN || araw.y < ALPHA_MAX) ? g.y : 0.0f);
-      const float2 ta = __fmul2_rn(Tn, am);
+      float2 ta = __fmul2_rn(Tn, am);
       // dC/dalpha = T_i c - S / (1 - alpha) = (T_{i+1} c - S) / (1 - alpha)
       const float2 dc = make_float2(fmaf(gb2.x, rc.z, fmaf(gg2.x, rc.y, gr2.x * rc.x)),
                                     fmaf(gb2.y, rc.z, fmaf(gg2.y, rc.y, gr2.y * rc.x)));
       float2 h = __fmul2_rn(__fmul2_rn(inv, __ffma2_rn(T2, dc, NG2)), gm);
       float2 ng = __ffma2_rn(ta, dc, NG2);
-      if constexpr (GATED) {
-        if (!v0) { h.x = 0.0f; ng.x = NG2.x; }
-        if (!v1) { h.y = 0.0f; ng.y = NG2.y; }
+      if constexpr (decltype(gate)::value) {
+        if (!v0) { h.x = ta.x = 0.0f; ng.x = NG2.x; Tn.x = T2.x; }
+        if (!v1) { h.y = ta.y = 0.0f; ng.y = NG2.y; Tn.y = T2.y; }
         if (v0 || v1) took |= 1u << row;
       }
       NG2 = ng;
@@ -1154,10 +1165,11 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
       return make_float4(h.x, h.y, ta.x, ta.y);
     };
     // turn round: the sums of entries i0 .. i0 + rows - 1 over the warp's pixels, and out
-    auto turn = [&](uint32_t i0, uint32_t rows) {
+    auto turn = [&](auto gate, uint32_t i0, uint32_t rows) {
       if constexpr (OCT) {
+        constexpr bool GATE = decltype(gate)::value;
         uint32_t taken = 0xFFFFFFFFu;
-        if constexpr (GATED) {
+        if constexpr (GATE) {
           taken = __reduce_or_sync(FULL_MASK, took);
           took = 0;
         }
@@ -1171,7 +1183,7 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
           const float2 h = make_float2(x.x, x.y), ta = make_float2(x.z, x.w);
           float4 rg = sm.red.rg[oq * 9 + j];
           float2 b = sm.red.b[oq * 9 + j];
-          if (GATED && odd) {  // T alpha is 0 where the pixel skips the entry only
+          if constexpr (GATE) {  // T alpha of a pixel that skips the entry is 0
             if (ta.x == 0.0f) rg.x = rg.z = b.x = 0.0f;
             if (ta.y == 0.0f) rg.y = rg.w = b.y = 0.0f;
           }
@@ -1192,7 +1204,7 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
         float c6[6], c3[3];
         rs_half<12, 16>(c, c6, lane);
         rs_half<6, 8>(c6, c3, lane);
-        if (oe < rows && oq < 3 && (taken >> oe & 1u)) send(i0 + oe, oq, make_float3(c3[0], c3[1], c3[2]));
+        if (oe < rows && oq < 3 && (!GATE || (taken >> oe & 1u))) send(i0 + oe, oq, make_float3(c3[0], c3[1], c3[2]));
         __syncwarp();  // the rows may be written again
       }
     };
@@ -1246,16 +1258,17 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
       uint32_t i = 0;
       if constexpr (OCT) {
         float4* row = sm.red.row + lane;
-        auto walk = [&](auto plain) {
+        auto walk = [&](auto plain, auto gate) {
+          constexpr int U = decltype(gate)::value ? 1 : OCT_E;  // the rare walk stays small
           for (; i + OCT_E <= n && !stopped; i += OCT_E) {
-#pragma unroll
-            for (int e = 0; e < OCT_E; ++e) row[e * OCT_ROW] = entry2(plain, i + e, e, sr + 3 * (i + e));
-            turn(i, OCT_E);
+#pragma unroll U
+            for (int e = 0; e < OCT_E; ++e) row[e * OCT_ROW] = entry2(plain, gate, i + e, e, sr + 3 * (i + e));
+            turn(gate, i, OCT_E);
             if (MODE == SC_BWD_REF) stopped = __all_sync(FULL_MASK, all_done);
           }
           if (i < n && !stopped) {
-            for (uint32_t e = 0; i + e < n; ++e) row[e * OCT_ROW] = entry2(plain, i + e, e, sr + 3 * (i + e));
-            turn(i, n - i);
+            for (uint32_t e = 0; i + e < n; ++e) row[e * OCT_ROW] = entry2(plain, gate, i + e, e, sr + 3 * (i + e));
+            turn(gate, i, n - i);
             if (MODE == SC_BWD_REF) stopped = __all_sync(FULL_MASK, all_done);
           }
         };
@@ -1264,8 +1277,11 @@ __global__ void __launch_bounds__(256) k_composite_backward(const float4* __rest
           const float4* r = sr + 3 * lane;
           plain = __all_sync(FULL_MASK, lane >= (int)n || plain_record(r[0], r[1], r[2].w));
         }
-        if (plain) walk(std::true_type{});
-        else walk(std::false_type{});
+        bool gate = false;
+        if constexpr (LIST != LIST_TAKERS) gate = odd || feed.odd;
+        if (LIST != LIST_TAKERS && gate) walk(std::false_type{}, std::true_type{});
+        else if (plain) walk(std::true_type{}, std::false_type{});
+        else walk(std::false_type{}, std::false_type{});
       } else {
         // two entries together: one 18-value reduce-scatter
         for (; i < n && !stopped; i += 2) {
