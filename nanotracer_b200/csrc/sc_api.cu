@@ -96,6 +96,11 @@ sc_status sc_ctx_create(int device, sc_ctx** out) {
   if (e == cudaSuccess) e = cudaDeviceGetAttribute(&ctx->sm_count, cudaDevAttrMultiProcessorCount, device);
   if (e == cudaSuccess) e = cudaMalloc(&ctx->d_error, 256);
   if (e == cudaSuccess) e = cudaMemset(ctx->d_error, 0, 256);
+  ctx->pinned = std::make_shared<sc_pinned>();
+  if (e == cudaSuccess && cudaMallocHost(&ctx->pinned->base, sc_pinned::SLOT * sc_pinned::SLOTS) != cudaSuccess) {
+    ctx->pinned->base = nullptr;  // the trainers allocate for themselves
+    cudaGetLastError();
+  }
   if (e != cudaSuccess) {
     sc_ctx_destroy(ctx);
     return SC_ERR_CUDA;

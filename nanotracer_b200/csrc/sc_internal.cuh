@@ -14,6 +14,8 @@
 #include <cuda_bf16.h>
 #include <stdint.h>
 
+#include <memory>
+#include <mutex>
 #include <string>
 #include <utility>
 
@@ -39,6 +41,32 @@
 // with a nanosleep back-off; ~1 s worst case before giving up)
 #define SC_SPIN_LIMIT (1u << 22)
 
+// A context's page-locked memory, one slot per trainer or view for its step
+// parameters and results: an allocation of its own took 2 to 3 ms, more than
+// the first frame of a small scene (20k splats, 640x360: constructor and first
+// frame 4.2 -> 1.7 ms).  The objects share the block, which goes with the last of
+// them; one that finds no slot free allocates for itself.
+struct sc_pinned {
+  static constexpr size_t SLOT = 8192, SLOTS = 16;
+  char* base = nullptr;
+  uint32_t used = 0;
+  std::mutex lock;
+  ~sc_pinned() { cudaFreeHost(base); }
+  void* take() {
+    std::lock_guard<std::mutex> g(lock);
+    for (uint32_t i = 0; base && i < SLOTS; ++i)
+      if (!(used >> i & 1u)) {
+        used |= 1u << i;
+        return base + i * SLOT;
+      }
+    return nullptr;
+  }
+  void give(void* p) {
+    std::lock_guard<std::mutex> g(lock);
+    used &= ~(1u << (uint32_t)((static_cast<char*>(p) - base) / SLOT));
+  }
+};
+
 struct sc_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -55,6 +83,7 @@ struct sc_ctx {
   // the trainer's chains of kernels launch with programmatic stream
   // serialization (sc_launch)
   bool overlap_launches = false;
+  std::shared_ptr<sc_pinned> pinned;
   // grow-only scratch arena for temporaries of the reference-shaped calls
   void* scratch = nullptr;
   size_t scratch_bytes = 0;

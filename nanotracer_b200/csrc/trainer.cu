@@ -121,9 +121,10 @@ struct sc_trainer {
   uint32_t V = 0, tiles_x = 0, tiles_y = 0, T = 0;
   uint64_t P = 0;
   uint32_t stride = 0;
+  std::shared_ptr<sc_pinned> pinned;  // whose slot h_params is, or null
   StepParams* h_params = nullptr;
   StepParams* d_params = nullptr;
-  StepOut* h_out = nullptr;  // page-locked, written by the step's last kernel
+  StepOut* h_out = nullptr;  // page-locked, behind h_params; written by the step's last kernel
   // per (view, splat)
   float4* rec = nullptr; float4* pgrad = nullptr;
   float4* pcomp = nullptr;  // compensation records of pgrad (cfg.compensated_sums)
@@ -608,6 +609,23 @@ static sc_status enqueue_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, floa
   return SC_OK;
 }
 
+// the step's parameters and results: one page-locked block, and the device's copy
+static cudaError_t alloc_step_params(sc_trainer* tr) {
+  constexpr size_t out_at = (sizeof(StepParams) + 63) / 64 * 64, bytes = out_at + sizeof(StepOut);
+  static_assert(bytes <= sc_pinned::SLOT, "a slot holds a step's parameters and results");
+  void* block = tr->ctx->pinned->take();
+  if (block) {
+    tr->pinned = tr->ctx->pinned;
+  } else {
+    const cudaError_t e = cudaMallocHost(&block, bytes);
+    if (e != cudaSuccess) return e;
+  }
+  std::memset(block, 0, bytes);
+  tr->h_params = static_cast<StepParams*>(block);
+  tr->h_out = reinterpret_cast<StepOut*>(static_cast<char*>(block) + out_at);
+  return cudaMalloc(&tr->d_params, sizeof(StepParams));
+}
+
 extern "C" {
 
 sc_status sc_trainer_create(sc_ctx* ctx, const sc_train_config* cfg, sc_trainer** out) {
@@ -652,9 +670,7 @@ sc_status sc_trainer_create(sc_ctx* ctx, const sc_train_config* cfg, sc_trainer*
   tr->two_level = cfg->sort_mode != 1 && tr->super_bits + bits_for(tr->V - 1) <= 16;
   tr->P = (uint64_t)t.width * t.height;
   const size_t pix = (size_t)tr->V * tr->P;
-  cudaError_t e = cudaMallocHost(&tr->h_params, sizeof(StepParams));
-  if (e == cudaSuccess) e = cudaMallocHost(&tr->h_out, sizeof(StepOut));
-  if (e == cudaSuccess) e = cudaMalloc(&tr->d_params, sizeof(StepParams));
+  cudaError_t e = alloc_step_params(tr);
   if (e == cudaSuccess) e = cudaMalloc(&tr->image, pix * 16);
   if (e == cudaSuccess) e = cudaMalloc(&tr->aux, pix * 8);
   if (e == cudaSuccess) e = cudaMalloc(&tr->dl_dc, pix * 16);
@@ -670,7 +686,6 @@ sc_status sc_trainer_create(sc_ctx* ctx, const sc_train_config* cfg, sc_trainer*
     sc_trainer_free(ctx, tr);
     return sc_cuda_fail(ctx, e, "trainer alloc");
   }
-  std::memset(tr->h_params, 0, sizeof(StepParams));
   // a first guess of 5 chunks a warp and a quarter more; a step that draws more
   // runs again with the number it needs
   const sc_status st = ensure_takers(tr, sc_div_up(5 * heads, sck::TAKER_POOLS) + 1);
@@ -708,8 +723,8 @@ void sc_trainer_free(sc_ctx* ctx, sc_trainer* tr) {
   cudaFree(tr->d_scenes);
   if (tr->h_scenes) cudaFreeHost(tr->h_scenes);
   if (tr->h_losses) cudaFreeHost(tr->h_losses);
-  if (tr->h_params) cudaFreeHost(tr->h_params);
-  if (tr->h_out) cudaFreeHost(tr->h_out);
+  if (tr->pinned) tr->pinned->give(tr->h_params);
+  else if (tr->h_params) cudaFreeHost(tr->h_params);
   for (int i = 0; i <= kStages; ++i)
     if (tr->ev[i]) cudaEventDestroy(tr->ev[i]);
   delete tr;
@@ -933,20 +948,16 @@ sc_status sc_view_create(sc_ctx* ctx, const sc_tiling* tl, sc_view** out) {
   tr->P = (uint64_t)tl->width * tl->height;
   tr->ST = sck::super_tiles_per_view(tl);
   tr->super_bits = bits_for(tr->ST);
-  tr->two_level = tr->super_bits <= 16;
-  cudaError_t e = (uint64_t)tr->tiles_x * tr->tiles_y > 65536 ? cudaErrorInvalidValue : cudaSuccess;
-  if (e != cudaSuccess) {
+  tr->two_level = true;  // at most 65536 tiles, so at most 16 bits of super tile
+  if ((uint64_t)tr->tiles_x * tr->tiles_y > 65536) {
     delete tr;
     return sc_fail(ctx, SC_ERR_INVALID_ARG, "REF32 keys hold at most 65536 tiles (tile_emit.wgsl key layout)");
   }
-  e = cudaMallocHost(&tr->h_params, sizeof(StepParams));
-  if (e == cudaSuccess) e = cudaMallocHost(&tr->h_out, sizeof(StepOut));
-  if (e == cudaSuccess) e = cudaMalloc(&tr->d_params, sizeof(StepParams));
+  const cudaError_t e = alloc_step_params(tr);
   if (e != cudaSuccess) {
     sc_trainer_free(ctx, tr);
     return sc_cuda_fail(ctx, e, "view alloc");
   }
-  std::memset(tr->h_params, 0, sizeof(StepParams));
   sc_view* v = new sc_view();
   v->tr = tr;
   *out = v;
@@ -975,7 +986,7 @@ sc_status sc_view_frame(sc_view* v, const sc_splats* s, const sc_camera* cam, fl
   tr->image = reinterpret_cast<float4*>(image);
   sc_status st = SC_OK;
   for (int attempt = 0; attempt < 4; ++attempt) {
-    const bool sizing = tr->two_level ? tr->icap == 0 : tr->kcap == 0;
+    const bool sizing = tr->icap == 0;
     tr->h_params->cams[0] = *cam;
     st = enqueue_step(tr, const_cast<sc_splats*>(s), nullptr, nullptr, false, sizing);
     if (st == SC_OK && rgba8)
@@ -996,7 +1007,6 @@ sc_status sc_view_frame(sc_view* v, const sc_splats* s, const sc_camera* cam, fl
     if (cudaMemsetAsync(ctx->d_error, 0, 4, ctx->stream) != cudaSuccess) st = sc_fail(ctx, SC_ERR_CUDA, "clear error");
     else if (o.err & SC_DEVERR_TIMEOUT) st = sc_fail(ctx, SC_ERR_TIMEOUT, "a bounded device wait gave up during the frame");
     if (st == SC_OK) st = ensure_items(tr, o.items);
-    if (st == SC_OK) st = ensure_pairs(tr, o.pairs);
     if (st != SC_OK) break;
     if (attempt == 3) st = sc_fail(ctx, SC_ERR_CAPACITY, "item capacity kept overflowing");
   }

@@ -16,7 +16,7 @@ from .gpu import CudaCtx
 from .raster import CameraUniform, Rasterizer
 from .splat_gpu import GpuSplatBuffer
 from .splat_store import SplatBuffer
-from .tile_binner import TileBinner, TilingParams
+from .tile_binner import TilingParams
 
 
 @dataclass
@@ -49,14 +49,19 @@ class HeadlessView:
         self.splats = splats if isinstance(splats, GpuSplatBuffer) else GpuSplatBuffer.upload(ctx, splats)
         self.width, self.height = int(width), int(height)
         self.rasterizer = Rasterizer(ctx)
-        self.binner = TileBinner(ctx)
         self.projected = ctx.storage_buffer_zeroed("projected", 48 * lib().sc_view_records(self.splats.handle))
         self.image = self.rasterizer.alloc_image(self.width, self.height, 1)
         self.rgba8 = ctx.storage_buffer_zeroed("rgba8", 4 * self.width * self.height)
-        self._view = None  # the library's frame state, made by the first frame
+        self._view = None
+        t, h = self._params(0.0).struct(), C.c_void_p()
+        check(lib().sc_view_create(ctx.handle, C.byref(t), C.byref(h)), ctx.handle)
+        self._view = h  # the library's working arrays, kept from frame to frame
+
+    def _params(self, depth_max: float) -> TilingParams:
+        return TilingParams(self.width, self.height, self.TILE, depth_max)
 
     def tiling(self, orbit: OrbitCamera) -> TilingParams:
-        return TilingParams(self.width, self.height, self.TILE, max(orbit.distance * 4.0, 50.0))
+        return self._params(max(orbit.distance * 4.0, 50.0))
 
     def frame(self, orbit: OrbitCamera) -> np.ndarray:
         """Render one frame; returns (height, width, 4) uint8 (sRGB, alpha = coverage)."""
@@ -64,10 +69,6 @@ class HeadlessView:
         cam = CameraUniform.from_pose(orbit.position(), np.asarray(orbit.target, np.float32), (0.0, 1.0, 0.0),
                                       orbit.fov_y, self.width, self.height, n)
         params = self.tiling(orbit)
-        if self._view is None:
-            t, h = params.struct(), C.c_void_p()
-            check(lib().sc_view_create(self.ctx.handle, C.byref(t), C.byref(h)), self.ctx.handle)
-            self._view = h
         out = np.empty((self.height, self.width, 4), np.uint8)
         check(lib().sc_view_frame(self._view, self.splats.handle, C.byref(cam.c), float(params.depth_max),
                                   self.projected.cptr, self.image.cptr, self.rgba8.cptr, ptr(out)), self.ctx.handle)

@@ -103,6 +103,7 @@ uint64_t fake_bad() { return g_bad; }
 uint64_t fake_composites() { return g_composites; }
 uint64_t fake_replays() { return g_replays; }
 uint64_t fake_pool_cap() { return g_pool_cap; }
+uint64_t fake_live() { return g_live.size(); }
 
 void** __cudaRegisterFatBinary(void*) { static void* h; return &h; }
 void __cudaRegisterFatBinaryEnd(void**) {}

@@ -19,7 +19,7 @@ from nanotracer_b200.scene import FOV_Y, orbit_pose, random_scene
 from nanotracer_b200.train import TrainConfig, Trainer
 import ctypes as C
 L = lib()
-for f in (L.fake_bad, L.fake_composites, L.fake_replays, L.fake_pool_cap):
+for f in (L.fake_bad, L.fake_composites, L.fake_replays, L.fake_pool_cap, L.fake_live):
     f.restype = C.c_uint64
 L.fake_step.argtypes = [C.c_uint64, C.c_uint64, C.c_uint32, C.c_uint32]
 L.fake_scan_total.argtypes = [C.c_uint64]
@@ -164,4 +164,39 @@ for i in range(2):
 for t in range(1, 6):
     tr.step([cam, cam], t)
 assert L.fake_replays() == 4 and L.fake_bad() == 0
+""")
+
+
+def test_trainers_and_views_share_the_contexts_page_locked_slots(fake_lib):
+    """More of them than there are slots, taken and given back in any order, and
+    the context closed while one lives: each reads its own results, and all
+    memory comes back."""
+    run(fake_lib, """
+import gc
+from nanotracer_b200.view import HeadlessView, OrbitCamera
+base = L.fake_live()
+trainers = [trainer() for _ in range(20)]
+for k, (tr, step) in enumerate(trainers):
+    L.fake_step(100 + k, 0, 0, 0)
+    step()
+assert [tr.stats()["pairs"] for tr, _ in trainers] == [100 + k for k in range(20)]
+views = [HeadlessView(ctx, scene, W, H) for _ in range(3)]
+del trainers[::2], tr, step
+gc.collect()
+views += [HeadlessView(ctx, scene, W, H) for _ in range(12)]
+for v in views:
+    v.frame(OrbitCamera())
+for k, (tr, step) in enumerate(trainers):
+    step()
+assert L.fake_bad() == 0
+del views, v, trainers, tr, step
+gc.collect()
+assert L.fake_live() == base, (L.fake_live(), base)
+tr, _ = trainer()
+handle, ctx2 = tr.handle, ctx.handle
+tr.handle = None
+gc.collect()
+lib().sc_ctx_destroy(ctx2)
+ctx.handle = None
+lib().sc_trainer_free(None, handle)
 """)
