@@ -798,7 +798,9 @@ static sc_status run_step(sc_trainer* tr, sc_splats* s, sc_moments* mo, float* a
       if (!tr->exec) {
         cudaGraph_t g = nullptr;
         SC_CUDA_TRY(ctx, cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeRelaxed), "begin capture");
+        const uint64_t launched = ctx->launches;
         sc_status st = enqueue_step(tr, s, mo, acc, true, false);
+        ctx->launches = launched;  // captured, not launched
         cudaError_t ce = cudaStreamEndCapture(ctx->stream, &g);
         if (st != SC_OK) { if (g) cudaGraphDestroy(g); return st; }
         if (ce != cudaSuccess) return sc_cuda_fail(ctx, ce, "end capture");

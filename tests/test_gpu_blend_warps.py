@@ -16,7 +16,8 @@ import ctypes as C
 import numpy as np
 import pytest
 
-from nanotracer_b200 import CameraUniform, GpuSplatBuffer, GradSplatBuffers, Rasterizer, TileBinner, TilingParams
+from nanotracer_b200 import (AdamMomentBuffers, CameraUniform, GpuSplatBuffer, GradSplatBuffers, Rasterizer, TileBinner,
+                             TilingParams)
 from nanotracer_b200._lib import SC_BWD_EXACT, SC_BWD_REF, SC_KEYS_REF32, check, lib
 from nanotracer_b200.raster import cameras_array
 from nanotracer_b200.scene import FOV_Y, orbit_pose, random_scene
@@ -86,6 +87,76 @@ def test_trainer_backward_over_the_takers_equals_the_list_backward(ctx, tile, n,
     for lo, hi in [(0, 3), (3, 7), (7, 10), (10, 11), (11, 14), (14, 59)]:
         d = np.linalg.norm((got[lo:hi] - want[lo:hi]).astype(np.float64))
         assert d <= 1e-5 * np.linalg.norm(want[lo:hi].astype(np.float64)) + 1e-30, (lo, d)
+
+
+def _faint(n):
+    """Wide and so faint that no pixel saturates: a warp takes a quarter of them
+    or more, over 40 chunks of 32 where a new trainer has room for some 70 in
+    a pool of one tile's warps."""
+    s = _scene(n)
+    s.scales[:] = np.log(0.6)
+    s.opacities[:] = -5.0
+    return s
+
+
+@pytest.mark.parametrize("tile", [(16, 16), (8, 8), (32, 3)])
+def test_a_step_that_takes_more_entries_than_there_is_room_for_runs_again(ctx, tile):
+    """The forward runs out of chunks: the step's backward and Adam are skipped,
+    the pools grow to the counted need and the step runs again.  Its gradients
+    are the list backward's, and a training step's parameters and moments those
+    of a trainer that had the room already (its second step; moments and
+    parameters start from the same values)."""
+    n, W, H = 8000, 64, 48
+    scene = _faint(n)
+    cam = CameraUniform.from_pose(*orbit_pose(20.0), FOV_Y, W, H, n)
+    tl = TilingParams(W, H, tile[0], 8.0, tile_h_override=tile[1])
+    tgt = _targets(W, H)
+    want, img = _stage_grads(ctx, scene, cam, tl, tgt, W, H)
+    cfg = TrainConfig(n_views=1, width=W, height=H, tile_w=tile[0], tile_h=tile[1], depth_max=8.0, tile_cull=False)
+    g = GpuSplatBuffer.upload(ctx, scene)
+    tr = Trainer(ctx, cfg)
+    tr.set_targets(ctx.storage_buffer("t", tgt))
+    shard = (n + 63) // 64 * 64
+    out = ctx.storage_buffer_zeroed("grads", 59 * shard * 4)
+    loss = C.c_double()
+
+    def grad_step():
+        before = ctx.launch_count
+        check(lib().sc_trainer_step_grads(tr.handle, g.handle, cameras_array([cam]), 1.0, 1, shard, out.cptr,
+                                          C.byref(loss)), ctx.handle)
+        return ctx.launch_count - before
+
+    runs = [grad_step() for _ in range(3)]
+    kernels = tr.stats()["kernels_per_step"]
+    assert runs[0] == 2 * kernels and runs[1:] == [kernels, kernels], (runs, kernels)
+    got = out.readback(np.float32, 59 * shard).reshape(59, shard)[:, :n]
+    assert np.array_equal(img, tr.images()[0])
+    for lo, hi in [(0, 3), (3, 7), (7, 10), (10, 11), (11, 14), (14, 59)]:
+        d = np.linalg.norm((got[lo:hi] - want[lo:hi]).astype(np.float64))
+        assert d <= 1e-5 * np.linalg.norm(want[lo:hi].astype(np.float64)), (lo, d)
+
+    def train_step(trainer):
+        gs = GpuSplatBuffer.upload(ctx, scene)
+        mo = AdamMomentBuffers(ctx, gs.capacity)
+        acc = ctx.storage_buffer_zeroed("acc", 4 * gs.capacity)
+        before = ctx.launch_count
+        ls = trainer.step(gs, mo, acc, [cam], 1)
+        m, v = mo.download(n)
+        return ctx.launch_count - before, ls, gs.readback().flat(), m.flat().astype(np.float64), v.flat(), \
+            acc.readback(np.float32, n)
+
+    fresh = Trainer(ctx, cfg)
+    fresh.set_targets(ctx.storage_buffer("t", tgt))
+    la, lossa, pa, ma, va, aa = train_step(fresh)
+    lb, lossb, pb, mb, vb, ab = train_step(fresh)
+    assert la >= 2 * lb - 2 and abs(lossa - lossb) <= 1e-9 * lossb
+    assert np.linalg.norm(ma - mb) <= 1e-5 * np.linalg.norm(mb)
+    assert np.linalg.norm((va - vb).astype(np.float64)) <= 2e-5 * np.linalg.norm(vb.astype(np.float64))
+    assert np.allclose(aa, ab, rtol=1e-3, atol=1e-5 * ab.max())
+    # the first Adam step moves a parameter by lr times its gradient's sign: where
+    # the gradient stands above its rounding, both moved alike
+    clear = np.abs(mb) > 1e-3 * np.abs(mb).max(axis=0)
+    assert np.allclose(pa[clear], pb[clear], rtol=1e-6, atol=1e-7) and clear.mean() > 0.3
 
 
 @pytest.mark.parametrize("mode", [SC_BWD_EXACT, SC_BWD_REF])
