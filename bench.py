@@ -436,9 +436,8 @@ def stage_bytes(N: int, V: int, P: int, K: int, items: int, bw: dict, bf16: bool
     bwd_list = bw.get("bwd_scanned", 0) * 8 + bw.get("bwd_blended", 0) * 48  # list entry, written and read + record
     tile_passes = max(1, math.ceil(max(1, (tiles - 1).bit_length()) / 8))
     return {
-        # records, cleared gradient records (by the projection backward, as
-        # far as they are nonzero), depth key, id, item count
-        "project": N * (56 + rest_b) + V * N * (48 + 48 + 4 + 4 + 4),
+        # parameters; records, depth key, id, item count
+        "project": N * (56 + rest_b) + V * N * (48 + 4 + 4 + 4),
         # segmented onesweep over the 16-bit depth keys: a histogram read, then 2 passes
         # of 8-bit digits each reading and writing key + id
         "depth_sort": V * N * 4 + 2 * V * N * 16,
@@ -453,8 +452,8 @@ def stage_bytes(N: int, V: int, P: int, K: int, items: int, bw: dict, bf16: bool
         "item_ranges": items * 4,
         "blend_fwd": fwd_list + V * P * (16 + 8),
         "blend_bwd": bwd_list + V * P * (16 + 8 + 12) + V * N * 48,
-        # projection backward: per-view gradient records + geometry in, 59 f32 gradient
-        # rows out; streaming Adam: rows, parameters, moments and statistic in and out
+        # projection backward: per-view gradient records (the few nonzero ones
+        # cleared, not counted) + geometry in, 59 f32 gradient rows out; streaming Adam: rows, parameters, moments and statistic in and out
         "bwd_adam": (V * N * 48 + N * 44 + N * 236 +
                      ((N * 236 + N * 2 * (56 + rest_b) + N * 2 * mom_b + N * 8) if adam else 0)),
     }

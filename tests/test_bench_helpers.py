@@ -66,7 +66,7 @@ def test_stage_bytes_follow_the_stated_formulas():
     full = bench.stage_bytes(N, V, P, K, items, bw, True, tiles)
     split = bench.stage_bytes(N, V, P, K, items, bw, True, tiles, adam=False)
     f32 = bench.stage_bytes(N, V, P, K, items, bw, False, tiles)
-    assert full["project"] == N * (56 + 90) + V * N * 108
+    assert full["project"] == N * (56 + 90) + V * N * 60
     assert full["depth_sort"] == V * N * 4 + 2 * V * N * 16
     assert full["item_sort"] == items * 20
     assert full["blend_fwd"] == 900 * 8 + 300 * 48 + V * P * 24
