@@ -380,7 +380,8 @@ typedef struct sc_train_config {
   sc_tiling tiling;            /* image size and tile shape                      */
   sc_adam_groups adam;         /* per-group learning rates                        */
   uint32_t bwd_mode;           /* sc_bwd_mode                                    */
-  uint32_t use_graph;          /* capture the iteration as a CUDA graph          */
+  uint32_t use_graph;          /* replay the iteration as a CUDA graph, captured when a step's inputs are
+                                  those of the step before                       */
   uint32_t blend_batch;        /* blend batch depth: list positions the blend forward takes per stage (a
                                   multiple of 32; a quarter of them entries, 8 to 32); 0 = 128 */
   uint32_t sort_mode;          /* 0 = auto (two-level), 1 = depth presort + stable sort of the

@@ -67,7 +67,7 @@ class Trial:
 
     @property
     def label(self) -> str:
-        return (f"{self.tile_w}x{self.tile_h}/sort_mode {self.sort_mode}/batch {self.blend_batch or 'all'}"
+        return (f"{self.tile_w}x{self.tile_h}/sort_mode {self.sort_mode}/batch {self.blend_batch or 128}"
                 f"/digits {self.sort_digit_bits or 'auto'}")
 
 
@@ -106,7 +106,7 @@ def time_steps(ctx: CudaCtx, scene: SplatBuffer, cams: list[CameraUniform], targ
                cfg: TrainConfig, warmup: int = 2, steps: int = 3):
     """(mean wall time in ms of `steps` training steps of `cfg` on a fresh
     device copy of `scene` after `warmup` untimed steps, hash of the first
-    step's images).  The first warm-up step captures the step's graph; each
+    step's images).  The second warm-up step captures the step's graph; each
     step reads its loss back, so the host clock brackets finished device work."""
     g = GpuSplatBuffer.upload(ctx, scene, bf16_rest=cfg.bf16)
     mo = AdamMomentBuffers(ctx, g.capacity, bf16=cfg.bf16)

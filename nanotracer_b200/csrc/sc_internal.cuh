@@ -345,10 +345,12 @@ sc_status sc_check_device_error(sc_ctx* ctx);
 // ctx->overlap_launches its launch overlaps the end of the kernel before it on
 // the stream: its blocks become resident as that one's last blocks leave, and
 // wait in sc_after_previous() until it has completed and its writes are
-// visible, so nothing else changes.  A step of 5k splats falls from 0.198 to
-// 0.175 ms, of 200k from 0.479 to 0.449, of 1M from 1.154 to 1.115, 8 views of 1M from 4.22 to 4.18
-// ms.  Letting the next kernel's blocks in from the start (launch_dependents
-// first of all) costs what they hold while they wait: 0.193, 0.496, 1.302, 4.28 ms.
+// visible, so nothing else changes.  Launched kernel by kernel, a step of 5k
+// splats falls from 0.198 to 0.175 ms, of 200k from 0.479 to 0.449, of 1M from
+// 1.154 to 1.115, 8 views of 1M from 4.22 to 4.18 ms; replayed from a graph from
+// 0.142 to 0.139, and not at all from 200k up (0.440, 1.093, 4.18 ms either way).
+// Letting the next kernel's blocks in from the start (launch_dependents first of
+// all) costs what they hold while they wait: 0.193, 0.496, 1.302, 4.28 ms.
 template <typename... P, typename... A>
 static inline void sc_launch(sc_ctx* ctx, void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, A&&... args) {
   cudaLaunchConfig_t c{};
